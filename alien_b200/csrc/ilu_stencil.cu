@@ -9,65 +9,49 @@
 //
 // Schedule.  In a 3-D 7-point matrix numbered i + nx (j + ny k), row (i,j,k)
 // of the forward sweep depends on (i,j,k-1), (i,j-1,k) and (i-1,j,k).  A CTA
-// of 16 x 16 threads owns a 16 x 16 tile of z-lines, one thread per line, and
-// walks the tile's diagonals: at step s thread (li,lj) computes cell
-// k = s - li - lj.  Its k-1 input is its own previous value (a register), the
-// i-1 and j-1 inputs were computed by neighbouring threads at step s-1 (shared
-// memory, one named barrier per step).  Only the first line of a tile reads a
-// value owned by another tile, 15 steps ahead in that tile's walk; those come
-// through global memory (the sentinel values of sentinel.cuh), fetched by a
-// ninth, polling warp that hands them over through shared memory.  Tiles
-// are claimed from an atomic ticket in dependency order (a tile waits only on
-// tiles with a smaller ticket), so no co-residency is needed.
+// owns a 16 x 16 tile of z-lines, in two strips of 16 x 8 lines; one warp computes
+// a strip, 2 x 2 lines a lane, and walks its diagonals: at step s lane (ti, tj)
+// computes its four cells of plane k = s - ti - tj.  Its k-1 inputs are its own
+// previous values, the i-1 and j-1 inputs the neighbouring lanes' values of step
+// s-1 (warp shuffles): nothing in a strip waits on a barrier.  Between strips and
+// tiles values are handed over word by word, the word being its own flag (the
+// sentinel of sentinel.cuh): from strip to strip through a ring in shared memory,
+// from tile to tile through global memory, where polling warps of the next tile
+// fetch them into such a ring.  Tiles are claimed from an atomic ticket in
+// row-major order (a tile waits only on tiles with a smaller ticket), so no
+// co-residency is needed.  Every wait is bounded.
 //
-// Walk layout.  At one step the 256 threads of a tile touch 31 different
-// z-planes, so in natural order every warp access would be 32 separate cache
-// lines, and a step would cost the LSU ~1.2 us instead of ~0.16 us (measured on
-// B200 for this access pattern against the same walk on contiguous data).  The
-// sweeps therefore read and write arrays stored in WALK order: index
-// ((tile * nsteps + s) * 256 + thread), nsteps = nz + 30 rounded up to the
-// prefetch depth, so one warp access is 32 consecutive doubles.  The factor
-// bands are gathered into that order once at set-up; each application gathers
-// y in (one bulk kernel), runs the two walks, and scatters z out (one bulk
-// kernel) -- bulk kernels have the whole GPU to hide latency, a wavefront
-// step does not.  Those two are transposes through shared memory
-// (k_walk_gather_t / k_walk_scatter_t), contiguous on both sides; against
-// element-wise gather/scatter they saved ~30 us per application at 192^3
-// (14 ms per CG+ILU0 solve of 286 applications, measured before the poll
-// warp below).
+// The backward sweep is the same walk in mirrored coordinates (i' = nx - 1 - i
+// and so on), its own coefficients packed in that order.
 //
-// The backward sweep is the forward walk run backwards: the U walk's thread
-// (li,lj) of tile T at step s handles the cell the L walk handles at the
-// mirrored position (15-li, 15-lj, ntiles-1-T, nsteps-1-s), whose walk index is
-// walk_n - 1 - w (the U walk's cells then start nsteps - nz - 30 steps
-// late).  So both walks use the same arrays, the U walk through the reversed
-// index, and both are coalesced.  Its dependencies (+i, +j, +k) are
-// then again "previous thread / previous tile / own previous step".
+// Everything else is kept away from the compute warps: loading warps bring the
+// coefficients (packed by strip and step at set-up, one bulk copy for two steps)
+// and the right-hand side (natural order, placed by the step that uses it) into
+// rings in shared memory, storing warps take the results out of a ring into
+// natural order.  So an application is two kernels and moves every band, the
+// input, the vector between the sweeps and the output once.
 //
-// The factorisation runs once per set-up on the natural-order bands with the
-// same walk (pivots propagate; in a 7-point matrix ILU(0) changes only the
-// diagonal and the L values).
+// What bounds it: the dependency chain, nx + ny + nz - 2 cells long.  A warp that
+// waits for its own results issues one instruction in three to four cycles, so a
+// step costs what its instructions cost: 165 ns forward, 272 ns backward (a lone
+// tile, 1.9 GHz; FP64 operations 8 cycles apart), and a hand-over to the next tile
+// 8 steps + 1.5 us (store, poll and read back through L2).  Four cells a lane and
+// step because the cost of a step is mostly not the cells: counting steps on the
+// critical path, nx/2 + ny/2 + nz instead of nx + ny + nz.  The division by the
+// pivot is three dependent FMAs longer than the subtraction chain instead of ~140
+// cycles, off a reciprocal stored at set-up (below).
 //
-// Measured on B200, one application at 192^3: 0.61 ms (gather + two walks +
-// scatter; 0.97 ms before the poll warp), against 1.69 ms for the same walk
-// on natural-order arrays and 3.45 ms for the wavefront schedule of
-// precond.cu.  Values loaded per poll round: 4 steps (2: 0.63 ms, 3: 0.60,
-// 8: 0.63, 16: 0.70).  The cluster walk further down (2 x 2 tiles a cluster,
-// hand-offs inside a cluster through distributed shared memory, step inputs
-// by bulk copy): 0.551 ms.
+// Measured on B200, one application (both sweeps, FP64): 192^3 541 -> 360 us,
+// 128^3 350 -> 200 us, 70 x 90 x 50 204 -> 101 us, against one line a thread, 16 x 16
+// threads and a barrier a step, tiles in 2 x 2 clusters, with separate passes that
+// brought the vectors into walk order and back.
 //
-// Where the time goes (per-tile timestamps of one L walk at 192^3, 144
-// tiles): a tile without upstream tiles steps in 0.265 us; tiles downstream
-// step in 0.34-0.42 us, since every step waits for a value its neighbour
-// produced 15 steps earlier plus the hand-off; a tile starts its walk ~8.5 us
-// (16 neighbour steps + hand-off) after its upstream tile.  The critical path
-// is 22 such lags plus one tile's walk: ~263 us.  The dependency depth
-// (nx + ny + nz - 2 = 574 steps) at the lone tile's step time would be 152 us.
-#include <cooperative_groups.h>
+// The factorisation runs once per set-up on the natural-order bands, one line a
+// thread (pivots propagate; in a 7-point matrix ILU(0) changes only the diagonal
+// and the L values).
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <atomic>
 #include <type_traits>
 
 #include "ab2_internal.cuh"
@@ -76,19 +60,13 @@
 
 namespace ab2 {
 
-namespace cg = cooperative_groups;
-
 namespace {
 
-constexpr int kTile = 16;
+constexpr int kTile = 16;  // the factorisation walk: one line a thread
 constexpr int kTileThreads = kTile * kTile;
-constexpr int kWalkPrefetch = 8;  // steps a walk loads ahead; the walk length is padded to a multiple
-// The sweeps' poll warp: steps whose neighbouring-tile values it loads per
-// round (all in flight at once), and the shared-memory ring it hands them to
-// the compute warps through.
-constexpr int kPollDepth = 4;
-constexpr int kBndRing = 16;
-static_assert(kBndRing >= kPollDepth, "a poll round fits in the ring");
+// AB2_ILU_STENCIL and AB2_ILU_STENCIL_CLUSTER name one walk now; callers still
+// get (and are refused) the second by the number of planes along z.
+constexpr int kClusterPlanes = 346;
 
 struct Geom {
   int nx, ny, nz, ntx, nty;
@@ -225,488 +203,107 @@ __global__ void __launch_bounds__(kTileThreads) k_stencil_factor(Geom g, Bands b
   }
 }
 
-// ------------------------------------------------------------------ walk layout
+// ------------------------------------------------------------------ walk shape
+constexpr int kTileI = 16, kTileJ = 16;          // lines of a tile (one CTA)
+constexpr int kStrips = 2;                       // strips of a tile, one compute warp each
+constexpr int kStripJ = kTileJ / kStrips;        // a strip: 16 x 8 lines, 2 x 2 a lane
+constexpr int kLanesI = kTileI / 2, kLanesJ = kStripJ / 2;
+constexpr int kSkew = kLanesI - 1 + kLanesJ - 1;  // steps between a strip's first and last lane
+constexpr int kStripCells = kTileI * kStripJ;    // cells a strip computes in one step
+constexpr int kDepth = 12;                       // steps of inputs in flight or waiting, two on an mbarrier
+constexpr int kInRing = 24;                      // ring of input cells by step: kDepth + kSkew and a margin (even)
+constexpr int kOutRing = 22;                     // ring of output cells by step (even)
+constexpr int kSlots = 32;                       // ring of hand-over slots by step (a power of two)
+constexpr int kPollDepth = 2;                    // words a polling lane loads at once
+static_assert(kLanesI * kLanesJ == 32 && kInRing > kDepth + kSkew && kOutRing >= kSkew + 12, "walk shape");
+// Warps by role.  Warps w, w + 4 and w + 8 share an SM sub-partition: each
+// compute warp (0 and 1) shares its own with two polling warps, which mostly wait
+// on L2; the helpers -- two loading warps a strip (every other pair of steps) and
+// a storing warp a strip -- share the other two.  A helper's loop is a chain of
+// dependent instructions, several cycles each: what keeps it out of the compute
+// warp's way is having few of them per step.
+constexpr int kWalkWarps = 12;
+enum class Role { Compute, Load, Store, Poll };
+struct WarpRole {
+  Role role;
+  int strip, part;
+};
+__device__ __forceinline__ WarpRole warp_role(int warp) {
+  if (warp < 2) return {Role::Compute, warp, 0};
+  const int turn = warp >> 2;
+  if ((warp & 3) < 2) return {Role::Poll, 0, (turn - 1) * 2 + (warp & 1)};
+  const int strip = (warp & 3) - 2;
+  return turn < 2 ? WarpRole{Role::Load, strip, turn} : WarpRole{Role::Store, strip, 0};
+}
+static_assert(kStrips == 2, "warp roles");
+
 struct Walk {
-  int nx, ny, nz, ntx, nty, nsteps;
-  long long nxny, nw;  // nw = ntx nty nsteps 256
+  int nx, ny, nz, ntx, nty;
+  int nsteps;  // of a strip (even)
+  int halo;    // planes of a tile's hand-over words, kSkew unused ones either side
+  long long nxny, n;
 };
 
-// The natural row handled at walk index w of the L walk, or -1 (padding).
-__device__ __forceinline__ long long walk_row(const Walk& g, long long w) {
-  const int t = (int)(w & (kTileThreads - 1));
-  const long long q = w >> 8;
-  const int s = (int)(q % g.nsteps);
-  const int tile = (int)(q / g.nsteps);
-  const int li = t & (kTile - 1), lj = t >> 4;
-  const int i = (tile % g.ntx) * kTile + li, j = (tile / g.ntx) * kTile + lj, k = s - li - lj;
-  if (i >= g.nx || j >= g.ny || k < 0 || k >= g.nz) return -1;
-  return i + (long long)g.nx * j + g.nxny * k;
-}
-
-// dst[w] = src[row(w)] (0 on padding), rounded to T (the FP32 walk arrays
-// are gathered from the FP64 factor).
-template <class S, class T>
-__global__ void k_walk_gather(Walk g, const S* __restrict__ src, T* __restrict__ dst) {
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < g.nw; w += (long long)gridDim.x * blockDim.x) {
-    const long long r = walk_row(g, w);
-    dst[w] = r >= 0 ? (T)__ldg(src + r) : T(0);
-  }
-}
-
-// dst[row(w)] = src[w], and src[w] back to the sentinel for the next walk
-// (element-wise; the FP32 walk's scatter).
-template <class T>
-__global__ void k_walk_scatter(Walk g, T* __restrict__ src, T* __restrict__ dst) {
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < g.nw; w += (long long)gridDim.x * blockDim.x) {
-    const long long r = walk_row(g, w);
-    if (r >= 0) {
-      dst[r] = src[w];
-      src[w] = sentinel_of<T>();
-    }
-  }
-}
-
-// Walk order <-> natural order for every application (y in, z out), both
-// sides coalesced.  A thread keeps one grid line (li, lj) of a tile: at walk
-// step s it owns cell k = s - li - lj, so at one step a warp touches 32
-// consecutive walk entries, and at one plane k a warp touches two runs of 16
-// consecutive natural rows.  Each thread stages its own cells in a ring of
-// planes in shared memory (its own column: no barrier) and moves a plane
-// once every lane has it.  One CTA per (tile, kTrPlanes planes).
-// Measured per application at 192^3 (planes a CTA / batch): 64/4 550 us,
-// 64/8 598, 64/16 555, 96/8 583, 96/12 542, 96/16 542, 96/20 551, 96/24 553,
-// 96/32 561, 128/16 551, 128/24 564, 192/16 560.
-constexpr int kTrPlanes = 96;
-constexpr int kTrBatch = 12;                         // steps (planes) per batch
-constexpr int kTrRing = 2 * (kTile - 1) + kTrBatch;  // planes live at once per thread
-
-template <class T>
-constexpr int tr_smem() {
-  return kTrRing * kTileThreads * (int)sizeof(T);
-}
-
-// dst[row(w)] = src[w], and src[w] back to the sentinel for the next walk.
-template <class T>
-__global__ void __launch_bounds__(kTileThreads) k_walk_scatter_t(Walk g, T* __restrict__ src, T* __restrict__ dst) {
-  extern __shared__ unsigned char tr_smem_raw[];
-  T* ring = reinterpret_cast<T*>(tr_smem_raw);
-  const int nch = (g.nz + kTrPlanes - 1) / kTrPlanes;
-  const int tile = blockIdx.x / nch, ch = blockIdx.x - tile * nch;
-  const int t = threadIdx.x, li = t & (kTile - 1), lj = t >> 4, d = li + lj;
-  const int i = (tile % g.ntx) * kTile + li, j = (tile / g.ntx) * kTile + lj;
-  const bool line = i < g.nx && j < g.ny;
-  const int k0 = ch * kTrPlanes, k1 = min(g.nz, k0 + kTrPlanes);
-  const long long wb = (long long)tile * g.nsteps * kTileThreads + t;
-  const long long rb = i + (long long)g.nx * j;
-  int out = k0;
-  for (int s0 = k0; s0 < k1 + 2 * (kTile - 1); s0 += kTrBatch) {
-    // the batch's loads first (all in flight together), then the stores
-    T v[kTrBatch];
-#pragma unroll
-    for (int u = 0; u < kTrBatch; ++u) {
-      const int k = s0 + u - d;
-      v[u] = (line && k >= k0 && k < k1) ? __ldcs(src + wb + (long long)(s0 + u) * kTileThreads) : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < kTrBatch; ++u) {
-      const int k = s0 + u - d;
-      if (line && k >= k0 && k < k1) {
-        ring[(k % kTrRing) * kTileThreads + t] = v[u];
-        src[wb + (long long)(s0 + u) * kTileThreads] = sentinel_of<T>();
-      }
-    }
-    const int last = min(k1, s0 + kTrBatch - 2 * (kTile - 1));  // planes every lane has read
-    for (; out < last; ++out)
-      if (line) dst[rb + g.nxny * out] = ring[(out % kTrRing) * kTileThreads + t];
-  }
-}
-
-// dst[w] = src[row(w)] for the cells of the grid (padding entries are left
-// as they are: zero since set-up).
-template <class T>
-__global__ void __launch_bounds__(kTileThreads) k_walk_gather_t(Walk g, const T* __restrict__ src, T* __restrict__ dst) {
-  extern __shared__ unsigned char tr_smem_raw[];
-  T* ring = reinterpret_cast<T*>(tr_smem_raw);
-  const int nch = (g.nz + kTrPlanes - 1) / kTrPlanes;
-  const int tile = blockIdx.x / nch, ch = blockIdx.x - tile * nch;
-  const int t = threadIdx.x, li = t & (kTile - 1), lj = t >> 4, d = li + lj;
-  const int i = (tile % g.ntx) * kTile + li, j = (tile / g.ntx) * kTile + lj;
-  const bool line = i < g.nx && j < g.ny;
-  const int k0 = ch * kTrPlanes, k1 = min(g.nz, k0 + kTrPlanes);
-  const long long wb = (long long)tile * g.nsteps * kTileThreads + t;
-  const long long rb = i + (long long)g.nx * j;
-  int s = k0;  // next step to write
-  for (int p0 = k0; p0 < k1 + 2 * (kTile - 1); p0 += kTrBatch) {
-    T v[kTrBatch];
-#pragma unroll
-    for (int u = 0; u < kTrBatch; ++u) {
-      const int k = p0 + u;
-      v[u] = (line && k < k1) ? __ldcs(src + rb + g.nxny * k) : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < kTrBatch; ++u) {
-      const int k = p0 + u;
-      if (line && k < k1) ring[(k % kTrRing) * kTileThreads + t] = v[u];
-    }
-    const int last = p0 + kTrBatch;  // steps whose cells every lane has read
-    for (; s < last; ++s) {
-      const int k = s - d;
-      if (line && k >= k0 && k < k1) dst[wb + (long long)s * kTileThreads] = ring[(k % kTrRing) * kTileThreads + t];
-    }
-  }
-}
-
-template <class T>
-void set_transpose_smem() {
-  AB2_CUDA(cudaFuncSetAttribute(k_walk_scatter_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<T>()));
-  AB2_CUDA(cudaFuncSetAttribute(k_walk_gather_t<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<T>()));
-}
-
-template <class T>
-struct WalkArrays {
-  const T *Lk, *Lj, *Li, *Ui, *Uj, *Uk, *P;
-};
-
-// Per-step inputs of a compute thread, loaded kWalkPrefetch steps ahead: the
-// right-hand side, three band values (L: -k,-j,-i ; U: +i,+j,+k) and the
-// pivot (U walk).
-template <class T>
-struct PreW {
-  T y, a1, a2, a3, piv;
-};
-
-__device__ __forceinline__ void compute_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kTileThreads) : "memory"); }
-
-template <class T>
-__device__ __forceinline__ T quiet_nan();
-template <>
-__device__ __forceinline__ double quiet_nan<double>() {
-  return __longlong_as_double(0x7FF8000000000000LL);
-}
-template <>
-__device__ __forceinline__ float quiet_nan<float>() {
-  return __uint_as_float(0x7FC00000u);
-}
-
-// One triangular sweep in walk layout.  UP = false: forward sweep
-// x_i = y_i - sum_{k<dcol} l_ik x_k (solveL, ILU0Preconditioner.h:181-198) from
-// `in` into `wave`.  UP = true: backward sweep x_i = (y_i - sum_{k>dcol} u_ik x_k)
-// / u_ii (solveU, :200-231), reading `in` through the reversed index and
-// putting it back to the sentinel.  `wave` must hold the sentinel on entry.
-//
-// A CTA is 8 compute warps (the 16 x 16 lines of a tile, synchronised per
-// step on named barrier 1) and one poll warp.  The 32 values a step needs
-// from the two neighbouring tiles (the first line's inputs: lane l < 16 the
-// j-side value of line (l, 0), lane 16 + l the i-side value of line (0, l))
-// are fetched by the poll warp: each round it loads the next kPollDepth
-// steps' values at once, publishes the leading steps whose values have all
-// arrived into a ring in shared memory (s_ready = last published step), and
-// reloads the rest in the next round.  A compute thread on the first line
-// spins on s_ready in shared memory, not on a global load.  Why: a tile's
-// first steps run right behind its neighbour's; a compute warp that found
-// the sentinel and polled L2 itself paid a full round trip inside every such
-// step (about 1 us against a 0.26 us step), and the next tile waits on those
-// steps -- at 192^3 that cost 16-18 us per tile boundary on the critical
-// path.  With the polls in flight beside the compute, a step waits only for
-// the value's arrival.
-//
-// Every wait is bounded (kWaitCycles without progress): the poll warp then
-// records the error and publishes quiet NaNs, so the compute warps and the
-// kernel always finish.
-//
-// Compute warps: a step is a handful of instructions per thread, and every
-// array is reached through a per-thread pointer that moves once per group of
-// kWalkPrefetch steps, with constant offsets inside the unrolled group.
-template <bool UP, class T>
-__global__ void __launch_bounds__(kTileThreads + 32, 1) k_walk_sweep(Walk g, WalkArrays<T> b, T* in, T* wave,
-                                                                   unsigned int* tickets, int* err) {
-  constexpr int kPre = kWalkPrefetch;
-  constexpr long long kStep = UP ? -kTileThreads : kTileThreads;  // element stride of one step
-  __shared__ T s_val[2][kTile][kTile + 1];
-  __shared__ T s_bnd[kBndRing][2 * kTile];
-  __shared__ int s_tile;
-  __shared__ volatile int s_ready;  // last step whose neighbouring values are in s_bnd
-  __shared__ volatile int s_done;   // last step the compute warps have finished
-  const bool poller = threadIdx.x >= kTileThreads;
-  const int lane = threadIdx.x & 31;
-  // The line this thread computes (compute warps) or feeds (poll warp).
-  const int li = poller ? (lane < kTile ? lane : 0) : threadIdx.x % kTile;
-  const int lj = poller ? (lane < kTile ? 0 : lane - kTile) : threadIdx.x / kTile;
-  const int ntiles = g.ntx * g.nty;
-  const int nsteps = g.nsteps;
-  // Walk coordinates of the grid's first cell (the U walk's tiles are the
-  // mirror images of the L walk's, so a partial tile comes first, and its
-  // cells start nsteps - nz - 30 steps into the walk).
-  const int ox = UP ? g.ntx * kTile - g.nx : 0;
-  const int oy = UP ? g.nty * kTile - g.ny : 0;
-  const int oz = UP ? nsteps - g.nz - 2 * (kTile - 1) : 0;
-  auto phys = [&](long long w) { return UP ? g.nw - 1 - w : w; };
-
-  for (;;) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      s_tile = (int)atomicAdd(tickets + (UP ? 2 : 1), 1u);
-      s_ready = -1;
-      s_done = -1;
-    }
-    __syncthreads();
-    const int tile = s_tile;
-    if (tile >= ntiles) break;
-    const int ai = (tile % g.ntx) * kTile + li;
-    const int aj = (tile / g.ntx) * kTile + lj;
-    const bool active = ai >= ox && ai < ox + g.nx && aj >= oy && aj < oy + g.ny;
-    const bool has_i = ai > ox, has_j = aj > oy;  // walk predecessor along i / j
-    const bool bnd_i = li == 0 && has_i, bnd_j = lj == 0 && has_j;  // that predecessor is in another tile
-    // valid steps: s_lo <= s < s_hi (cell k = s - li - lj - oz in [0, nz))
-    const int s_lo = active ? li + lj + oz : nsteps;
-    const int s_hi = active ? s_lo + g.nz : nsteps;
-    const long long tbase = (long long)tile * nsteps * kTileThreads;
-
-    if (poller) {
-      // Neighbouring tile's cell at the same k: 15 steps further in that
-      // tile's walk (its last line along i, resp. j).
-      const bool need = lane < kTile ? bnd_j : bnd_i;
-      if (!__any_sync(0xffffffffu, need)) continue;  // first tile row and column: nothing to fetch
-      const long long w_nb =
-          lane < kTile ? phys(tbase - (long long)g.ntx * nsteps * kTileThreads + 15 * kTileThreads + 15 * kTile + li)
-                       : phys(tbase - (long long)nsteps * kTileThreads + 15 * kTileThreads + lj * kTile + 15);
-      const T* p_nb = wave + (need ? w_nb : 0);
-      long long t_last = clock64();
-      bool failed = false;
-      for (int t = 0; t < nsteps;) {
-        // ring space: slot (t + d) % kBndRing is free once step t + d - kBndRing is done
-        const int space = __shfl_sync(0xffffffffu, s_done, 0) + kBndRing - t + 1;
-        if (space <= 0) {
-          __nanosleep(64);
-          bool stop = (clock64() - t_last > kWaitCycles) || *(volatile int*)err;
-          if (__any_sync(0xffffffffu, stop)) {  // the compute warps stopped progressing: give up
-            if (lane == 0) atomicOr(err, 1);
-            break;
-          }
-          continue;
-        }
-        T v[kPollDepth];
-#pragma unroll
-        for (int d = 0; d < kPollDepth; ++d) {
-          const int st = t + d;
-          v[d] = (need && st >= s_lo && st < s_hi && !failed) ? ld_relaxed(p_nb + (long long)st * kStep) : T(0);
-        }
-        int first_missing = kPollDepth;
-#pragma unroll
-        for (int d = kPollDepth - 1; d >= 0; --d) {
-          const int st = t + d;
-          if (need && st >= s_lo && st < s_hi && is_sentinel(v[d]) && !failed) first_missing = d;
-        }
-        int n_pub = __reduce_min_sync(0xffffffffu, first_missing);
-        if (n_pub == 0) {
-          bool stop = (clock64() - t_last > kWaitCycles) || *(volatile int*)err;
-          if (__any_sync(0xffffffffu, stop)) {
-            // give up on the missing values: quiet NaNs from here on
-            if (lane == 0) atomicOr(err, 1);
-            failed = true;
-          }
-          continue;
-        }
-        n_pub = min(n_pub, space);
-#pragma unroll
-        for (int d = 0; d < kPollDepth; ++d) {
-          const int st = t + d;
-          if (d < n_pub && need && st >= s_lo && st < s_hi)
-            s_bnd[st % kBndRing][lane] = failed ? quiet_nan<T>() : v[d];
-        }
-        __syncwarp();
-        if (lane == 0) {
-          __threadfence_block();
-          s_ready = t + n_pub - 1;
-        }
-        t += n_pub;
-        t_last = clock64();
-      }
-      continue;
-    }
-
-    // Compute warps.  Step-0 pointers: own cell at walk index tbase + thread.
-    const long long w_own = phys(tbase + threadIdx.x);
-    const T* p_y = in + w_own;
-    const T* p_a1 = (UP ? b.Ui : b.Lk) + w_own;
-    const T* p_a2 = (UP ? b.Uj : b.Lj) + w_own;
-    const T* p_a3 = (UP ? b.Uk : b.Li) + w_own;
-    const T* p_piv = b.P + w_own;
-    T* p_in = in + w_own;
-    T* p_out = wave + w_own;
-
-    // Loads of step s (offset o = s * kStep from the step-0 pointers).
-    auto load = [&](int s, long long o, PreW<T>& p) {
-      if (s < s_lo || s >= s_hi) return;
-      // Read-only path: none of these is written during the walk except
-      // in[] by the U walk, after its one read here.
-      p.y = __ldg(p_y + o);
-      p.a1 = __ldg(p_a1 + o);
-      p.a2 = __ldg(p_a2 + o);
-      p.a3 = __ldg(p_a3 + o);
-      if (UP) p.piv = __ldg(p_piv + o);
-    };
-    // The step's neighbouring-tile values, from the poll warp's ring.
-    auto boundary = [&](int s, T& vi, T& vj) {
-      if (s_ready < s) {
-        const long long t0 = clock64();
-        for (unsigned it = 1; s_ready < s; ++it) {
-          if ((it & 255) == 0 && (clock64() - t0 > kWaitCycles || *(volatile int*)err)) {
-            atomicOr(err, 1);
-            vi = vj = quiet_nan<T>();
-            return;
-          }
-        }
-      }
-      __threadfence_block();
-      if (bnd_j) vj = s_bnd[s % kBndRing][li];
-      if (bnd_i) vi = s_bnd[s % kBndRing][kTile + lj];
-    };
-
-    PreW<T> pre[kPre];
-#pragma unroll
-    for (int u = 0; u < kPre; ++u) {
-      pre[u] = PreW<T>{0, 0, 0, 0, 0};
-      load(u, u * kStep, pre[u]);
-    }
-    T own = 0;
-    for (int s0 = 0; s0 < nsteps; s0 += kPre) {  // nsteps is a multiple of kPre
-      const long long o0 = (long long)s0 * kStep;
-#pragma unroll
-      for (int u = 0; u < kPre; ++u) {
-        const int s = s0 + u;
-        const long long o = o0 + u * kStep;
-        const PreW<T> c = pre[u];
-        load(s + kPre, o + kPre * kStep, pre[u]);
-        T val = 0;
-        if (s >= s_lo && s < s_hi) {
-          const T* prev = &s_val[(s + 1) & 1][0][0];
-          T vi = 0, vj = 0;
-          if (bnd_i || bnd_j) boundary(s, vi, vj);
-          if (has_j && lj > 0) vj = prev[(lj - 1) * (kTile + 1) + li];
-          if (has_i && li > 0) vi = prev[lj * (kTile + 1) + li - 1];
-          const bool has_k = s > s_lo;
-          T acc = c.y;
-          if (!UP) {  // columns ascending: -k, -j, -i
-            if (has_k) acc = mul_sub_rn(c.a1, own, acc);
-            if (has_j) acc = mul_sub_rn(c.a2, vj, acc);
-            if (has_i) acc = mul_sub_rn(c.a3, vi, acc);
-            val = acc;
-          } else {  // columns ascending: +i, +j, +k
-            if (has_i) acc = mul_sub_rn(c.a1, vi, acc);
-            if (has_j) acc = mul_sub_rn(c.a2, vj, acc);
-            if (has_k) acc = mul_sub_rn(c.a3, own, acc);
-            p_in[o] = sentinel_of<T>();  // the L walk's output, ready for the next application
-            val = acc / c.piv;
-          }
-          st_relaxed(p_out + o, not_sentinel(val));
-          own = val;
-        }
-        s_val[s & 1][lj][li] = val;
-        compute_bar();
-        if (threadIdx.x == 0) {
-          __threadfence_block();
-          s_done = s;
-        }
-      }
-    }
-  }
-  // Hand the other sweep its ticket back (it does not run concurrently).
-  if (blockIdx.x == 0 && threadIdx.x == 0) tickets[UP ? 1 : 2] = 0u;
-}
-
-// ------------------------------------------------------------------ cluster walk
-// The same sweep with the tiles grouped into thread-block clusters of CX x CY
-// tiles, one tile per CTA.  Inside a cluster a tile's boundary values are
-// pushed by the producing threads (the last line along i, resp. j) straight
-// into the consuming CTA's shared memory, so a hand-off costs one store to a
-// neighbouring SM instead of a store to L2 followed by a poll of L2.
-// Hand-offs between clusters keep the poll warp's path through global memory.
-//
-// Every boundary value reaches the consuming compute thread through a buffer
-// of one slot per walk step (nsteps x 32 words of dynamic shared memory: the
-// j-side values of lines (l, 0) in lanes 0-15, the i-side values of lines
-// (0, l) in lanes 16-31).  Each slot is written once per launch and holds the
-// sentinel until its value arrives -- the value is the flag, as in global
-// memory -- so neither side waits for space and nothing is reset.  The poll
-// warp fills the slots of the sides whose upstream tile is in another
-// cluster; the producers in the cluster fill the others.
-//
-// The step inputs (y and the three bands, plus the pivot in the backward
-// sweep: 256 consecutive words per array and step in walk order) come by bulk
-// copy (cp.async.bulk, no multicast) into a ring of kInRing steps in shared
-// memory, issued by a tenth warp as soon as the compute warps free a slot and
-// completed on one mbarrier per slot; every compute thread waits on the slot
-// (bounded) and reads its words.  Against the single-CTA walk's register
-// prefetch this frees the compute warps' registers and load instructions; the
-// issuing warp is separate from the poll warp, whose rounds through L2 would
-// otherwise hold the copies back.
-//
-// Clusters take super-tiles from a ticket in row-major order, so a cluster
-// waits only on clusters that run or are done; the CTAs of one cluster run
-// together by construction.  Every wait is bounded as in the single-CTA walk.
-// A cluster barrier at the start makes every buffer valid before a peer
-// writes to it, and one at the end keeps each CTA's shared memory alive until
-// no peer can write to it any more; before it the issuing warp waits
-// (bounded) for its copies still in flight.
-
-// Shared-memory words by 32-bit address: this CTA's (shared::cta) and a
-// peer's (shared::cluster, from mapa).
+// ------------------------------------------------------------------ strip walk
+// Shared-memory words by 32-bit address.  asm volatile keeps these accesses
+// in program order among themselves, which is the order one warp's shared
+// memory accesses are performed in; no "memory" clobber, so arithmetic and
+// prefetched loads may be scheduled around them.
 __device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ unsigned peer_addr(unsigned a, int rank) {
-  unsigned r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-  return r;
+// By predicate (on: 0 or 1), so that a lane's share of a step is not a
+// branch: a divergent branch and its reconvergence cost the compute warp more
+// than the access itself.
+__device__ __forceinline__ void lds2_if(int on, unsigned a, double& x, double& y) {
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.volatile.shared.v2.f64 {%0, %1}, [%3];}"
+               : "+d"(x), "+d"(y) : "r"(on), "r"(a));
 }
-// No "memory" clobber: the value is its own flag, so no other access needs
-// ordering against the store, and a clobber would pin the walk's prefetched
-// loads in place (register spills in the FP64 backward sweep).
-__device__ __forceinline__ void st_peer(unsigned a, double v) {
-  asm volatile("st.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(a),
-               "l"((unsigned long long)__double_as_longlong(v)));
+__device__ __forceinline__ void lds2_if(int on, unsigned a, float& x, float& y) {
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; @p ld.volatile.shared.v2.f32 {%0, %1}, [%3];}"
+               : "+f"(x), "+f"(y) : "r"(on), "r"(a));
 }
-__device__ __forceinline__ void st_peer(unsigned a, float v) {
-  asm volatile("st.relaxed.cluster.shared::cluster.b32 [%0], %1;" ::"r"(a), "r"(__float_as_uint(v)));
+__device__ __forceinline__ void sts2_if(int on, unsigned a, double x, double y) {
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %0, 0; @p st.volatile.shared.v2.f64 [%1], {%2, %3};}" ::"r"(on), "r"(a),
+               "d"(x), "d"(y));
 }
-__device__ __forceinline__ double ld_slot(unsigned a, double) {
-  unsigned long long v;
-  asm volatile("ld.volatile.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
-  return __longlong_as_double((long long)v);
+__device__ __forceinline__ void sts2_if(int on, unsigned a, float x, float y) {
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %0, 0; @p st.volatile.shared.v2.f32 [%1], {%2, %3};}" ::"r"(on), "r"(a),
+               "f"(x), "f"(y));
 }
-__device__ __forceinline__ float ld_slot(unsigned a, float) {
-  unsigned v;
-  asm volatile("ld.volatile.shared.b32 %0, [%1];" : "=r"(v) : "r"(a));
-  return __uint_as_float(v);
+__device__ __forceinline__ void sts_int_if(int on, unsigned a, int v) {
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %0, 0; @p st.volatile.shared.s32 [%1], %2;}" ::"r"(on), "r"(a), "r"(v));
 }
-
-// A slot of this CTA's buffer: its value, waited for (bounded) if it has not
-// arrived yet.
-template <class T>
-__device__ __noinline__ T wait_slot(unsigned a, int* err) {
-  const long long t0 = clock64();
-  for (unsigned it = 1;; ++it) {
-    const T v = ld_slot(a, T());
-    if (!is_sentinel(v)) return v;
-    if ((it & 255) == 0 && (clock64() - t0 > kWaitCycles || *(volatile int*)err)) {
-      atomicOr(err, 1);
-      return quiet_nan<T>();
-    }
-  }
+// Weak forms for words handed over by an mbarrier or a counter.
+__device__ __forceinline__ void ldw2(unsigned a, double& x, double& y) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(x), "=d"(y) : "r"(a));
 }
-
-template <class T>
-__device__ __forceinline__ T take_slot(unsigned a, int* err) {
-  const T v = ld_slot(a, T());
-  return is_sentinel(v) ? wait_slot<T>(a, err) : v;
+__device__ __forceinline__ void ldw2(unsigned a, float& x, float& y) {
+  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(a));
 }
-
-// Step inputs by bulk copy: each step's rows of the walk arrays (256
-// consecutive words per array, in walk order) land in a ring of kInRing steps
-// in shared memory, each slot completed on its own mbarrier.
-constexpr int kInRing = 12;
-template <bool UP>
-constexpr int walk_in_fields() {
-  return UP ? 5 : 4;  // y, three bands (and the pivot)
+__device__ __forceinline__ void stw2(unsigned a, double x, double y) {
+  asm volatile("st.shared.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(x), "d"(y));
+}
+__device__ __forceinline__ void stw2(unsigned a, float x, float y) {
+  asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(x), "f"(y));
+}
+__device__ __forceinline__ void sts1(unsigned a, double x) {
+  asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(a), "d"(x));
+}
+__device__ __forceinline__ void sts1(unsigned a, float x) {
+  asm volatile("st.volatile.shared.f32 [%0], %1;" ::"r"(a), "f"(x));
+}
+__device__ __forceinline__ void lds1(unsigned a, double& x) {
+  asm volatile("ld.volatile.shared.f64 %0, [%1];" : "=d"(x) : "r"(a));
+}
+__device__ __forceinline__ void lds1(unsigned a, float& x) {
+  asm volatile("ld.volatile.shared.f32 %0, [%1];" : "=f"(x) : "r"(a));
+}
+__device__ __forceinline__ int lds_int(unsigned a) {
+  int v;
+  asm volatile("ld.volatile.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void sts_int(unsigned a, int v) {
+  asm volatile("st.volatile.shared.s32 [%0], %1;" ::"r"(a), "r"(v));
 }
 
 __device__ __forceinline__ void mbar_init(unsigned a, unsigned count) {
@@ -726,290 +323,618 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned a, unsigned parity) {
       : "memory");
   return done != 0;
 }
-// Global -> this CTA's shared memory, completing on the mbarrier (no
-// multicast: the destination is this CTA's own window).
+// The same without the wait (try_wait may suspend the warp for a while).
+__device__ __forceinline__ bool mbar_test(unsigned a, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(a), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Global -> this CTA's shared memory, completing on the mbarrier.
 __device__ __forceinline__ void bulk_load(unsigned dst, const void* src, unsigned bytes, unsigned mbar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(mbar)
                : "memory");
 }
-// The walk's output word, its own flag for the next tiles (no "memory"
-// clobber: no other access needs ordering against it).
-__device__ __forceinline__ void st_flag(double* p, double x) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)__double_as_longlong(x)));
+template <int BYTES>
+__device__ __forceinline__ void copy_word(unsigned dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
 }
-__device__ __forceinline__ void st_flag(float* p, float x) {
-  asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(__float_as_uint(x)));
+// This thread's copies so far, one arrival of the mbarrier's count.
+__device__ __forceinline__ void copy_arrive(unsigned mbar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Two hand-over words in global memory, each its own flag (no "memory"
+// clobber: no other access needs ordering against them).
+__device__ __forceinline__ void st_flag2_if(int on, double* p, double x, double y) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.s32 p, %0, 0; @p st.relaxed.gpu.global.f64 [%1], %2; @p st.relaxed.gpu.global.f64 "
+      "[%1+8], %3;}" ::"r"(on), "l"(p), "d"(x), "d"(y));
+}
+__device__ __forceinline__ void st_flag2_if(int on, float* p, float x, float y) {
+  asm volatile(
+      "{.reg .pred p; setp.ne.s32 p, %0, 0; @p st.relaxed.gpu.global.f32 [%1], %2; @p st.relaxed.gpu.global.f32 "
+      "[%1+4], %3;}" ::"r"(on), "l"(p), "f"(x), "f"(y));
 }
 
-// A word of the input ring (after the mbarrier wait, whose "memory" clobber
-// keeps the load behind it).
-__device__ __forceinline__ double ld_in(unsigned a, double) {
-  unsigned long long v;
-  asm("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
-  return __longlong_as_double((long long)v);
+template <class T>
+__device__ __forceinline__ T quiet_nan();
+template <>
+__device__ __forceinline__ double quiet_nan<double>() {
+  return __longlong_as_double(0x7FF8000000000000LL);
 }
-__device__ __forceinline__ float ld_in(unsigned a, float) {
-  unsigned v;
-  asm("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
-  return __uint_as_float(v);
+template <>
+__device__ __forceinline__ float quiet_nan<float>() {
+  return __uint_as_float(0x7FC00000u);
 }
 
-// Waits for the phase of the given parity within the time bound only (the
-// end-of-kernel drain of copies in flight); false if it gave up.
+// Whether a hand-over word has not arrived: the sentinel by its upper half
+// alone (a signalling NaN, which no arithmetic result is).
+__device__ __forceinline__ bool waiting(double v) { return __double2hiint(v) == (int)(kSentinel >> 32); }
+__device__ __forceinline__ bool waiting(float v) { return is_sentinel(v); }
+
+// A bounded wait's give-up test, asked every 256 polls.
+__device__ __forceinline__ bool give_up(unsigned it, long long t0, int* err) {
+  if ((it & 255) != 0) return false;
+  if (clock64() - t0 <= kWaitCycles && *(volatile int*)err == 0) return false;
+  atomicOr(err, 1);
+  return true;
+}
+
+__device__ __noinline__ bool mbar_wait(unsigned a, unsigned parity, int* err) {
+  const long long t0 = clock64();
+  for (unsigned it = 16;; it += 16) {
+    if (mbar_try_wait(a, parity)) return true;
+    if (give_up(it, t0, err)) return false;
+  }
+}
+// Waits within the time bound only (copies in flight at the kernel's end).
 __device__ __noinline__ bool mbar_drain(unsigned a, unsigned parity) {
   const long long t0 = clock64();
   while (!mbar_try_wait(a, parity))
     if (clock64() - t0 > kWaitCycles) return false;
   return true;
 }
-
-// Waits (bounded) for the phase of the given parity; false if it gave up.
-__device__ __noinline__ bool mbar_wait(unsigned a, unsigned parity, int* err) {
+// Waits until the counter at `a` is at least `v`.
+__device__ __noinline__ bool wait_count(unsigned a, int v, int* err) {
   const long long t0 = clock64();
   for (unsigned it = 1;; ++it) {
-    if (mbar_try_wait(a, parity)) return true;
-    if ((it & 15) == 0 && (clock64() - t0 > kWaitCycles || *(volatile int*)err)) {
-      atomicOr(err, 1);
-      return false;
+    if (lds_int(a) >= v) return true;
+    if (give_up(it, t0, err)) return false;
+  }
+}
+
+// ---- the division by the pivot, off a stored reciprocal
+// FP64, r = RN(1/p): q0 = RN(x r) is within 2^-52 of x/p, one correction
+// q1 = RN(q0 + r RN(x - q0 p)) leaves the rounding of a value within 2^-103 of
+// x/p (so q1 is one of the two doubles around it), and then
+// q2 = RN(q1 + r (x - q1 p)), whose residual is exact, is x/p correctly rounded
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34, 1990, theorem on the quotient
+// from a correctly rounded reciprocal and a neighbouring quotient).  That holds
+// where nothing over- or underflows: recip() marks pivots outside
+// 2^-400..2^400 with a NaN, and a q0 outside 2^-400..2^400 (so also NaN,
+// infinities and zeros) sends the step to the plain division.
+template <class T>
+struct Recip;
+template <>
+struct Recip<double> {
+  using type = double;
+  static constexpr bool keep_pivot = true;
+  __device__ static double of(double p) {
+    const int e = (__double2hiint(p) >> 20) & 0x7FF;
+    return (unsigned)(e - (1023 - 400)) <= 800u ? 1.0 / p : __longlong_as_double(0x7FF8000000000000LL);
+  }
+  __device__ static __forceinline__ double div(double x, double p, double r, bool& bad) {
+    const double q0 = __dmul_rn(x, r);
+    const double q1 = __fma_rn(__fma_rn(-q0, p, x), r, q0);
+    const int e = (__double2hiint(q0) >> 20) & 0x7FF;
+    bad = (unsigned)(e - (1023 - 400)) > 800u;
+    return __fma_rn(__fma_rn(-q1, p, x), r, q1);
+  }
+  __device__ static __forceinline__ double slow(double x, double p, double) { return x / p; }
+};
+// FP32, r = RN64(1/p): x r in FP64 is within 2^-52 of x/p, and a quotient of
+// two 24-bit numbers is never nearer than 2^-49 to the middle of two floats
+// (an odd 25-bit middle m would need |x - m p| of at least one unit), so
+// rounding x r to float rounds x/p.  Zeros, infinities and NaNs come out as
+// the division's; only results below the normal range (coarser middles) go to
+// the plain division, whose pivot is 1/r rounded to float.
+template <>
+struct Recip<float> {
+  using type = double;
+  static constexpr bool keep_pivot = false;
+  __device__ static double of(float p) { return 1.0 / (double)p; }
+  __device__ static __forceinline__ float div(float x, float, double r, bool& bad) {
+    const float q = (float)((double)x * r);
+    bad = fabsf(q) < 1.17549435e-38f && x != 0.0f;
+    return q;
+  }
+  __device__ static __forceinline__ float slow(float x, float, double r) { return x / (float)(1.0 / r); }
+};
+
+// Bytes of one strip step's coefficients: the three bands, and in the
+// backward sweep the reciprocal of the pivot (and the pivot, FP64).
+template <bool UP, class T>
+constexpr int coef_bytes() {
+  return kStripCells * (3 * (int)sizeof(T) +
+                        (UP ? (int)sizeof(typename Recip<T>::type) + (Recip<T>::keep_pivot ? (int)sizeof(T) : 0) : 0));
+}
+
+// Where the two sweeps of one precision keep their arrays (byte offsets from
+// one allocation).
+struct WalkMem {
+  long long coef_l, coef_u, tmp, halo_l, halo_u, total;
+  long long halo_words;  // words of one sweep's hand-over buffers
+};
+template <class T>
+WalkMem walk_mem(const Walk& w) {
+  const long long steps = (long long)w.ntx * w.nty * kStrips * w.nsteps;
+  WalkMem m;
+  m.halo_words = (long long)w.ntx * w.nty * w.halo * (kTileI + kTileJ);
+  m.coef_l = 0;
+  m.coef_u = m.coef_l + steps * coef_bytes<false, T>();
+  m.tmp = m.coef_u + steps * coef_bytes<true, T>();
+  m.halo_l = m.tmp + (w.n * (long long)sizeof(T) + 255) / 256 * 256;
+  m.halo_u = m.halo_l + m.halo_words * (long long)sizeof(T);
+  m.total = m.halo_u + m.halo_words * (long long)sizeof(T);
+  return m;
+}
+
+// The natural row of walk cell (i, j, k), or -1 outside the grid.
+template <bool UP>
+__device__ __forceinline__ long long walk_row(const Walk& g, int i, int j, int k) {
+  if (i >= g.nx || j >= g.ny || (unsigned)k >= (unsigned)g.nz) return -1;
+  const long long w = i + (long long)g.nx * j + g.nxny * k;
+  return UP ? g.n - 1 - w : w;
+}
+
+// The coefficients of every strip step, from the natural-order bands: bands
+// 0 and pivots 1 outside the grid.  One thread per pair of cells along i.
+template <bool UP>
+__global__ void k_walk_pack(Walk g, Bands b, unsigned char* __restrict__ dst) {
+  const long long pairs = (long long)g.ntx * g.nty * kStrips * g.nsteps * (kStripCells / 2);
+  const double* band[3] = {UP ? b.Ui : b.Lk, UP ? b.Uj : b.Lj, UP ? b.Uk : b.Li};
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < pairs; q += (long long)gridDim.x * blockDim.x) {
+    const int pr = (int)(q % (kStripCells / 2));
+    const long long st = q / (kStripCells / 2);
+    const int lane = pr & 31, row = pr >> 5;
+    const int s = (int)(st % g.nsteps);
+    const int strip = (int)(st / g.nsteps) % kStrips, tile = (int)(st / g.nsteps) / kStrips;
+    const int ti = lane % kLanesI, tj = lane / kLanesI;
+    const int i = (tile % g.ntx) * kTileI + 2 * ti, j = (tile / g.ntx) * kTileJ + strip * kStripJ + 2 * tj + row;
+    double2* out = reinterpret_cast<double2*>(dst + st * coef_bytes<UP, double>()) + pr;
+    const long long r0 = walk_row<UP>(g, i, j, s - ti - tj), r1 = walk_row<UP>(g, i + 1, j, s - ti - tj);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      out[a * (kStripCells / 2)] = make_double2(r0 >= 0 ? band[a][r0] : 0.0, r1 >= 0 ? band[a][r1] : 0.0);
+    if (UP) {
+      const double p0 = r0 >= 0 ? b.P[r0] : 1.0, p1 = r1 >= 0 ? b.P[r1] : 1.0;
+      out[3 * (kStripCells / 2)] = make_double2(Recip<double>::of(p0), Recip<double>::of(p1));
+      out[4 * (kStripCells / 2)] = make_double2(p0, p1);
     }
   }
 }
 
-// Dynamic shared memory of the cluster walk: the boundary buffer (nsteps x
-// 32 words), the input ring (kInRing x fields x 256 words) and its mbarriers.
-template <bool UP, class T>
-constexpr size_t walk_cl_smem(int nsteps) {
-  return ((size_t)nsteps * 2 * kTile + (size_t)kInRing * walk_in_fields<UP>() * kTileThreads) * sizeof(T) +
-         kInRing * sizeof(unsigned long long);
+// FP32 coefficients: the FP64 ones rounded (bands, pivots), the reciprocal
+// in FP64 from the rounded pivot.
+template <bool UP>
+__global__ void k_walk_pack32(long long steps, const unsigned char* __restrict__ src, unsigned char* __restrict__ dst) {
+  constexpr int kP = kStripCells / 2;
+  for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < steps * kP; q += (long long)gridDim.x * blockDim.x) {
+    const int pr = (int)(q % kP);
+    const long long st = q / kP;
+    const double2* in = reinterpret_cast<const double2*>(src + st * coef_bytes<UP, double>()) + pr;
+    unsigned char* o = dst + st * coef_bytes<UP, float>();
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double2 v = in[a * kP];
+      reinterpret_cast<float2*>(o)[a * kP + pr] = make_float2((float)v.x, (float)v.y);
+    }
+    if (UP) {
+      const double2 p = in[4 * kP];
+      reinterpret_cast<double2*>(o + 3 * kP * sizeof(float2))[pr] =
+          make_double2(Recip<float>::of((float)p.x), Recip<float>::of((float)p.y));
+    }
+  }
 }
 
-template <bool UP, class T, int CX, int CY>
-__global__ void __launch_bounds__(kTileThreads + 64, 1)
-    k_walk_sweep_cl(Walk g, WalkArrays<T> b, T* in, T* wave, unsigned int* tickets, int* err) {
-  constexpr int kPre = kWalkPrefetch;
-  constexpr long long kStep = UP ? -kTileThreads : kTileThreads;
-  constexpr int kLanes = 2 * kTile;
-  constexpr int kF = walk_in_fields<UP>();
-  constexpr unsigned kRowBytes = kTileThreads * sizeof(T);
-  __shared__ T s_val[2][kTile][kTile + 1];
-  __shared__ int s_tile;
-  __shared__ volatile int s_done;  // last step the compute warps finished (the input ring's producer)
-  extern __shared__ __align__(128) unsigned char walk_cl_raw[];
-  T* s_bnd = reinterpret_cast<T*>(walk_cl_raw);                   // [step][lane]
-  T* s_in = s_bnd + (size_t)g.nsteps * kLanes;                    // [slot][field][256]
-  unsigned long long* s_mbar = reinterpret_cast<unsigned long long*>(s_in + (size_t)kInRing * kF * kTileThreads);
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
-  const int cx = rank % CX, cy = rank / CX;
-  const int nsteps = g.nsteps;
-  for (int q = threadIdx.x; q < nsteps * kLanes; q += blockDim.x) s_bnd[q] = sentinel_of<T>();
+// Shared memory of one sweep's CTA (byte offsets).
+template <bool UP, class T>
+struct WalkSmem {
+  static constexpr int kCellBytes = kStripCells * (int)sizeof(T);                 // one step's cells of a strip
+  static constexpr int coef = 0;                                                  // [strip][kDepth][coef_bytes]
+  static constexpr int in = coef + kStrips * kDepth * coef_bytes<UP, T>();        // [strip][kInRing][cells]
+  static constexpr int out = in + kStrips * kInRing * kCellBytes;                 // [strip][kOutRing][cells]
+  static constexpr int jslot = out + kStrips * kOutRing * kCellBytes;             // [strip][kSlots][16]
+  static constexpr int islot = jslot + kStrips * kSlots * kTileI * (int)sizeof(T);  // [kSlots][16]
+  static constexpr int mbar = islot + kSlots * kTileJ * (int)sizeof(T);           // [strip][kDepth / 2]
+  static constexpr int done = mbar + kStrips * kDepth / 2 * 8;                        // [strip] last finished step
+  static constexpr int outdone = done + kStrips * 4;                              // [strip] last plane written out
+  static constexpr int tile = outdone + kStrips * 4;
+  static constexpr int always = tile + 4;                                         // a counter that is never behind
+  static constexpr int total = tile + 16;
+};
+// Where a cell of a strip (column c, row r) lives among a step's cells: pairs
+// along i, lane by lane, the lanes' lower rows first.
+__device__ __forceinline__ int cell_word(int c, int r) { return (((r & 1) * 32 + (r >> 1) * kLanesI + (c >> 1)) << 1) + (c & 1); }
+
+// One triangular sweep.  UP = false: forward sweep x_i = y_i - sum_{k<dcol}
+// l_ik x_k (solveL, ILU0Preconditioner.h:181-198).  UP = true: backward sweep
+// x_i = (y_i - sum_{k>dcol} u_ik x_k) / u_ii (solveU, :200-231), in mirrored
+// coordinates.  src and dst in natural order (different vectors); hi / hj: the
+// hand-over words of every tile's last column / last row, [tile][plane][16], at
+// the sentinel before and after.
+template <bool UP, class T>
+__global__ void __launch_bounds__(kWalkWarps * 32, 1)
+    k_walk_sweep(Walk g, const unsigned char* __restrict__ coef, const T* __restrict__ src, T* __restrict__ dst,
+                 T* __restrict__ hi, T* __restrict__ hj, unsigned int* tickets, int* err) {
+  using S = WalkSmem<UP, T>;
+  using R = typename Recip<T>::type;
+  constexpr int kCoef = coef_bytes<UP, T>();
+  constexpr int kT = (int)sizeof(T);
+  extern __shared__ __align__(128) unsigned char walk_smem[];
+  const unsigned sm = smem_addr(walk_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    s_done = -1;
-    if (rank == 0) s_tile = (int)atomicAdd(tickets + (UP ? 2 : 1), 1u);
-  }
-  if (threadIdx.x == kTileThreads + 32) {
-    for (int q = 0; q < kInRing; ++q) mbar_init(smem_addr(s_mbar + q), 1);
+    sts_int(sm + S::tile, (int)atomicAdd(tickets + (UP ? 2 : 1), 1u));
+    sts_int(sm + S::always, 0x7FFFFFFF);
+    for (int w = 0; w < kStrips; ++w) {
+      sts_int(sm + S::done + 4 * w, -1);
+      sts_int(sm + S::outdone + 4 * w, -1);
+      for (int q = 0; q < kDepth / 2; ++q) mbar_init(sm + S::mbar + (w * kDepth / 2 + q) * 8, 33);
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  cl.sync();
-  const int super = *cl.map_shared_rank(&s_tile, 0);
-  const int nsx = (g.ntx + CX - 1) / CX;
-  const int tx = (super % nsx) * CX + cx, ty = (super / nsx) * CY + cy;
-  const unsigned mbar0 = smem_addr(s_mbar);
+  for (int q = threadIdx.x; q < kStrips * kInRing * kStripCells; q += blockDim.x) sts1(sm + S::in + q * kT, T(1));
+  for (int q = threadIdx.x; q < (kStrips * kTileI + kTileJ) * kSlots; q += blockDim.x)
+    sts1(sm + S::jslot + q * kT, sentinel_of<T>());
+  __syncthreads();
+  const int tile = lds_int(sm + S::tile);
+  const int tx = tile % g.ntx, ty = tile / g.ntx;
+  const int nsteps = g.nsteps, nz = g.nz;
+  // A strip without any line in the grid has nothing to do (and feeds none).
+  const int strips = min(kStrips, (g.ny - ty * kTileJ + kStripJ - 1) / kStripJ);
+  // Hand the other sweep its ticket back (it does not run concurrently).
+  if (blockIdx.x == 0 && threadIdx.x == 0) tickets[UP ? 1 : 2] = 0u;
 
-  if (tx < g.ntx && ty < g.nty) {
-    const int tile = ty * g.ntx + tx;
-    const bool copier = threadIdx.x >= kTileThreads + 32;
-    const bool poller = !copier && threadIdx.x >= kTileThreads;
-    const int lane = threadIdx.x & 31;
-    const int li = poller ? (lane < kTile ? lane : 0) : threadIdx.x % kTile;
-    const int lj = poller ? (lane < kTile ? 0 : lane - kTile) : (threadIdx.x / kTile) % kTile;
-    const int ox = UP ? g.ntx * kTile - g.nx : 0;
-    const int oy = UP ? g.nty * kTile - g.ny : 0;
-    const int oz = UP ? nsteps - g.nz - 2 * (kTile - 1) : 0;
-    auto phys = [&](long long w) { return UP ? g.nw - 1 - w : w; };
-    const int ai = tx * kTile + li;
-    const int aj = ty * kTile + lj;
-    const bool active = ai >= ox && ai < ox + g.nx && aj >= oy && aj < oy + g.ny;
-    const bool has_i = ai > ox, has_j = aj > oy;
-    const bool bnd_i = li == 0 && has_i, bnd_j = lj == 0 && has_j;
-    const int s_lo = active ? li + lj + oz : nsteps;
-    const int s_hi = active ? s_lo + g.nz : nsteps;
-    const long long tbase = (long long)tile * nsteps * kTileThreads;
+  const WarpRole me = warp_role(warp);
+  if (me.role == Role::Compute) {
+    // ---------------------------------------------------------------- compute
+    const int w = me.strip;
+    if (w >= strips) return;
+    const int ti = lane % kLanesI, tj = lane / kLanesI, d = ti + tj;
+    const int slot_i = ti == 0 && tx > 0;              // left values from islot
+    const int slot_j = tj == 0 && (w > 0 || ty > 0);   // lower values from jslot
+    const int feed_i = ti == kLanesI - 1 && tx + 1 < g.ntx;
+    const int feed_w = tj == kLanesJ - 1 && w + 1 < strips;
+    const int feed_j = tj == kLanesJ - 1 && w == kStrips - 1 && ty + 1 < g.nty;
+    // Shared addresses.  All rings are indexed by this strip's step, the same for
+    // every lane: a lane's share of plane k is at step k + d.
+    const unsigned a_coef = sm + S::coef + w * kDepth * kCoef + lane * 2 * kT;
+    const unsigned a_recip = sm + S::coef + w * kDepth * kCoef + 6 * 64 * kT + lane * 2 * (int)sizeof(R);
+    const unsigned a_mbar = sm + S::mbar + w * (kDepth / 2) * 8;
+    const unsigned a_in = sm + S::in + w * kInRing * S::kCellBytes + lane * 2 * kT;
+    const unsigned a_out = sm + S::out + w * kOutRing * S::kCellBytes + lane * 2 * kT;
+    const unsigned a_i = sm + S::islot + (w * kStripJ + 2 * tj) * kT;
+    const unsigned a_j = sm + S::jslot + (w * kSlots * kTileI + 2 * ti) * kT;
+    const unsigned a_next = a_j + kSlots * kTileI * kT;
+    const unsigned a_done = sm + S::done + 4 * w, a_outdone = sm + S::outdone + 4 * w;
+    const unsigned a_room = sm + (w + 1 < strips ? S::done + 4 * (w + 1) : S::always);
+    T* p_hi = hi + ((long long)tile * g.halo + kSkew - d) * kTileJ + w * kStripJ + 2 * tj;
+    T* p_hj = hj + ((long long)tile * g.halo + kSkew - d) * kTileI + 2 * ti;
 
-    if (copier) {
-      // Lane 0 issues each step's bulk copies once its slot is free.
+    struct In {
+      T y[4], a[3][4], p[4];
+      R r[4];
+    };
+    // Ring positions of the current pair of steps; odd steps are an immediate
+    // offset further (the rings have even sizes).
+    unsigned f_coef = 0, f_in = 0, o_out = 0;
+    auto fetch = [&](In& c, unsigned off_coef, unsigned off_in) {
+      const unsigned a = a_coef + f_coef + off_coef, y = a_in + f_in + off_in;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        ldw2(y + h * 64 * kT, c.y[2 * h], c.y[2 * h + 1]);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) ldw2(a + (b * 2 + h) * 64 * kT, c.a[b][2 * h], c.a[b][2 * h + 1]);
+        if constexpr (UP) {
+          ldw2(a_recip + f_coef + off_coef + h * 64 * (int)sizeof(R), c.r[2 * h], c.r[2 * h + 1]);
+          if constexpr (Recip<T>::keep_pivot) ldw2(a + (8 + h) * 64 * kT, c.p[2 * h], c.p[2 * h + 1]);
+        }
+      }
+    };
+
+    // What a step waits for -- its hand-over words and, in an odd step, the
+    // inputs of the pair after it -- is read and voted on during the step before
+    // it, so that in the steady state no load, vote or branch stands between a
+    // step's arithmetic and the previous one's.
+    T v[4] = {T(0), T(0), T(0), T(0)};             // the previous step's cells
+    T l0 = T(0), l1 = T(0), b0 = T(0), b1 = T(0);  // the next step's hand-over words
+    unsigned m_next = a_mbar, m_par = 0;           // the next pair's mbarrier
+    bool ok = true, go = false;
+    auto look = [&](int s, auto odd) {  // the state of what step s waits for
+      const unsigned so = (unsigned)(s & (kSlots - 1)) * kTileI * kT;
+      lds2_if(slot_i, a_i + so, l0, l1);
+      lds2_if(slot_j, a_j + so, b0, b1);
+      if constexpr (decltype(odd)::value) ok = mbar_test(m_next, m_par) || s + 1 >= nsteps;
+    };
+    auto ready = [&]() { return ok && !(waiting(l0) | waiting(l1) | waiting(b0) | waiting(b1)); };
+    auto step = [&](int s, In& c, In& nxt, auto odd) {
+      constexpr bool kOdd = decltype(odd)::value;
+      using Odd = std::bool_constant<kOdd>;
+      using NotOdd = std::bool_constant<!kOdd>;
+      const unsigned so = (unsigned)(s & (kSlots - 1)) * kTileI * kT;
+      const T sl0 = __shfl_up_sync(0xffffffffu, v[1], 1), sl1 = __shfl_up_sync(0xffffffffu, v[3], 1);
+      const T sb0 = __shfl_up_sync(0xffffffffu, v[2], kLanesI), sb1 = __shfl_up_sync(0xffffffffu, v[3], kLanesI);
+      if (!go) {
+        const long long t0 = clock64();
+        for (unsigned it = 1;; ++it) {
+          look(s, Odd());
+          if (__all_sync(0xffffffffu, ready())) break;
+          if (__any_sync(0xffffffffu, give_up(it, t0, err))) {  // quiet NaNs from here on
+            l0 = l1 = b0 = b1 = quiet_nan<T>();
+            break;
+          }
+        }
+      }
+      const T xl0 = ti > 0 ? sl0 : l0, xl1 = ti > 0 ? sl1 : l1, xb0 = tj > 0 ? sb0 : b0, xb1 = tj > 0 ? sb1 : b1;
+      if constexpr (!kOdd) {
+        fetch(nxt, kCoef, S::kCellBytes);
+      } else {  // on to the next pair
+        f_coef += 2 * kCoef;
+        f_in += 2 * S::kCellBytes;
+        const bool wrap = f_coef == kDepth * kCoef;
+        f_coef = wrap ? 0u : f_coef;
+        m_next = wrap ? a_mbar + 8 : m_next + 8;
+        f_in = f_in == kInRing * S::kCellBytes ? 0u : f_in;
+        fetch(nxt, 0, 0);
+        if (m_next == a_mbar + kDepth / 2 * 8) {
+          m_next = a_mbar;
+          m_par ^= 1u;
+        }
+      }
+      sts2_if(slot_i, a_i + so, sentinel_of<T>(), sentinel_of<T>());
+      sts2_if(slot_j, a_j + so, sentinel_of<T>(), sentinel_of<T>());
+      look(s + 1, NotOdd());
+      if constexpr (!UP) {  // columns ascending: -k, -j, -i
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = mul_sub_rn(c.a[0][q], v[q], c.y[q]);
+        v[0] = mul_sub_rn(c.a[2][0], xl0, mul_sub_rn(c.a[1][0], xb0, v[0]));
+        v[1] = mul_sub_rn(c.a[2][1], v[0], mul_sub_rn(c.a[1][1], xb1, v[1]));
+        v[2] = mul_sub_rn(c.a[2][2], xl1, mul_sub_rn(c.a[1][2], v[0], v[2]));
+        v[3] = mul_sub_rn(c.a[2][3], v[2], mul_sub_rn(c.a[1][3], v[1], v[3]));
+      } else {  // columns ascending: +i, +j, +k
+        T m[4], n[4];
+        bool bad[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) m[q] = mul_rn(c.a[2][q], v[q]);
+        auto num = [&](int q, T xi, T xj) {
+          return sub_rn(mul_sub_rn(c.a[1][q], xj, mul_sub_rn(c.a[0][q], xi, c.y[q])), m[q]);
+        };
+        n[0] = Recip<T>::div(num(0, xl0, xb0), c.p[0], c.r[0], bad[0]);
+        n[1] = Recip<T>::div(num(1, n[0], xb1), c.p[1], c.r[1], bad[1]);
+        n[2] = Recip<T>::div(num(2, xl1, n[0]), c.p[2], c.r[2], bad[2]);
+        n[3] = Recip<T>::div(num(3, n[2], n[1]), c.p[3], c.r[3], bad[3]);
+        if (__any_sync(0xffffffffu, bad[0] | bad[1] | bad[2] | bad[3])) {  // the step again, with plain divisions
+          n[0] = Recip<T>::slow(num(0, xl0, xb0), c.p[0], c.r[0]);
+          n[1] = Recip<T>::slow(num(1, n[0], xb1), c.p[1], c.r[1]);
+          n[2] = Recip<T>::slow(num(2, xl1, n[0]), c.p[2], c.r[2]);
+          n[3] = Recip<T>::slow(num(3, n[2], n[1]), c.p[3], c.r[3]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = n[q];
+      }
+      // (results of arithmetic are never the sentinel, a signalling NaN)
+      st_flag2_if(feed_i, p_hi + (kOdd ? kTileJ : 0), v[1], v[3]);
+      st_flag2_if(feed_j, p_hj + (kOdd ? kTileI : 0), v[2], v[3]);
+      // the next strip's step: this one less the lanes between (before its first step there is none)
+      const int fs = s - (kLanesJ - 1);
+      sts2_if(fs >= 0 ? feed_w : 0, a_next + (unsigned)(fs & (kSlots - 1)) * kTileI * kT, v[2], v[3]);
+      stw2(a_out + o_out + (kOdd ? S::kCellBytes : 0), v[0], v[1]);
+      stw2(a_out + o_out + (kOdd ? S::kCellBytes : 0) + 64 * kT, v[2], v[3]);
+      go = __all_sync(0xffffffffu, ready());
+      if constexpr (kOdd) {
+        p_hi += 2 * kTileJ;
+        p_hj += 2 * kTileI;
+        o_out = o_out + 2 * S::kCellBytes == kOutRing * S::kCellBytes ? 0u : o_out + 2 * S::kCellBytes;
+        sts_int_if(lane == 0, a_done, s);
+      }
+    };
+    In c0, c1;
+    if (!mbar_test(m_next, 0)) mbar_wait(m_next, 0, err);
+    m_next += 8;
+    fetch(c0, 0, 0);
+    for (int s = 0; s < nsteps; s += 2) {  // two buffers of inputs, no moves between them
+      if ((s & 7) == 0) {
+        // room for the next eight steps: in the ring of output cells (step s + 7
+        // overwrites step s + 7 - kOutRing, whose cells are of planes up to that
+        // number) and in the next strip's slots (step s + 4 at most)
+        if (lds_int(a_outdone) < s + 7 - kOutRing) wait_count(a_outdone, min(s + 7 - kOutRing, nz - 1), err);
+        if (lds_int(a_room) < s + 4 - kSlots) wait_count(a_room, s + 4 - kSlots, err);
+        __syncwarp();
+      }
+      step(s, c0, c1, std::false_type());
+      step(s + 1, c1, c0, std::true_type());
+    }
+    // the next strip's last steps have no values to wait for
+    if (w + 1 < strips) {
+      wait_count(a_room, nsteps - 1 - kSlots, err);
+      for (int t = nsteps - (kLanesJ - 1); t < nsteps; ++t)
+        sts2_if(feed_w, a_next + (unsigned)(t & (kSlots - 1)) * kTileI * kT, T(1), T(1));
+    }
+  } else if (me.role == Role::Poll) {
+    // ---------------------------------------------------------------- hand-overs from other tiles
+    // Warps 0 and 2: the columns of the tile's first row; 1 and 3: the rows of its
+    // first column.  A side's four half-warps take the steps in turn, a word a
+    // lane, kPollDepth of them at once; a step whose plane is outside the grid
+    // gets a 1 (its coefficients are 0).  Several warps with little to do in a
+    // round, because a round is a trip to L2 and every instruction in it is
+    // latency on the next tile's critical path.
+    const bool jside = (me.part & 1) == 0;
+    const int q = lane & 15;  // column, resp. row
+    const int w = jside ? 0 : q / kStripJ;
+    const bool need = jside ? ty > 0 : tx > 0 && w < strips;
+    const int d = jside ? q / 2 : q % kStripJ / 2;  // the using lane's skew: plane k is its step k + d
+    T* p = (jside ? hj + (long long)(tile - g.ntx) * g.halo * kTileI : hi + (long long)(tile - 1) * g.halo * kTileJ) + q +
+           (kSkew - d) * 16;
+    const unsigned slot = sm + (jside ? S::jslot : S::islot) + q * kT;
+    const unsigned a_done = sm + S::done + 4 * w;
+    const int phase = (me.part >> 1) * 2 + (lane >> 4);
+    int x[kPollDepth];  // the steps this lane waits for, each on its own
+#pragma unroll
+    for (int u = 0; u < kPollDepth; ++u) x[u] = need ? phase + 4 * u : nsteps;
+    unsigned it = 0;
+    long long t0 = clock64();
+    for (;;) {
+      const int lim = min(nsteps, lds_int(a_done) + kSlots + 1);  // a slot is free once its previous step is done
+      T v[kPollDepth];
+#pragma unroll
+      for (int u = 0; u < kPollDepth; ++u) {
+        v[u] = T(1);
+        if (x[u] < lim && (unsigned)(x[u] - d) < (unsigned)nz) v[u] = ld_relaxed(p + (long long)x[u] * 16);
+      }
+      bool some = false, left = false;
+#pragma unroll
+      for (int u = 0; u < kPollDepth; ++u) {
+        if (x[u] < lim && !waiting(v[u])) {
+          sts1(slot + (unsigned)(x[u] & (kSlots - 1)) * 16 * kT, v[u]);
+          p[(long long)x[u] * 16] = sentinel_of<T>();  // ready for the next application
+          x[u] += 4 * kPollDepth;
+          some = true;
+        }
+        left |= x[u] < nsteps;
+      }
+      if (!__any_sync(0xffffffffu, left)) break;
+      if (__any_sync(0xffffffffu, some)) {
+        it = 0;
+      } else if ((++it & 15) == 0) {  // (the same count in every lane)
+        if (it == 16) t0 = clock64();
+        if (__any_sync(0xffffffffu, give_up(0, t0, err))) break;  // the compute warps' own waits end the same way
+      }
+    }
+  } else if (me.role == Role::Load) {
+    // ---------------------------------------------------------------- inputs
+    // Two steps' coefficients (one bulk copy) and two planes of src, up to kDepth
+    // steps ahead of the compute warp, on one mbarrier; every other pair of
+    // steps.  A lane copies column lane & 15 of rows (lane >> 4) + 2 q, each
+    // word to its step's cells.  Words outside the grid are left at 1.
+    const int w = me.strip, first = me.part;
+    if (w >= strips) return;
+    const unsigned char* cf = coef + (((long long)tile * kStrips + w) * nsteps + 2 * first) * kCoef;
+    const unsigned a_done = sm + S::done + 4 * w, a_mbar = sm + S::mbar + w * (kDepth / 2) * 8;
+    const unsigned a_cf = sm + S::coef + w * kDepth * kCoef;
+    const unsigned ring = sm + S::in + w * kInRing * S::kCellBytes, ring_end = ring + kInRing * S::kCellBytes;
+    const int col = lane & 15, row0 = lane >> 4;
+    const long long dz = UP ? -g.nxny : g.nxny;
+    const T* from[4];
+    unsigned to[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long r = walk_row<UP>(g, tx * kTileI + col, ty * kTileJ + w * kStripJ + row0 + 2 * q, 0);
+      in[q] = r >= 0;
+      from[q] = src + (in[q] ? r + 2 * first * dz : 0);
+      to[q] = ring + (unsigned)(2 * first + (col >> 1) + q) * S::kCellBytes + cell_word(col, row0 + 2 * q) * kT;
+    }
+    int s = 2 * first, seen = -1;
+    unsigned slot = first;
+    for (; s < nsteps; s += 4) {
+      if (seen < s + 1 - kDepth) {
+        seen = lds_int(a_done);
+        if (seen < s + 1 - kDepth) {
+          if (!wait_count(a_done, s + 1 - kDepth, err)) break;
+          seen = s + 1 - kDepth;
+        }
+        __syncwarp();
+      }
+      const unsigned mb = a_mbar + slot * 8;
       if (lane == 0) {
-        const T* src[kF];
-        src[0] = in;
-        src[1] = UP ? b.Ui : b.Lk;
-        src[2] = UP ? b.Uj : b.Lj;
-        src[3] = UP ? b.Uk : b.Li;
-        if constexpr (kF == 5) src[4] = b.P;
-        // first word of step t's 256 in the arrays (the U walk reads its block reversed)
-        auto row0 = [&](int t) { return UP ? g.nw - kTileThreads - tbase - (long long)t * kTileThreads
-                                           : tbase + (long long)t * kTileThreads; };
-        const unsigned in0 = smem_addr(s_in);
-        int t_issue = 0;  // next step whose inputs are copied
-        long long t_last = clock64();
-        while (t_issue < nsteps) {
-          const int lim = min(nsteps, s_done + kInRing + 1);
-          if (t_issue < lim) {
-            for (; t_issue < lim; ++t_issue) {
-              const int q = t_issue % kInRing;
-              const unsigned mb = mbar0 + q * 8;
-              mbar_expect_tx(mb, kF * kRowBytes);
-              const long long w0 = row0(t_issue);
-#pragma unroll
-              for (int f = 0; f < kF; ++f) bulk_load(in0 + (q * kF + f) * kRowBytes, src[f] + w0, kRowBytes, mb);
-            }
-            t_last = clock64();
-          } else {
-            __nanosleep(100);  // waiting for the compute warps to free a slot
-            if (clock64() - t_last > kWaitCycles || *(volatile int*)err) {
-              atomicOr(err, 1);
-              break;
-            }
-          }
-        }
-        // Copies still in flight land before the CTA may leave (bounded by
-        // time only: also after a failure, whatever the error flag says).
-        for (int x = max(0, t_issue - kInRing); x < t_issue; ++x)
-          if (!mbar_drain(mbar0 + (x % kInRing) * 8, (x / kInRing) & 1)) break;
+        mbar_expect_tx(mb, 2 * kCoef);
+        bulk_load(a_cf + slot * 2 * kCoef, cf, 2 * kCoef, mb);
       }
-    } else if (poller) {
-      // The sides whose upstream tile is in another cluster: global memory.
-      const bool need = lane < kTile ? (bnd_j && cy == 0) : (bnd_i && cx == 0);
-      if (__any_sync(0xffffffffu, need)) {
-        const long long w_nb =
-            lane < kTile ? phys(tbase - (long long)g.ntx * nsteps * kTileThreads + 15 * kTileThreads + 15 * kTile + li)
-                         : phys(tbase - (long long)nsteps * kTileThreads + 15 * kTileThreads + lj * kTile + 15);
-        const T* p_nb = wave + (need ? w_nb : 0);
-        volatile T* slots = s_bnd + lane;
-        int t = need ? s_lo : s_hi;  // next step this lane hands over
-        long long t_last = clock64();
-        bool failed = false;
-        while (__any_sync(0xffffffffu, t < s_hi)) {
-          T v[kPollDepth];
 #pragma unroll
-          for (int d = 0; d < kPollDepth; ++d) {
-            const int st = t + d;
-            v[d] = (st < s_hi && !failed) ? ld_relaxed(p_nb + (long long)st * kStep) : sentinel_of<T>();
-          }
-          int adv = 0;  // leading steps whose values arrived
+      for (int u = 0; u < 2; ++u) {
+        if (s + u < nz) {
 #pragma unroll
-          for (int d = 0; d < kPollDepth; ++d) {
-            const int st = t + d;
-            if (adv == d && st < s_hi && (failed || !is_sentinel(v[d]))) {
-              slots[st * kLanes] = failed ? quiet_nan<T>() : v[d];
-              ++adv;
-            }
-          }
-          t += adv;
-          if (__any_sync(0xffffffffu, adv > 0)) {
-            t_last = clock64();
-          } else {  // (warp-uniform) give up after the bound: quiet NaNs from here on
-            const bool stop = __any_sync(0xffffffffu, clock64() - t_last > kWaitCycles || *(volatile int*)err != 0);
-            if (stop && !failed) {
-              if (lane == 0) atomicOr(err, 1);
-              failed = true;
-            }
+          for (int q = 0; q < 4; ++q) {
+            if (in[q]) copy_word<kT>(to[q], from[q] + u * dz);
+            to[q] += S::kCellBytes;
+            to[q] -= to[q] >= ring_end ? kInRing * S::kCellBytes : 0;
           }
         }
       }
-    } else {
-      // In-cluster consumers of this tile's last lines.
-      const bool feed_i = active && li == kTile - 1 && cx < CX - 1 && tx + 1 < g.ntx;
-      const bool feed_j = active && lj == kTile - 1 && cy < CY - 1 && ty + 1 < g.nty;
-      // 32-bit shared addresses of this thread's slots at step 0: own (read)
-      // and the consumers' (written); a step is kLanes words further.
-      const unsigned a_j = smem_addr(s_bnd + li), a_i = smem_addr(s_bnd + kTile + lj);
-      const unsigned r_i = feed_i ? peer_addr(a_i, rank + 1) : 0u;  // consumer line (0, lj)
-      const unsigned r_j = feed_j ? peer_addr(a_j, rank + CX) : 0u;  // consumer line (li, 0)
-      constexpr unsigned kSlotStep = kLanes * sizeof(T);
-
-      const long long w_own = phys(tbase + threadIdx.x);
-      T* p_in = in + w_own;
-      T* p_out = wave + w_own;
-      // this thread's word of each input row in the ring (the U walk's rows are reversed)
-      const unsigned a_in = smem_addr(s_in) + (UP ? kTileThreads - 1 - threadIdx.x : threadIdx.x) * sizeof(T);
-
-      // Step s's inputs, once their slot's copies have landed.
-      int f_slot = 0;
-      unsigned f_par = 0;  // slot and phase parity of the next step to fetch
-      auto fetch = [&](int s, PreW<T>& c) {
-        (void)s;
-        const int q = f_slot;
-        const unsigned mb = mbar0 + q * 8, par = f_par;
-        if (++f_slot == kInRing) {
-          f_slot = 0;
-          f_par ^= 1u;
-        }
-        if (!mbar_try_wait(mb, par)) mbar_wait(mb, par, err);
-        const unsigned a = a_in + q * kF * kRowBytes;
-        c.y = ld_in(a, T());
-        c.a1 = ld_in(a + kRowBytes, T());
-        c.a2 = ld_in(a + 2 * kRowBytes, T());
-        c.a3 = ld_in(a + 3 * kRowBytes, T());
-        if constexpr (kF == 5) c.piv = ld_in(a + 4 * kRowBytes, T());
-      };
-
-      T own = 0;
-      PreW<T> nxt{0, 0, 0, 0, 0};
-      fetch(0, nxt);
-      for (int s0 = 0; s0 < nsteps; s0 += kPre) {
+      copy_arrive(mb);
 #pragma unroll
-        for (int u = 0; u < kPre; ++u) {
-          const int s = s0 + u;
-          const long long o = (long long)s * kStep;
-          const PreW<T> c = nxt;
-          T val = 0;
-          if (s >= s_lo && s < s_hi) {
-            const T* prev = &s_val[(s + 1) & 1][0][0];
-            T vi = 0, vj = 0;
-            if (bnd_j) vj = take_slot<T>(a_j + s * kSlotStep, err);
-            if (bnd_i) vi = take_slot<T>(a_i + s * kSlotStep, err);
-            if (has_j && lj > 0) vj = prev[(lj - 1) * (kTile + 1) + li];
-            if (has_i && li > 0) vi = prev[lj * (kTile + 1) + li - 1];
-            const bool has_k = s > s_lo;
-            T acc = c.y;
-            if (!UP) {  // columns ascending: -k, -j, -i
-              if (has_k) acc = mul_sub_rn(c.a1, own, acc);
-              if (has_j) acc = mul_sub_rn(c.a2, vj, acc);
-              if (has_i) acc = mul_sub_rn(c.a3, vi, acc);
-              val = acc;
-            } else {  // columns ascending: +i, +j, +k
-              if (has_i) acc = mul_sub_rn(c.a1, vi, acc);
-              if (has_j) acc = mul_sub_rn(c.a2, vj, acc);
-              if (has_k) acc = mul_sub_rn(c.a3, own, acc);
-              p_in[o] = sentinel_of<T>();
-              val = acc / c.piv;
-            }
-            const T out = not_sentinel(val);
-            st_flag(p_out + o, out);
-            // the consumer's step: this one less the 15 lines between
-            const int cs = s - (kTile - 1);
-            if (feed_i) st_peer(r_i + cs * kSlotStep, out);
-            if (feed_j) st_peer(r_j + cs * kSlotStep, out);
-            own = val;
-          }
-          s_val[s & 1][lj][li] = val;
-          // the next step's inputs, before the barrier (this step's slot is
-          // handed back to the producer once s_done passes it)
-          if (s + 1 < nsteps) fetch(s + 1, nxt);
-          compute_bar();
-          // (no fence: the only reader, the copy warp, reuses the slot of a
-          // step whose words every thread read into registers before the
-          // barrier; a fence here cost ~13 us per application at 192^3)
-          if (threadIdx.x == 0) s_done = s;
+      for (int q = 0; q < 4; ++q) {
+        from[q] += 4 * dz;
+        to[q] += 2 * S::kCellBytes;
+        to[q] -= to[q] >= ring_end ? kInRing * S::kCellBytes : 0;
+      }
+      cf += 4 * kCoef;
+      slot = slot + 2 >= kDepth / 2 ? first : slot + 2;
+    }
+    // Copies in flight land before the CTA may leave (also after a failure).
+    copy_wait_all();
+    __syncwarp();
+    if (lane == 0)
+      for (int x = s - kDepth; x < s; x += 4)
+        if (x >= 0 && !mbar_drain(a_mbar + (x % kDepth) / 2 * 8, (x / kDepth) & 1)) break;
+  } else if (me.role == Role::Store) {
+    // ---------------------------------------------------------------- outputs
+    // Two planes at a time, once the second one's last lane's step is done.
+    const int w = me.strip;
+    if (w >= strips) return;
+    const int col = lane & 15, row0 = lane >> 4;
+    const unsigned ring = sm + S::out + w * kOutRing * S::kCellBytes, ring_end = ring + kOutRing * S::kCellBytes;
+    const unsigned a_done = sm + S::done + 4 * w, a_outdone = sm + S::outdone + 4 * w;
+    const long long dz = UP ? -g.nxny : g.nxny;
+    T* to[4];
+    unsigned from[4];
+    bool in[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const long long r = walk_row<UP>(g, tx * kTileI + col, ty * kTileJ + w * kStripJ + row0 + 2 * q, 0);
+      in[q] = r >= 0;
+      to[q] = dst + (in[q] ? r : 0);
+      from[q] = ring + (unsigned)((col >> 1) + q) * S::kCellBytes + cell_word(col, row0 + 2 * q) * kT;
+    }
+    int seen = -1;
+    for (int k = 0; k < nz; k += 2) {
+      const int last = min(k + 1 + kSkew, nsteps - 1);
+      if (seen < last) {
+        seen = lds_int(a_done);
+        if (seen < last) {
+          if (!wait_count(a_done, last, err)) return;
+          seen = last;
         }
+        __syncwarp();
+      }
+      T v[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          lds1(from[q], v[u][q]);
+          from[q] += S::kCellBytes;
+          from[q] -= from[q] >= ring_end ? kOutRing * S::kCellBytes : 0;
+        }
+      sts_int_if(lane == 0, a_outdone, k + 1);  // (read: the slots may be written again)
+      const bool two = k + 1 < nz;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (in[q]) *to[q] = v[0][q];
+        if (in[q] && two) *(to[q] + dz) = v[1][q];
+        to[q] += 2 * dz;
       }
     }
   }
-  // Hand the other sweep its ticket back (it does not run concurrently).
-  if (blockIdx.x == 0 && threadIdx.x == 0) tickets[UP ? 1 : 2] = 0u;
-  cl.sync();
 }
 
 Geom geom_of(const Ilu0Data& d) {
@@ -1029,11 +954,12 @@ Walk walk_of(const Ilu0Data& d) {
   w.nx = g.nx;
   w.ny = g.ny;
   w.nz = g.nz;
-  w.ntx = g.ntx;
-  w.nty = g.nty;
-  w.nsteps = (g.nz + 2 * (kTile - 1) + kWalkPrefetch - 1) / kWalkPrefetch * kWalkPrefetch;
+  w.ntx = (g.nx + kTileI - 1) / kTileI;
+  w.nty = (g.ny + kTileJ - 1) / kTileJ;
+  w.nsteps = (g.nz + kSkew + 1) / 2 * 2;
+  w.halo = w.nsteps + kSkew;
   w.nxny = g.nxny;
-  w.nw = (long long)g.ntx * g.nty * w.nsteps * kTileThreads;
+  w.n = g.nxny * g.nz;
   return w;
 }
 
@@ -1042,107 +968,43 @@ Bands bands_of(double* p, int n) {
   return Bands{p, p + m, p + 2 * m, p + 3 * m, p + 4 * m, p + 5 * m, p + 6 * m, p + 7 * m};
 }
 
-// d_walk (and d_walk32): Lk Lj Li Ui Uj Uk P | y | L-walk output | U-walk output
-enum { kWalkBands = 7, kWalkY = 7, kWalkL = 8, kWalkU = 9, kWalkArrays = 10 };
-
-template <class T>
-T* walk_array(T* base, const Ilu0Data& d, int a) {
-  return base + (size_t)a * (size_t)d.walk_n;
-}
-
-template <class T>
-WalkArrays<T> walk_bands(T* base, const Ilu0Data& d) {
-  return WalkArrays<T>{walk_array(base, d, 0), walk_array(base, d, 1), walk_array(base, d, 2),
-                       walk_array(base, d, 3), walk_array(base, d, 4), walk_array(base, d, 5),
-                       walk_array(base, d, 6)};
-}
-
 int wave_grid(ab2_context* ctx, int ntiles) { return std::max(1, std::min(ntiles, ctx->num_sms * 2)); }
-
-// The cluster walk: 2 x 2 tiles per cluster.  Measured at 192^3 (one ILU(0)
-// application, B200): 2 x 2 0.581 ms, 2 x 4 0.588, 4 x 2 0.646, 4 x 4 0.642,
-// against 0.609 for the single-CTA walk.  With one CTA an SM (the walk's
-// shared memory), a GPC holds fewer large clusters than its SMs allow CTAs,
-// and the remaining clusters start late.
-constexpr int kClX = 2, kClY = 2;
-// Its buffers live in shared memory: up to this many bytes (nz up to ~350 in
-// FP64); longer walks take the single-CTA walk.
-constexpr size_t kWalkClSmemMax = 216 * 1024;
-
-template <bool UP, class T>
-cudaLaunchConfig_t walk_cl_config(cudaStream_t stream, const Walk& w, cudaLaunchAttribute* attr) {
-  const int nsx = (w.ntx + kClX - 1) / kClX, nsy = (w.nty + kClY - 1) / kClY;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kClX * kClY;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(nsx * nsy * kClX * kClY));
-  cfg.blockDim = dim3(kTileThreads + 64);
-  cfg.dynamicSmemBytes = walk_cl_smem<UP, T>(w.nsteps);
-  cfg.stream = stream;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cfg;
-}
-
-// Whether the device runs the cluster walk at all: both sweeps, at the
-// shared-memory cap, asked once per device and word size (the kernels'
-// shared-memory limit is raised to the cap on the way, so that no set-up can
-// lower it under another factor's walk).
-template <class T>
-bool walk_cl_device_ok(ab2_context* ctx) {
-  static std::atomic<int> ok[64];  // 0: not asked, 1: yes, 2: no
-  const int dev = ctx->device;
-  if (dev >= 0 && dev < 64 && ok[dev].load() != 0) return ok[dev].load() == 1;
-  bool fits = true;
-  Walk w{};
-  w.ntx = w.nty = kClX * kClY;
-  cudaLaunchAttribute attr[1];
-  for (int up = 0; up < 2 && fits; ++up) {
-    const void* k = up ? (const void*)k_walk_sweep_cl<true, T, kClX, kClY> : (const void*)k_walk_sweep_cl<false, T, kClX, kClY>;
-    AB2_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWalkClSmemMax));
-    cudaLaunchConfig_t cfg = up ? walk_cl_config<true, T>(nullptr, w, attr) : walk_cl_config<false, T>(nullptr, w, attr);
-    cfg.dynamicSmemBytes = kWalkClSmemMax;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
-      (void)cudaGetLastError();
-      fits = false;
-    }
-  }
-  if (dev >= 0 && dev < 64) ok[dev].store(fits ? 1 : 2);
-  return fits;
-}
-
-// Whether this factor's walk can take the cluster walk (both word sizes: the
-// mixed-precision solvers run the FP32 copy on the same schedule).
-bool walk_cl_possible(ab2_context* ctx, const Walk& w) {
-  const bool size_ok = walk_cl_smem<true, double>(w.nsteps) <= kWalkClSmemMax &&
-                       walk_cl_smem<false, double>(w.nsteps) <= kWalkClSmemMax;
-  return size_ok && walk_cl_device_ok<double>(ctx) && walk_cl_device_ok<float>(ctx);
-}
-
-template <bool UP, class T>
-void launch_walk_cl(ab2_context* ctx, const Walk& w, const WalkArrays<T>& b, T* in, T* wave, unsigned int* tickets,
-                    int* err) {
-  cudaLaunchAttribute attr[1];
-  const cudaLaunchConfig_t cfg = walk_cl_config<UP, T>(ctx->stream, w, attr);
-  AB2_CUDA(cudaLaunchKernelEx(&cfg, k_walk_sweep_cl<UP, T, kClX, kClY>, w, b, in, wave, tickets, err));
-}
-
-// One sweep (UP: the backward one) on the factor's walk.
-template <bool UP, class T>
-void walk_sweep(ab2_context* ctx, const Ilu0Data& d, const Walk& w, const WalkArrays<T>& b, T* in, T* wave) {
-  if (d.walk_cluster)
-    launch_walk_cl<UP, T>(ctx, w, b, in, wave, d.d_tile_tickets, d.d_err);
-  else
-    k_walk_sweep<UP, T><<<wave_grid(ctx, w.ntx * w.nty), kTileThreads + 32, 0, ctx->stream>>>(
-        w, b, in, wave, d.d_tile_tickets, d.d_err);
-  check_launch(ctx, UP ? "walk_usweep" : "walk_lsweep");
-}
 
 int bulk_grid(ab2_context* ctx, long long n) {
   return (int)std::max(1LL, std::min((n + kThreads - 1) / kThreads, (long long)ctx->num_sms * 16));
+}
+
+template <class T>
+void set_walk_smem() {
+  AB2_CUDA(cudaFuncSetAttribute(k_walk_sweep<false, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                WalkSmem<false, T>::total));
+  AB2_CUDA(cudaFuncSetAttribute(k_walk_sweep<true, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                WalkSmem<true, T>::total));
+}
+
+// One sweep (UP: the backward one); base: the precision's arrays.
+template <bool UP, class T>
+void walk_sweep(ab2_context* ctx, const Ilu0Data& d, const Walk& w, unsigned char* base, const T* src, T* dst) {
+  const WalkMem m = walk_mem<T>(w);
+  T* hi = reinterpret_cast<T*>(base + (UP ? m.halo_u : m.halo_l));
+  T* hj = hi + (long long)w.ntx * w.nty * w.halo * kTileJ;
+  k_walk_sweep<UP, T><<<w.ntx * w.nty, kWalkWarps * 32, WalkSmem<UP, T>::total, ctx->stream>>>(
+      w, base + (UP ? m.coef_u : m.coef_l), src, dst, hi, hj, d.d_tile_tickets, d.d_err);
+  check_launch(ctx, UP ? "walk_usweep" : "walk_lsweep");
+}
+
+// The hand-over words of both sweeps at the sentinel.
+void fill_halo(ab2_context* ctx, const Walk& w, double* base) {
+  const WalkMem m = walk_mem<double>(w);
+  k_fill_bits<<<bulk_grid(ctx, 2 * m.halo_words), kThreads, 0, ctx->stream>>>(2 * m.halo_words, kSentinel,
+                                                                              base + m.halo_l / 8);
+  check_launch(ctx, "walk_fill");
+}
+void fill_halo(ab2_context* ctx, const Walk& w, float* base) {
+  const WalkMem m = walk_mem<float>(w);
+  k_fill_bits32<<<bulk_grid(ctx, 2 * m.halo_words), kThreads, 0, ctx->stream>>>(2 * m.halo_words, kSentinel32,
+                                                                                base + m.halo_l / 4);
+  check_launch(ctx, "walk_fill32");
 }
 
 }  // namespace
@@ -1180,26 +1042,24 @@ bool ilu_stencil_setup(ab2_context* ctx, const ab2_matrix* A, Ilu0Data& d, bool 
     check_launch(ctx, "stencil_pack");
   }
 
-  // The sweeps' arrays in walk order.
+  // The sweeps' arrays.
   const Walk w = walk_of(d);
-  d.walk_n = w.nw;
-  d.d_walk = dev_alloc<double>(ctx, (size_t)kWalkArrays * (size_t)w.nw);
-  const double* nat[kWalkBands] = {b.Lk, b.Lj, b.Li, b.Ui, b.Uj, b.Uk, b.P};
-  for (int a = 0; a < kWalkBands; ++a) {
-    k_walk_gather<<<bulk_grid(ctx, w.nw), kThreads, 0, ctx->stream>>>(w, nat[a], walk_array(d.d_walk, d, a));
-    check_launch(ctx, "walk_gather");
-  }
-  AB2_CUDA(cudaMemsetAsync(walk_array(d.d_walk, d, kWalkY), 0, sizeof(double) * (size_t)w.nw, ctx->stream));
-  k_fill_bits<<<bulk_grid(ctx, 2 * w.nw), kThreads, 0, ctx->stream>>>(2 * w.nw, kSentinel,
-                                                                      walk_array(d.d_walk, d, kWalkL));
-  check_launch(ctx, "walk_fill");
+  const WalkMem m = walk_mem<double>(w);
+  d.d_walk = dev_alloc<double>(ctx, (size_t)(m.total + 7) / 8);
+  unsigned char* base = reinterpret_cast<unsigned char*>(d.d_walk);
+  const long long pairs = (long long)w.ntx * w.nty * kStrips * w.nsteps * (kStripCells / 2);
+  k_walk_pack<false><<<bulk_grid(ctx, pairs), kThreads, 0, ctx->stream>>>(w, b, base + m.coef_l);
+  check_launch(ctx, "walk_pack");
+  k_walk_pack<true><<<bulk_grid(ctx, pairs), kThreads, 0, ctx->stream>>>(w, b, base + m.coef_u);
+  check_launch(ctx, "walk_pack");
+  fill_halo(ctx, w, d.d_walk);
   AB2_CUDA(cudaStreamSynchronize(ctx->stream));
   dev_free(ctx, d.d_bands);
   d.d_bands = nullptr;
-  set_transpose_smem<double>();
-  d.walk_cluster = schedule != AB2_ILU_STENCIL && walk_cl_possible(ctx, w);
+  set_walk_smem<double>();
+  d.walk_cluster = schedule != AB2_ILU_STENCIL && nz <= kClusterPlanes;
   require(schedule != AB2_ILU_STENCIL_CLUSTER || d.walk_cluster,
-          "ILU0 cluster schedule requested but its buffers do not fit shared memory (too many planes along z)");
+          "ILU0 cluster schedule requested with more planes along z than it is offered for");
   d.stencil = true;
   d.levels_l = d.levels_u = (int)(nx + ny + nz - 2);
   return true;
@@ -1210,44 +1070,35 @@ namespace {
 template <class T>
 void walk_apply(ab2_context* ctx, const Ilu0Data& d, T* base, const T* y, T* z) {
   const Walk w = walk_of(d);
-  const WalkArrays<T> b = walk_bands(base, d);
-  const int tiles = w.ntx * w.nty;
-  T* yw = walk_array(base, d, kWalkY);
-  T* lw = walk_array(base, d, kWalkL);
-  T* uw = walk_array(base, d, kWalkU);
-  // FP64: shared-memory transposes; FP32 (half the bytes): element-wise
-  // kernels, which move them faster than the latency-bound transposes (both
-  // measured back to back on one GPU).
-  constexpr bool kTranspose = std::is_same<T, double>::value;
-  const int tr_grid = tiles * ((w.nz + kTrPlanes - 1) / kTrPlanes);
-  if (kTranspose) k_walk_gather_t<T><<<tr_grid, kTileThreads, tr_smem<T>(), ctx->stream>>>(w, y, yw);
-  else k_walk_gather<<<bulk_grid(ctx, w.nw), kThreads, 0, ctx->stream>>>(w, y, yw);
-  check_launch(ctx, "walk_gather");
-  walk_sweep<false, T>(ctx, d, w, b, yw, lw);
-  walk_sweep<true, T>(ctx, d, w, b, lw, uw);
-  if (kTranspose) k_walk_scatter_t<T><<<tr_grid, kTileThreads, tr_smem<T>(), ctx->stream>>>(w, uw, z);
-  else k_walk_scatter<<<bulk_grid(ctx, w.nw), kThreads, 0, ctx->stream>>>(w, uw, z);
-  check_launch(ctx, "walk_scatter");
+  unsigned char* mem = reinterpret_cast<unsigned char*>(base);
+  T* tmp = reinterpret_cast<T*>(mem + walk_mem<T>(w).tmp);
+  walk_sweep<false, T>(ctx, d, w, mem, y, tmp);
+  walk_sweep<true, T>(ctx, d, w, mem, tmp, z);
 }
 
 }  // namespace
 
-// y -> walk order -> L walk -> U walk (reversed index) -> z.
+// y -> forward walk -> backward walk -> z (y and z may be the same vector).
 void ilu_stencil_apply(ab2_context* ctx, const ab2_matrix* A, const Ilu0Data& d, const double* y, double* z) {
   (void)A;
   walk_apply(ctx, d, d.d_walk, y, z);
 }
 
-// FP32 walk arrays: the FP64 factor's bands rounded to float.
+// FP32 walk arrays: the FP64 factor rounded to float.
 void ilu_stencil_enable_f32(ab2_context* ctx, Ilu0Data& d) {
   if (d.d_walk32) return;
   const Walk w = walk_of(d);
-  d.d_walk32 = dev_alloc<float>(ctx, (size_t)kWalkArrays * (size_t)w.nw);
-  op_to_f32(ctx, kWalkBands * w.nw, d.d_walk, d.d_walk32);
-  AB2_CUDA(cudaMemsetAsync(walk_array(d.d_walk32, d, kWalkY), 0, sizeof(float) * (size_t)w.nw, ctx->stream));
-  k_fill_bits32<<<bulk_grid(ctx, 2 * w.nw), kThreads, 0, ctx->stream>>>(2 * w.nw, kSentinel32,
-                                                                        walk_array(d.d_walk32, d, kWalkL));
-  check_launch(ctx, "walk_fill32");
+  const WalkMem m = walk_mem<float>(w), m64 = walk_mem<double>(w);
+  d.d_walk32 = dev_alloc<float>(ctx, (size_t)(m.total + 3) / 4);
+  const unsigned char* from = reinterpret_cast<const unsigned char*>(d.d_walk);
+  unsigned char* to = reinterpret_cast<unsigned char*>(d.d_walk32);
+  const long long steps = (long long)w.ntx * w.nty * kStrips * w.nsteps;
+  k_walk_pack32<false><<<bulk_grid(ctx, steps * 64), kThreads, 0, ctx->stream>>>(steps, from + m64.coef_l, to + m.coef_l);
+  check_launch(ctx, "walk_pack32");
+  k_walk_pack32<true><<<bulk_grid(ctx, steps * 64), kThreads, 0, ctx->stream>>>(steps, from + m64.coef_u, to + m.coef_u);
+  check_launch(ctx, "walk_pack32");
+  fill_halo(ctx, w, d.d_walk32);
+  set_walk_smem<float>();
 }
 
 void ilu_stencil_apply_f32(ab2_context* ctx, const Ilu0Data& d, const float* y, float* z) {
@@ -1255,19 +1106,12 @@ void ilu_stencil_apply_f32(ab2_context* ctx, const Ilu0Data& d, const float* y, 
   walk_apply(ctx, d, d.d_walk32, y, z);
 }
 
-// After a failed application: the propagation arrays back to the sentinel
-// (the tickets are reset by pc_reset).
+// After a failed application: the hand-over words back to the sentinel (the
+// tickets are reset by pc_reset).
 void ilu_stencil_reset(ab2_context* ctx, const Ilu0Data& d) {
-  if (d.d_walk) {
-    k_fill_bits<<<bulk_grid(ctx, 2 * d.walk_n), kThreads, 0, ctx->stream>>>(2 * d.walk_n, kSentinel,
-                                                                            walk_array(d.d_walk, d, kWalkL));
-    check_launch(ctx, "walk_fill");
-  }
-  if (d.d_walk32) {
-    k_fill_bits32<<<bulk_grid(ctx, 2 * d.walk_n), kThreads, 0, ctx->stream>>>(2 * d.walk_n, kSentinel32,
-                                                                              walk_array(d.d_walk32, d, kWalkL));
-    check_launch(ctx, "walk_fill32");
-  }
+  const Walk w = walk_of(d);
+  if (d.d_walk) fill_halo(ctx, w, d.d_walk);
+  if (d.d_walk32) fill_halo(ctx, w, d.d_walk32);
 }
 
 }  // namespace ab2

@@ -33,21 +33,18 @@ struct Ilu0Data {
   int st_nx = 0, st_ny = 0, st_nz = 0;
   double* d_bands = nullptr;            // set-up only: 8 n-vectors L(-k,-j,-i) U(+i,+j,+k) pivot diag
   unsigned int* d_tile_tickets = nullptr;  // factorisation, L sweep, U sweep
-  // Walk layout (ilu_stencil.cu): 10 arrays of walk_n doubles -- the factor's
-  // L(-k,-j,-i), U(+i,+j,+k) and pivot bands, the gathered right-hand side,
-  // and the two sweeps' propagation arrays.
-  long long walk_n = 0;
+  // The walk's arrays in one allocation each (ilu_stencil.cu, WalkMem):
+  // coefficients of both sweeps, the forward sweep's output, hand-over words.
   double* d_walk = nullptr;
-  float* d_walk32 = nullptr;  // the same arrays in FP32 (mixed-precision inner solves), built on demand
-  bool walk_cluster = false;  // sweeps in 2 x 2-tile clusters (else one tile per CTA)
+  float* d_walk32 = nullptr;  // the same in FP32 (mixed-precision inner solves), built on demand
+  bool walk_cluster = false;  // the name the walk is reported by (AB2_ILU_STENCIL_CLUSTER)
 };
 
 // Detects a 3-D 7-point matrix in lexicographic order and, if found,
 // factorises it on the tile-walk schedule (bands + CSR copy in d_lu); with
 // factored, d_lu already holds the factor and only the walk arrays are built.
-// schedule (AB2_ILU_*): AB2_ILU_STENCIL keeps one tile per CTA; AUTO and
-// AB2_ILU_STENCIL_CLUSTER take the cluster walk when it fits (the latter
-// fails otherwise).
+// schedule (AB2_ILU_*): AB2_ILU_STENCIL_CLUSTER fails beyond the planes along z
+// it is offered for.
 bool ilu_stencil_setup(ab2_context* ctx, const ab2_matrix* A, Ilu0Data& d, bool factored, int schedule);
 void ilu_stencil_apply(ab2_context* ctx, const ab2_matrix* A, const Ilu0Data& d, const double* y, double* z);
 // Puts the sweeps' propagation arrays back to the sentinel (after a failed application).

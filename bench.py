@@ -1249,7 +1249,7 @@ def main():
     if METHODS[a.method]["precond"] == "ilu0":
         pc = abi.Precond(ctx, A, "ilu0")
         ilu_ms = timed(lambda: pc.apply(b, vy), 20)
-        roofline = roof("k_walk_gather_t + k_walk_sweep_cl<L> + k_walk_sweep_cl<U> + k_walk_scatter_t (ILU0 apply, tile walk in 2x2-tile clusters)",
+        roofline = roof("k_walk_sweep<L> + k_walk_sweep<U> (ILU0 apply, strip walk)",
                         ilu_bytes(P.n, P.nnz), ilu_ms, f"ilu0_apply_{n1}")
         roofline["bytes_formula"] = "B_LU = 12 nnz + 4 (n + 1) + 8 n"
         smin = ilu_stencil_min_bytes(P.n, P.nnz)

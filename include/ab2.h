@@ -212,12 +212,10 @@ int ab2_dot_noalloc(const double* x, const double* y, int n, double* result, voi
  * WAVEFRONT: any CSR matrix; rows grouped by wavefront of the triangular
  *   graphs, one warp per 32 rows, cross-warp waits through global memory.
  * STENCIL: 3-D 7-point matrices in lexicographic order; 16x16 tiles of
- *   grid lines per CTA walk their diagonals through shared memory; values
+ *   grid lines per CTA, a warp per 16x8 lines walks their diagonals; values
  *   between tiles through global memory.
- * STENCIL_CLUSTER: the STENCIL walk with 2x2 tiles per thread-block cluster;
- *   values between the tiles of a cluster go straight into the neighbour's
- *   shared memory.  Its buffers must fit shared memory: up to ~350 planes
- *   along z (a request beyond that is refused).
+ * STENCIL_CLUSTER: the same walk, for up to 346 planes along z (a request
+ *   beyond that is refused).
  * AUTO: STENCIL_CLUSTER, else STENCIL when the matrix has that structure,
  *   else WAVEFRONT. */
 #define AB2_ILU_AUTO 0

@@ -95,3 +95,18 @@ def test_mixed_null_rhs_and_repeat(ctx):
         assert st.succeeded
         xs.append(x.download())
     np.testing.assert_array_equal(xs[0], xs[1])
+
+
+@pytest.mark.parametrize("dims", [(37, 21, 19), (16, 9, 2), (5, 33, 48)])
+def test_mixed_ilu0_strip_walk_bit_exact(ctx, dims):
+    """The FP32 strip walk on grids with partial tiles and strips, against the oracle."""
+    P = abi.convdiff(*dims, seed=6)
+    kw = dict(solver="bicgs", precond="ilu0", tol=1e-10, max_outer=10, inner_tol=1e-4, inner_max_iter=500)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals, F32)
+    M = abi.Mixed(ctx, A, **kw)
+    x = ctx.vector(P.n)
+    st = M.solve(ctx.vector(P.b), x)
+    o = O.mixed_solve(P.row_ptr, P.cols, P.vals, P.b, dot_mode=O.DOT_DEVICE_TREE,
+                      tree_blocks=ctx.info.reduction_max_blocks, **kw)
+    assert (st.outer_iterations, st.inner_iterations) == (o.outer_iterations, o.inner_iterations)
+    np.testing.assert_array_equal(x.download(), o.x)

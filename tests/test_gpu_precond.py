@@ -145,3 +145,33 @@ def test_ilu0_stencil_walks_bit_exact(ctx, schedule, dims):
         vy, vx = ctx.vector(y), ctx.vector(P.n)
         pc.apply(vy, vx)
         np.testing.assert_array_equal(vx.download(), O.ilu0_apply(P.row_ptr, P.cols, P.vals, y))
+
+
+# The strip walk at the edges of its tiles, strips, rings and lanes (odd sides,
+# one line, planes below and above the ring sizes), with right-hand sides that
+# leave the fast division's range: zeros, tiny and huge values, denormals,
+# infinities and NaN.  Same bits as the sequential sweeps.
+@pytest.mark.parametrize("dims", [(2, 2, 2), (3, 2, 41), (16, 8, 24), (17, 9, 23), (15, 24, 11), (33, 31, 37)])
+@pytest.mark.parametrize("scale", [1.0, 1e-140, 1e140])
+def test_ilu0_strip_walk_division_range(ctx, dims, scale):
+    P = abi.diffusion(*dims, sigma=1.0, smooth=2.0, seed=7)
+    vals = P.vals * scale
+    A = ctx.matrix(P.row_ptr, P.cols, vals)
+    pc = abi.Precond(ctx, A, "ilu0")  # (a 2 x 2 x 2 profile is no 7-point grid by its entries alone: wavefronts)
+    rng = np.random.default_rng(3)
+    n = P.n
+    y0 = rng.uniform(-1, 1, n)
+    zeros = y0 * (rng.uniform(size=n) < 0.3)
+    zeros[::5] = -0.0
+    wide = y0 * 10.0 ** rng.uniform(-300, 150, n)
+    inf, nan = y0.copy(), y0.copy()
+    inf[n // 3] = np.inf
+    nan[n // 2] = np.nan
+    for y in (y0, zeros, wide, np.zeros(n), inf, nan, y0):
+        vy, vx = ctx.vector(y), ctx.vector(n)
+        pc.apply(vy, vx)
+        with np.errstate(all="ignore"):
+            ref = O.ilu0_apply(P.row_ptr, P.cols, vals, y)
+        got = vx.download()
+        np.testing.assert_array_equal(got, ref)
+        np.testing.assert_array_equal(np.signbit(got)[~np.isnan(ref)], np.signbit(ref)[~np.isnan(ref)])
