@@ -16,6 +16,11 @@
 
 namespace ab2 {
 
+// Orders this thread's accesses (and those it has seen through a barrier) at GPU
+// scope.  __threadfence() is the sequentially consistent fence, which nothing here
+// needs and which costs more.
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 enum class Combine { Sum, Max };
 
 template <Combine C, class T>
@@ -36,10 +41,58 @@ __device__ __forceinline__ T reduce_identity() {
   return C == Combine::Sum ? T(0) : -T(1) / T(0);
 }
 
+// The last step of every grid reduction, by one whole block of 256 threads: out[c]
+// = partials[c * G + 0 .. G) summed as one warp would, lane l taking l, l + 32, ...
+// in order, then the shuffle tree.  All 256 threads fetch (up to 6 words each in
+// flight, staged through shared memory for the summing warp): one warp fetching
+// for itself waits on L2 several times over, ~3 us of a kernel's tail at G = 1184.
+// Ends with a barrier, after which every thread may read out[].
+constexpr int kRedThreads = 256;
+template <int NC, Combine C, class T>
+__device__ __forceinline__ void sum_partials(int G, const T* partials, T* out) {
+  constexpr int kRound = 2 * kRedThreads, kRounds = 3;
+  __shared__ T s_stage[kRound];
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    const T* p = partials + (size_t)c * G;
+    T v = reduce_identity<C, T>();
+    for (int base = 0; base < G; base += kRound * kRounds) {
+      T t[kRounds][2];
+#pragma unroll
+      for (int k = 0; k < kRounds; ++k)
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int b = base + k * kRound + u * kRedThreads + (int)threadIdx.x;
+          t[k][u] = b < G ? __ldcg(p + b) : T(0);
+        }
+#pragma unroll
+      for (int k = 0; k < kRounds; ++k) {
+        const int at = base + k * kRound;
+        if (at >= G) break;
+        __syncthreads();  // the round before has been summed
+        s_stage[threadIdx.x] = t[k][0];
+        s_stage[kRedThreads + threadIdx.x] = t[k][1];
+        __syncthreads();
+        if (threadIdx.x < 32) {
+          const int m = G - at < kRound ? G - at : kRound;
+#pragma unroll 8
+          for (int b = lane; b < m; b += 32) v = combine<C, T>(v, s_stage[b]);
+        }
+      }
+    }
+    if (threadIdx.x < 32) {
+      v = warp_reduce<C, T>(v);
+      if (lane == 0) out[c] = v;
+    }
+  }
+  __syncthreads();
+}
+
 // Reduces acc[0..NC) over the whole grid.  Must be called by every thread of
 // every block (no early returns before it).  Returns true in the thread that
 // wrote the final results (thread 0 of the last block), so callers can run
-// scalar epilogues there; `out` then holds the NC results.
+// scalar epilogues there; `out` then holds the NC results.  256-thread blocks.
 template <int NC, Combine C = Combine::Sum, class T>
 __device__ __forceinline__ bool grid_reduce(T (&acc)[NC], T* partials, unsigned int* counter, T* out) {
   __shared__ T s_warp[NC][32];
@@ -61,29 +114,20 @@ __device__ __forceinline__ bool grid_reduce(T (&acc)[NC], T* partials, unsigned 
       if (lane == 0) partials[(size_t)c * gridDim.x + blockIdx.x] = v;
     }
     if (lane == 0) {
-      __threadfence();
+      fence_gpu();
       unsigned int ticket = atomicAdd(counter, 1u);
       s_last = (ticket == gridDim.x - 1);
     }
   }
   __syncthreads();
-  bool writer = false;
-  if (s_last && warp == 0) {
-    __threadfence();
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      T v = reduce_identity<C, T>();
-      for (int b = lane; b < (int)gridDim.x; b += 32) v = combine<C, T>(v, __ldcg(partials + (size_t)c * gridDim.x + b));
-      v = warp_reduce<C, T>(v);
-      if (lane == 0) out[c] = v;
-    }
-    if (lane == 0) {
-      *counter = 0u;  // ready for the next launch that uses this slot
-      __threadfence();
-      writer = true;
-    }
+  if (!s_last) return false;
+  fence_gpu();
+  sum_partials<NC, C, T>((int)gridDim.x, partials, out);
+  if (threadIdx.x == 0) {
+    *counter = 0u;  // ready for the next launch that uses this slot
+    fence_gpu();
   }
-  return writer;
+  return threadIdx.x == 0;
 }
 
 // The same reduction for a kernel whose logical grid of V * gridDim.x blocks
@@ -123,29 +167,20 @@ __device__ __forceinline__ bool grid_reduce_v(T (&acc)[V][NC], T* partials, unsi
           if (lane == 0) partials[(size_t)c * G + v * gridDim.x + blockIdx.x] = x;
         }
       if (lane == 0) {
-        __threadfence();
+        fence_gpu();
         unsigned int ticket = atomicAdd(counter, 1u);
         s_last = (ticket == gridDim.x - 1);
       }
     }
     __syncthreads();
-    bool writer = false;
-    if (s_last && warp == 0) {
-      __threadfence();
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        T x = reduce_identity<C, T>();
-        for (int b = lane; b < G; b += 32) x = combine<C, T>(x, __ldcg(partials + (size_t)c * G + b));
-        x = warp_reduce<C, T>(x);
-        if (lane == 0) out[c] = x;
-      }
-      if (lane == 0) {
-        *counter = 0u;
-        __threadfence();
-        writer = true;
-      }
+    if (!s_last) return false;
+    fence_gpu();
+    sum_partials<NC, C, T>(G, partials, out);
+    if (threadIdx.x == 0) {
+      *counter = 0u;  // ready for the next launch that uses this slot
+      fence_gpu();
     }
-    return writer;
+    return threadIdx.x == 0;
   }
 }
 
@@ -189,32 +224,23 @@ __device__ __forceinline__ bool grid_reduce_r(const T (&acc)[R][NC], int G, T* p
       x = warp_reduce<Combine::Sum, T>(x);
       if (lane == 0 && L < G) partials[(size_t)c * G + L] = x;
     }
-    if (lane == 0) __threadfence();
+    if (lane == 0) fence_gpu();
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
+    fence_gpu();
     unsigned int ticket = atomicAdd(counter, 1u);
     s_last = (ticket == gridDim.x - 1);
   }
   __syncthreads();
-  bool writer = false;
-  if (s_last && warp == 0) {
-    __threadfence();
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      T x = T(0);
-      for (int b = lane; b < G; b += 32) x = x + __ldcg(partials + (size_t)c * G + b);
-      x = warp_reduce<Combine::Sum, T>(x);
-      if (lane == 0) out[c] = x;
-    }
-    if (lane == 0) {
-      *counter = 0u;
-      __threadfence();
-      writer = true;
-    }
+  if (!s_last) return false;
+  fence_gpu();
+  sum_partials<NC, Combine::Sum, T>(G, partials, out);
+  if (threadIdx.x == 0) {
+    *counter = 0u;  // ready for the next launch that uses this slot
+    fence_gpu();
   }
-  return writer;
+  return threadIdx.x == 0;
 }
 
 }  // namespace ab2
