@@ -44,6 +44,7 @@ namespace ab2 {
 namespace {
 
 constexpr int kCtlThreads = 256;
+constexpr long long kLoopWaitCycles = 4000000000LL;  // a grid barrier's bound, ~2 s
 
 template <class T>
 __device__ __forceinline__ void record(SolveStateT<T>* st, T v) {
@@ -110,6 +111,7 @@ __global__ void k_state_init(SolveStateT<T>* st, T tol, int max_iter, T* x, cons
   st->exit_fixup = 0;
   st->x_pending = 0;
   st->bodies = 0;
+  st->barrier = 0;
   st->rho = st->rho1 = st->den = st->alpha = st->beta = st->omega = st->rr_r = 0;
 }
 
@@ -609,6 +611,290 @@ __global__ void __launch_bounds__(kCtlThreads) k_cgj_update_x4(int n, const floa
     cgj_update_scalars<float, DEFER_X>(st, red.result[0], red.result[1], ok, alpha, h, use_graph);
 }
 
+// ------------------------------------------------------------------ the Jacobi-CG loop in one launch
+// The same iteration, all of it in one cooperative launch: between its two
+// reductions an iteration of a system that fits L2 moves little, and two kernels
+// and a conditional node a turn cost more than the work.  One block an SM stands
+// for `slots` = blockDim / 256 logical blocks of the reduction grid at a time and V
+// times over, a thread for its logical threads' V * M rows; each logical block's
+// partials are reduced by k_cgj_update's shuffle tree and written at their place,
+// and after a grid barrier every block sums all G partials in grid_reduce's
+// order, so every block holds the same scalars, bit for bit the graph loop's, and
+// decides alike.  z and the previous p sit side by side (one 2-word load a
+// neighbour); q and p stay in registers between the two halves; r, x and the
+// matrix are read by the same thread every time and stay in its SM's L1.
+//
+template <class T>
+struct Pair2;
+template <>
+struct Pair2<double> {
+  using type = double2;
+};
+template <>
+struct Pair2<float> {
+  using type = float2;
+};
+
+// The partials of this block's logical blocks (acc[v]: logical block v of the
+// thread's slot), reduced as grid_reduce does.
+template <int NC, int V, class T>
+__device__ __forceinline__ void loop_partials(T (&acc)[V][NC], T (&s_warp)[V][2][32], int G, T* partials) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int slots = blockDim.x >> 8;
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const T x = warp_reduce<Combine::Sum, T>(acc[v][c]);
+      if (lane == 0) s_warp[v][c][warp] = x;
+    }
+  __syncthreads();
+  if (warp < slots * V) {
+    const int v = V == 1 ? 0 : warp / slots, sl = V == 1 ? warp : warp - v * slots;
+    const int L = (v * (int)gridDim.x + (int)blockIdx.x) * slots + sl;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      T x = lane < 8 ? s_warp[v][c][sl * 8 + lane] : T(0);
+      x = warp_reduce<Combine::Sum, T>(x);
+      if (lane == 0 && L < G) partials[(size_t)c * G + L] = x;
+    }
+  }
+}
+
+// The sums of all logical blocks' partials, in every thread: staged in shared
+// memory, summed by a warp a component in grid_reduce's order.
+constexpr int kLoopBlocks = 1280;  // most logical blocks
+template <int NC, class T>
+__device__ __forceinline__ void sum_stage(int G, const T* s_stage, T (&s_sum)[2], T (&out)[NC]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp < NC) {
+    T v = T(0);
+#pragma unroll 8
+    for (int b = lane; b < G; b += 32) v = v + s_stage[warp * G + b];
+    v = warp_reduce<Combine::Sum, T>(v);
+    if (lane == 0) s_sum[warp] = v;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < NC; ++c) out[c] = s_sum[c];
+}
+template <int NC, class T>
+__device__ __forceinline__ void loop_sums(int G, const T* partials, T* s_stage, T (&s_sum)[2], T (&out)[NC]) {
+  for (int b = threadIdx.x; b < NC * G; b += blockDim.x) s_stage[b] = __ldcg(partials + b);
+  __syncthreads();
+  sum_stage<NC>(G, s_stage, s_sum, out);
+}
+
+// One reduction over the grid, which every block passes together: the sums of
+// acc over it, in every thread.  Every block writes its partials and passes a
+// counter barrier, then every block fetches and sums all of them.  False, in every
+// thread of the block, once the wait has run out of time (the caller then leaves).
+//
+// Measured against it, us an iteration at 32^3 (this: 6.6): the last block to
+// arrive sums and publishes, the others poll that, 9.5 (an arrival that returns its
+// ticket is a round trip more); every block polling tagged partials instead of a
+// counter, 14.2 (all SMs then read the lines being written); one cluster of 16
+// blocks with partials in distributed shared memory, 9.9 (16 SMs' FP64 units).
+template <int NC, int V, class T>
+__device__ __forceinline__ bool loop_exchange(T (&acc)[V][NC], T* partials, unsigned int* count, unsigned int& target,
+                                              T (&s_warp)[V][2][32], int G, T* s_stage, T (&s_sum)[2], int& s_ok,
+                                              T (&out)[NC]) {
+  loop_partials<NC, V>(acc, s_warp, G, partials);
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    const long long t0 = clock64();
+    int ok = 1;
+    for (unsigned it = 1;; ++it) {
+      unsigned int c;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+      if ((int)(c - target) >= 0) break;
+      if ((it & 255) == 0 && clock64() - t0 > kLoopWaitCycles) {
+        ok = 0;
+        break;
+      }
+    }
+    s_ok = ok;
+  }
+  __syncthreads();
+  const bool ok = s_ok != 0;
+  loop_sums<NC>(G, partials, s_stage, s_sum, out);
+  return ok;
+}
+
+template <class View, class T, int V, int M>
+__global__ void __launch_bounds__(1024, 1)
+    k_cgj_loop(int n, View A, typename Pair2<T>::type* zp, T* r, const T* __restrict__ inv, const T* __restrict__ w,
+               SolveStateT<T>* st, Red<T> red_a, Red<T> red_b, int G) {
+  using P2 = typename Pair2<T>::type;
+  __shared__ T s_warp[V][2][32];
+  __shared__ T s_sum[2];
+  __shared__ T s_stage[2 * kLoopBlocks];
+  __shared__ int s_ok;
+  if (st->done) return;  // (nobody writes the state before every block has passed an exchange)
+  unsigned int target = 0;
+  // odd: which of two partials buffers (alternate ones, so that none is written while it is read)
+  auto exchange = [&](auto& acc, auto& out, int odd) {
+    return loop_exchange<sizeof(out) / sizeof(T), V>(acc, odd ? red_b.partials : red_a.partials, &st->barrier, target,
+                                                     s_warp, G, s_stage, s_sum, s_ok, out);
+  };
+  const int slots = blockDim.x >> 8, slot = threadIdx.x >> 8, lt = threadIdx.x & 255;
+  int row[V][M];  // this thread's rows, n where it has none
+#pragma unroll
+  for (int v = 0; v < V; ++v) {
+    const int L = (v * (int)gridDim.x + (int)blockIdx.x) * slots + slot;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const long long g = (long long)L * 256 + lt + (long long)m * 256 * G;
+      row[v][m] = L < G && g < n ? (int)g : n;
+    }
+  }
+  T* const x = st->x;
+  const T crit = st->crit;
+  const int max_iter = st->max_iter, hist_cap = st->hist_cap;
+  T* const hist = st->hist;
+  const bool scribe = blockIdx.x == 0 && threadIdx.x == 0;
+
+  // z = D^-1 r, rho1 = r.z (k_cgj_start)
+  T acc1[V][1] = {};
+#pragma unroll
+  for (int v = 0; v < V; ++v)
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int i = row[v][m];
+      if (i < n) {
+        const T rv = r[i], zv = inv ? mul_rn(inv[i], rv) : rv;
+        P2 o;
+        o.x = zv;
+        o.y = T(0);
+        zp[i] = o;
+        acc1[v][0] = fma_rn(rv, zv, acc1[v][0]);
+      }
+    }
+  T one[1] = {T(0)}, two[2];
+  bool live = exchange(acc1, one, 1);
+  T rho1 = one[0], rho = T(0), beta = T(0), alpha = T(0), den = T(0), rr = st->rr;
+  int iter = st->iter, hist_len = st->hist_len, first = 1, converged = 0, error = 0, breakdown = 0, bodies = 0;
+  auto stop = [&](T v) {  // stop_test
+    if (iter >= max_iter) return true;
+    rr = v;
+    if (scribe && hist_len < hist_cap) hist[hist_len] = v;
+    ++hist_len;
+    converged = v < crit ? 1 : 0;
+    return converged != 0;
+  };
+  for (bool done = false; live && !done;) {
+    // p = first ? z : z + beta p_old ; q = A p ; den = q.p (k_cgj_spmv)
+    T q[V][M], pn[V][M];
+    T acc[V][1] = {};
+    auto pval = [&](int c) {
+      const P2 o = __ldcg(zp + c);
+      return first ? o.x : fma_rn(beta, o.y, o.x);
+    };
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int i = row[v][m];
+        q[v][m] = pn[v][m] = T(0);
+        if (i < n) {
+          q[v][m] = A.row_f(i, pval);
+          pn[v][m] = pval(i);
+          acc[v][0] = fma_rn(q[v][m], pn[v][m], acc[v][0]);
+        }
+      }
+    if (!(live = exchange(acc, one, 0))) break;
+    den = one[0];
+    // x += alpha p ; r -= alpha q ; z = D^-1 r ; r.r and r.z (k_cgj_update)
+    const bool ok = den != T(0);
+    alpha = ok ? rho1 / den : T(0);
+    T acc2[V][2] = {};
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int i = row[v][m];
+        if (i < n) {
+          T rv = r[i];
+          if (ok) {
+            x[i] = fma_rn(alpha, pn[v][m], x[i]);
+            rv = fma_rn(-alpha, q[v][m], rv);
+            r[i] = rv;
+          }
+          acc2[v][0] = fma_rn(w ? mul_rn(rv, w[i]) : rv, rv, acc2[v][0]);
+          const T zv = inv ? mul_rn(inv[i], rv) : rv;
+          P2 o;
+          o.x = zv;
+          o.y = pn[v][m];
+          zp[i] = o;
+          acc2[v][1] = fma_rn(rv, zv, acc2[v][1]);
+        }
+      }
+    if (!(live = exchange(acc2, two, 1))) break;
+    // cgj_update_scalars
+    ++bodies;
+    if (!ok) {
+      if (stop(two[0])) {
+        ++iter;
+      } else {
+        error = AB2_ERR_BREAKDOWN;
+        breakdown = AB2_BREAKDOWN_ALPHA;
+      }
+      done = true;
+    } else {
+      rho = rho1;
+      ++iter;
+      first = 0;
+      rho1 = two[1];
+      beta = two[1] / rho;
+      done = stop(two[0]);
+    }
+  }
+  if (scribe) {
+    st->rr = rr;
+    st->rho = rho;
+    st->rho1 = rho1;
+    st->den = den;
+    st->alpha = alpha;
+    st->beta = beta;
+    st->iter = iter;
+    st->hist_len = hist_len;
+    st->first = first;
+    st->converged = converged;
+    st->error = live ? error : AB2_ERR_TIMEOUT;
+    st->breakdown = breakdown;
+    st->bodies = bodies;
+    st->done = 1;
+  }
+}
+
+// How a system of n rows fits the one-launch loop: threads a block, blocks, and
+// the rows of a thread (V logical blocks of the reduction grid, M rows each).
+// Where the line lies: up to three rows a logical thread in FP64 (909,000 rows on 148
+// SMs), four in FP32, beyond which the graph loop's two bandwidth-bound kernels are
+// as fast.  Measured on B200, us an iteration, graph loop / one launch: 7-point
+// bands FP64 32^3 15.2 / 6.6, 64^3 21.8 / 11.9, 491,111 rows 24.7 / 18.1, 96^3 32.4 /
+// 28.6, 104^3 40.3 / 40.3 (ELL 43.6 / 47.8); FP32 (scaled Jacobi) 32^3 19.9 / 6.9, 96^3
+// 26.6 / 20.3, 104^3 28.4 / 23.8, 128 x 96 x 96 28.0 / 24.6.
+struct CgLoopFit {
+  int threads = 0, blocks = 0, V = 0, M = 0;  // V = 0: too large
+};
+CgLoopFit cg_loop_fit(const ab2_context* ctx, int n, bool fp32) {
+  CgLoopFit f;
+  const int G = red_grid(ctx, n);
+  if (n <= 0) return f;
+  f.threads = G <= ctx->num_sms ? 256 : G <= 2 * ctx->num_sms ? 512 : 1024;
+  const int slots = f.threads / 256;
+  f.blocks = std::min(ctx->num_sms, (G + slots - 1) / slots);
+  const int v = (G + f.blocks * slots - 1) / (f.blocks * slots);
+  const int m = (int)(((long long)n + 256LL * G - 1) / (256LL * G));
+  if (G > kLoopBlocks || v > 2 || m > (fp32 ? 4 : 3)) return f;
+  f.V = v;
+  f.M = m == 1 ? 1 : m == 2 ? 2 : 4;
+  return f;
+}
+
 // ------------------------------------------------------------------ BiCGStab
 // p = r (first) or p = r + beta (p - omega v)  (BiCGStab.h:273-276, three BLAS-1 calls)
 template <class T>
@@ -944,6 +1230,30 @@ int Krylov<T>::enqueue_body(cudaGraphConditionalHandle h, int graph_loop) {
   return (int)(ctx->launches - before);
 }
 
+// The whole Jacobi-CG loop in one launch (k_cgj_loop).
+template <class T>
+void Krylov<T>::launch_loop() {
+  const int n = A->n;
+  const CgLoopFit f = cg_loop_fit(ctx, n, sizeof(T) == 4);
+  int g = red_grid(ctx, n);
+  auto* zp = reinterpret_cast<typename Pair2<T>::type*>(w[1]);
+  T* r = w[0];
+  const T* inv = diag_inv();
+  const T* weight = stop_weight;
+  Red<T> ra = red_of<T>(ctx, 2), rb = red_of<T>(ctx, 3);
+  with_op([&](auto view) {
+    using View = decltype(view);
+    int nn = n;
+    void* args[] = {&nn, &view, &zp, &r, (void*)&inv, (void*)&weight, &d_st, &ra, &rb, &g};
+    const void* k = f.V == 1 ? (const void*)k_cgj_loop<View, T, 1, 1>
+                    : f.M == 1 ? (const void*)k_cgj_loop<View, T, 2, 1>
+                    : f.M == 2 ? (const void*)k_cgj_loop<View, T, 2, 2>
+                               : (const void*)k_cgj_loop<View, T, 2, 4>;
+    AB2_CUDA(cudaLaunchCooperativeKernel(k, dim3((unsigned)f.blocks), dim3((unsigned)f.threads), args, 0, ctx->stream));
+  });
+  check_launch(ctx, "cgj_loop");
+}
+
 template <class T>
 const T* Krylov<T>::diag_inv() const {
   if (pc->kind != AB2_PC_DIAG) return nullptr;
@@ -988,10 +1298,13 @@ void Krylov<T>::init(ab2_context* c, const ab2_matrix* a, const ab2_precond* p, 
   variant = spmv_variant;
   use_graph = graph_loop;
   fused_diag = solver == AB2_SOLVER_CG && pc && (pc->kind == AB2_PC_DIAG || pc->kind == AB2_PC_NONE);
-  const int nw = fused_diag ? 5 : solver == AB2_SOLVER_CG ? (sizeof(T) == sizeof(double) ? 5 : 4) : 8;
+  one_launch = use_graph && fused_diag && cg_loop_fit(ctx, A->n, sizeof(T) == 4).V > 0;
+  // (the one-launch loop keeps r, and z and p side by side)
+  const int nw = one_launch ? 2 : fused_diag ? 5 : solver == AB2_SOLVER_CG ? (sizeof(T) == sizeof(double) ? 5 : 4) : 8;
   for (int i = 0; i < nw; ++i) {
-    w[i] = dev_alloc<T>(ctx, (size_t)A->n);
-    AB2_CUDA(cudaMemsetAsync(w[i], 0, sizeof(T) * (size_t)std::max(A->n, 1), ctx->stream));
+    const size_t words = (size_t)A->n * (one_launch && i == 1 ? 2 : 1);
+    w[i] = dev_alloc<T>(ctx, words);
+    AB2_CUDA(cudaMemsetAsync(w[i], 0, sizeof(T) * std::max<size_t>(words, 1), ctx->stream));
   }
   d_st = dev_alloc<SolveStateT<T>>(ctx, 1);
   AB2_CUDA(cudaMemsetAsync(d_st, 0, sizeof(SolveStateT<T>), ctx->stream));
@@ -999,7 +1312,7 @@ void Krylov<T>::init(ab2_context* c, const ab2_matrix* a, const ab2_precond* p, 
   std::memset(h_st, 0, sizeof(SolveStateT<T>));
   hist_cap = 2 * max_iter + 8;  // BiCGStab tests s and r each iteration
   d_hist = dev_alloc<T>(ctx, (size_t)hist_cap);
-  if (use_graph) build_graph();
+  if (use_graph && !one_launch) build_graph();
 }
 
 template <class T>
@@ -1017,6 +1330,12 @@ void Krylov<T>::solve(const T* b, T* x, T tol, int max_iter) {
     k_residual<<<g, kCtlThreads, 0, ctx->stream>>>(n, view, d_st, w[0], r0, red_of<T>(ctx, 0));
   });
   check_launch(ctx, "residual");
+  if (one_launch) {
+    launch_loop();  // (returns at once for a null right-hand side)
+    AB2_CUDA(cudaMemcpyAsync(h_st, d_st, sizeof(SolveStateT<T>), cudaMemcpyDeviceToHost, ctx->stream));
+    AB2_CUDA(cudaStreamSynchronize(ctx->stream));
+    return;
+  }
   if (fused_diag) {
     const T* inv = diag_inv();
     k_cgj_start<<<g, kCtlThreads, 0, ctx->stream>>>(n, w[0], inv, inv ? w[1] : nullptr, d_st, red_of<T>(ctx, 1));

@@ -26,6 +26,7 @@ struct SolveStateT {
   int exit_fixup;  // BiCGStab exits on ||s||: x += alpha phat still to do
   int x_pending;   // CG with the deferred x update: x += alpha p still owed
   int bodies;      // loop bodies executed (for launch accounting)
+  unsigned int barrier;  // arrivals at the one-launch loop's grid barriers
 };
 
 using SolveState = SolveStateT<double>;
@@ -50,6 +51,7 @@ struct Krylov {
   cudaGraphConditionalHandle handle = 0;
   int body_launches = 0;
   bool fused_diag = false;  // CG with Diag or no preconditioner: the two-kernel body
+  bool one_launch = false;  // ... and its whole loop in one cooperative launch
   // Operator override (set before init): the symmetric unit-diagonal 7-point
   // operator kept as three upper bands on A's grid (the mixed solver's
   // symmetrically scaled Jacobi form), used in place of A's own values.
@@ -73,6 +75,7 @@ struct Krylov {
   template <class F>
   void with_op(F&& f) const;  // f(view of the operator): unit_bands or A in `variant`
   void build_graph();
+  void launch_loop();
   const T* diag_inv() const;  // 1/a_ii of a Diag preconditioner in T, else null
 };
 

@@ -237,3 +237,60 @@ def test_breakdown_reported(ctx):
         assert r.error == -3 and r.breakdown == "alpha"
         assert st.error == abi.AB2_ERR_BREAKDOWN and st.breakdown == "alpha"
         assert st.iterations == r.iterations and not st.succeeded
+
+
+# CG with Diag or no preconditioner runs its loop in one launch up to some size
+# (graph loop beyond it); the host-driven loop runs the two kernels an iteration.
+# Row counts around the launch's block, slot and row limits: same iterations,
+# history and solution, bit for bit.
+@pytest.mark.parametrize("precond", ["diag", "none"])
+@pytest.mark.parametrize("n", [1, 255, 257, 2048, 37889, 75777, 151553, 303105, 606209, 909313])
+def test_one_launch_cg_equals_host_loop(ctx, n, precond):
+    rng = np.random.default_rng(n)
+    off = -rng.uniform(0.1, 1.0, n - 1)
+    diag = np.full(n, 0.3) + np.append(-off, 0.0) + np.append(0.0, -off)
+    rows = np.arange(n)
+    ci = np.concatenate([rows, rows[1:] - 1, rows[:-1] + 1])
+    ri = np.concatenate([rows, rows[1:], rows[:-1]])
+    vv = np.concatenate([diag, off, off])
+    order = np.lexsort((ci, ri))
+    rp = np.zeros(n + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(ri, minlength=n))
+    A = ctx.matrix(rp, ci[order], vv[order])
+    b = ctx.vector(rng.uniform(-1, 1, n))
+    for max_iter in (0, 1, 12):
+        got = []
+        for graph in (True, False):
+            S = abi.Solver(ctx, A, solver="cg", precond=precond, tol=1e-14, max_iter=max_iter, use_graph=graph)
+            for _ in range(2):  # the second solve reuses the launch's state
+                x = ctx.vector(n)
+                st = S.solve(b, x)
+            got.append((st.iterations, st.succeeded, st.breakdown, st.residual, x.download(), S.history()))
+            S.close()
+        assert got[0][:4] == got[1][:4]
+        np.testing.assert_array_equal(got[0][4], got[1][4])
+        np.testing.assert_array_equal(got[0][5], got[1][5])
+
+
+def test_one_launch_cg_breakdown_and_null_rhs(ctx):
+    """p.q = 0 (a zero matrix entry by entry) ends as the host loop ends; a null
+    right-hand side leaves x untouched."""
+    n = 700
+    rp, ci = np.arange(n + 1, dtype=np.int32), np.arange(n, dtype=np.int32)
+    A = ctx.matrix(rp, ci, np.zeros(n))
+    b = ctx.vector(np.ones(n))
+    res = []
+    for graph in (True, False):
+        S = abi.Solver(ctx, A, solver="cg", precond="none", tol=1e-8, max_iter=9, use_graph=graph)
+        x = ctx.vector(n)
+        try:
+            st = S.solve(b, x)
+            res.append((st.iterations, st.succeeded, st.error, st.breakdown))
+        except abi.AB2Error as e:
+            res.append(e.code)
+        z = ctx.vector(np.full(n, 3.0))
+        st = S.solve(ctx.vector(n), z)
+        assert st.succeeded and st.iterations == 0
+        np.testing.assert_array_equal(z.download(), np.full(n, 3.0))
+        S.close()
+    assert res[0] == res[1]
