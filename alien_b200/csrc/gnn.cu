@@ -975,48 +975,89 @@ __global__ void __launch_bounds__(256) k_gnn_agg_bwd(int n, const int* __restric
   }
 }
 
-// Partials of grad W (64 x 128) and grad b (64): sum_i dpre_i [h_i ; m_i]^T,
-// staged 32 nodes at a time; thread t owns output o = t/4, inputs (t%4)*32 ..+32.
+// Partials of grad W (64 x 128) and grad b (64): sum_i dpre_i [h_i ; m_i]^T in
+// FP32, node by node in order (a block's nodes are consecutive).  32 nodes at a
+// time are staged in shared memory as floats, the next 32 already on their way
+// into registers (five 16-byte loads a thread); a thread owns 4 outputs x 8
+// inputs, so a node costs it three 16-byte shared loads and 32 multiply-adds.
+// Bound by the FP32 multiply-adds (60 us of them at 64^3 nodes).  Measured at 64^3
+// on B200: 1627 us with 1 x 32 tiles a thread, single-word shared loads and a
+// four-way bank conflict on each; 120 us now, the same sums in the same order.
 __global__ void __launch_bounds__(256) k_gnn_wgrad(int n, const float* __restrict__ dh, const bf16* __restrict__ hout,
                                                    const bf16* __restrict__ h, const bf16* __restrict__ m,
                                                    float* __restrict__ part) {
-  __shared__ float s_dp[32][kH + 1];
-  __shared__ float s_in[32][kIn + 1];
-  const int o = threadIdx.x >> 2, k0 = (threadIdx.x & 3) * 32;
-  float acc[32];
+  constexpr int kRows = 32;
+  __shared__ __align__(16) float s_dp[kRows][kH];
+  __shared__ __align__(16) float s_in[kRows][kIn];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;  // inputs 4 tx.. and 64 + 4 tx.., outputs 4 ty..
+  const int lr = threadIdx.x >> 3, lc = (threadIdx.x & 7) * 8;  // staged: row, first of 8 columns
+  float acc[4][8], accb[4];
 #pragma unroll
-  for (int q = 0; q < 32; ++q) acc[q] = 0.f;
-  float accb = 0.f;
+  for (int p = 0; p < 4; ++p) {
+    accb[p] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[p][q] = 0.f;
+  }
   const int per = (n + gridDim.x - 1) / gridDim.x;
   const int lo = blockIdx.x * per, hi = min(n, lo + per);
-  for (int base = lo; base < hi; base += 32) {
+  float4 d0, d1;
+  uint4 vo, vh, vm;
+  auto load = [&](int base) {
+    const int i = base + lr;
+    d0 = d1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    vo = vh = vm = make_uint4(0u, 0u, 0u, 0u);
+    if (i < hi) {
+      const size_t at = (size_t)i * kH + lc;
+      d0 = __ldg(reinterpret_cast<const float4*>(dh + at));
+      d1 = __ldg(reinterpret_cast<const float4*>(dh + at + 4));
+      vo = __ldg(reinterpret_cast<const uint4*>(hout + at));
+      vh = __ldg(reinterpret_cast<const uint4*>(h + at));
+      vm = __ldg(reinterpret_cast<const uint4*>(m + at));
+    }
+  };
+  auto put = [](float* to, const uint4& v) {
+    const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), c = unpack_bf16(v.z), d = unpack_bf16(v.w);
+    *reinterpret_cast<float4*>(to) = make_float4(a.x, a.y, b.x, b.y);
+    *reinterpret_cast<float4*>(to + 4) = make_float4(c.x, c.y, d.x, d.y);
+  };
+  if (lo < hi) load(lo);
+  for (int base = lo; base < hi; base += kRows) {
     __syncthreads();
-    for (int t = threadIdx.x; t < 32 * kH; t += blockDim.x) {
-      const int r = t / kH, c = t % kH, i = base + r;
-      float dp = 0.f, hh = 0.f, mm = 0.f;
-      if (i < hi) {
-        const float hv = __bfloat162float(hout[(size_t)i * kH + c]);
-        dp = hv > 0.f ? dh[(size_t)i * kH + c] : 0.f;
-        hh = __bfloat162float(h[(size_t)i * kH + c]);
-        mm = __bfloat162float(m[(size_t)i * kH + c]);
-      }
-      s_dp[r][c] = dp;
-      s_in[r][c] = hh;
-      s_in[r][kH + c] = mm;
+    {
+      const float2 a = unpack_bf16(vo.x), b = unpack_bf16(vo.y), c = unpack_bf16(vo.z), d = unpack_bf16(vo.w);
+      *reinterpret_cast<float4*>(&s_dp[lr][lc]) = make_float4(a.x > 0.f ? d0.x : 0.f, a.y > 0.f ? d0.y : 0.f,
+                                                             b.x > 0.f ? d0.z : 0.f, b.y > 0.f ? d0.w : 0.f);
+      *reinterpret_cast<float4*>(&s_dp[lr][lc + 4]) = make_float4(c.x > 0.f ? d1.x : 0.f, c.y > 0.f ? d1.y : 0.f,
+                                                                 d.x > 0.f ? d1.z : 0.f, d.y > 0.f ? d1.w : 0.f);
+      put(&s_in[lr][lc], vh);
+      put(&s_in[lr][kH + lc], vm);
     }
     __syncthreads();
-    const int rows = min(32, hi - base);
+    if (base + kRows < hi) load(base + kRows);
+    const int rows = min(kRows, hi - base);
+#pragma unroll 4
     for (int r = 0; r < rows; ++r) {
-      const float d = s_dp[r][o];
+      const float4 dv = *reinterpret_cast<const float4*>(&s_dp[r][4 * ty]);
+      const float4 x0 = *reinterpret_cast<const float4*>(&s_in[r][4 * tx]);
+      const float4 x1 = *reinterpret_cast<const float4*>(&s_in[r][kH + 4 * tx]);
+      const float d[4] = {dv.x, dv.y, dv.z, dv.w};
+      const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-      for (int q = 0; q < 32; ++q) acc[q] = fmaf(d, s_in[r][k0 + q], acc[q]);
-      if (k0 == 0) accb += d;
+      for (int p = 0; p < 4; ++p) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) acc[p][q] = fmaf(d[p], x[q], acc[p][q]);
+        if (tx == 0) accb[p] += d[p];
+      }
     }
   }
   float* out = part + (size_t)blockIdx.x * (kH * kIn + kH);
 #pragma unroll
-  for (int q = 0; q < 32; ++q) out[o * kIn + k0 + q] = acc[q];
-  if (k0 == 0) out[kH * kIn + o] = accb;
+  for (int p = 0; p < 4; ++p) {
+    float* row = out + (4 * ty + p) * kIn;
+    *reinterpret_cast<float4*>(row + 4 * tx) = make_float4(acc[p][0], acc[p][1], acc[p][2], acc[p][3]);
+    *reinterpret_cast<float4*>(row + kH + 4 * tx) = make_float4(acc[p][4], acc[p][5], acc[p][6], acc[p][7]);
+    if (tx == 0) out[kH * kIn + 4 * ty + p] = accb[p];
+  }
 }
 
 // Partials of grad W0 (64 x 2) and b0: dpre0 = dh1 (.) (h1 > 0), x0 recomputed.
@@ -1055,13 +1096,38 @@ __global__ void __launch_bounds__(256) k_gnn_encode_bwd(int n, const float* __re
   }
 }
 
-// out[k] = sum_b part[b][k], block order.
-__global__ void k_gnn_reduce_partials(int nb, int width, const float* __restrict__ part, float* __restrict__ out) {
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < width; k += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < nb; ++b) s += part[(size_t)b * width + k];
-    out[k] = s;
+// out[k] = sum_b part[b][k], block order.  A block sums 32 outputs: all its
+// threads stage 128 blocks' partials at a time in shared memory, one warp adds them in
+// order.  (One thread an output fetching for itself waited on L2 for every few
+// of its up to ~1,200 partials: 47 us a call against 9 us, the same sums.)
+__global__ void __launch_bounds__(256) k_gnn_reduce_partials(int nb, int width, const float* __restrict__ part,
+                                                             float* __restrict__ out) {
+  constexpr int kStage = 128;
+  __shared__ float s_part[2][kStage][32];
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  float v[kStage / 8];
+  auto load = [&](int base) {
+#pragma unroll
+    for (int u = 0; u < kStage / 8; ++u) {
+      const int b = base + row + 8 * u;
+      v[u] = b < nb && k < width ? __ldg(part + (size_t)b * width + k) : 0.f;
+    }
+  };
+  float s = 0.f;
+  load(0);
+  for (int base = 0, buf = 0; base < nb; base += kStage, buf ^= 1) {
+#pragma unroll
+    for (int u = 0; u < kStage / 8; ++u) s_part[buf][row + 8 * u][lane] = v[u];
+    __syncthreads();
+    if (base + kStage < nb) load(base + kStage);
+    if (row == 0) {
+      const int m = min(kStage, nb - base);
+#pragma unroll 16
+      for (int b = 0; b < m; ++b) s += s_part[buf][b][lane];
+    }
   }
+  if (row == 0 && k < width) out[k] = s;
 }
 
 // Adam on the FP32 master weights.
@@ -1206,7 +1272,8 @@ int warp_grid(ab2_context* ctx, int n) {
   return std::max(1, std::min((n + kWarpsPerBlock - 1) / kWarpsPerBlock, ctx->num_sms * 8));
 }
 int tile_grid(ab2_context* ctx, int n) { return std::max(1, std::min((n + 127) / 128, ctx->num_sms * 4)); }
-int wgrad_grid(ab2_context* ctx, int n) { return std::max(1, std::min((n + 2047) / 2048, ctx->num_sms * 2)); }
+// Two blocks an SM from ~150,000 nodes on (64^3 nodes: 120 us a layer, 157 us with one an SM).
+int wgrad_grid(ab2_context* ctx, int n) { return std::max(1, std::min((n + 511) / 512, ctx->num_sms * 2)); }
 
 bf16* hbuf(ab2_gnn* G, int l) { return G->d_h + (size_t)l * G->n * kH; }
 bf16* mbuf(ab2_gnn* G, int l) { return G->d_m + (size_t)l * G->n * kH; }
@@ -1327,7 +1394,7 @@ void gnn_forward(ab2_gnn* G, const double* r, double* z, bool training = false) 
 }
 
 void reduce_into(ab2_gnn* G, int nb, int width, float* out) {
-  k_gnn_reduce_partials<<<(width + 255) / 256, 256, 0, G->ctx->stream>>>(nb, width, G->d_part, out);
+  k_gnn_reduce_partials<<<(width + 31) / 32, 256, 0, G->ctx->stream>>>(nb, width, G->d_part, out);
   check_launch(G->ctx, "gnn_reduce");
 }
 

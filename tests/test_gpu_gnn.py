@@ -217,3 +217,27 @@ def test_trained_network_gains_over_its_jacobi_path(ctx):
         res[name] = r.iterations
     print("flexible CG iterations, held-out 48^3 field:", res)
     assert res["trained"] <= 0.9 * res["skip_only"], res
+
+
+@pytest.mark.parametrize("shape", [(3, 3, 3), (8, 8, 8), (17, 13, 11), (33, 16, 9)])
+def test_gradient_blocks_ragged(ctx, shape):
+    """Weight gradients on node counts below one staged group, at a block's
+    boundary and with ragged last groups in several blocks, against the oracle
+    (bounds of test_gradient_matches_oracle)."""
+    P = abi.diffusion(*shape, sigma=1.0, smooth=2.0, seed=8)
+    rng = np.random.default_rng(5)
+    e = rng.normal(size=P.n)
+    graph = G.Graph.from_csr(P.row_ptr, P.cols, P.vals)
+    r = graph.matvec(e)
+    p = G.init_params(3)
+    net = abi.Gnn(ctx, p.flat().astype(np.float32))
+    net.bind(ctx.matrix(P.row_ptr, P.cols, P.vals))
+    L, g = net.loss_grad(ctx.vector(r), ctx.vector(e))
+    Lo, go = G.backward(p, graph, r, e, bf16_round=True)
+    assert abs(L - Lo) <= 2e-2 * abs(Lo)
+    gb, gob = blocks(g.astype(np.float64)), blocks(go.flat())
+    for name in gb:
+        a, b = gb[name], gob[name]
+        err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+        cos = a @ b / max(np.linalg.norm(a) * np.linalg.norm(b), 1e-30)
+        assert err < 5e-2 and cos > 0.998, (name, err, cos)
