@@ -31,16 +31,23 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <initializer_list>
 #include <random>
+#include <type_traits>
 
 #include "ab2_internal.cuh"
 #include "precond.cuh"
+#include "recip.cuh"
 #include "sentinel.cuh"
 #include "spmv_view.cuh"
 
 namespace ab2 {
 
 namespace {
+
+// The one-CTA sweeps: shared memory they may use, entries of a row they pack.
+constexpr int kCtaSmemMax = 220 * 1024;
+constexpr int kCtaMaxEntries = 8;
 
 // acc - sum_{k in [kb, ke)} a_k x[c_k], k ascending, waiting for each x value to
 // be produced.  Up to 8 dependencies are loaded at once, so a row whose inputs
@@ -151,6 +158,235 @@ __global__ void __launch_bounds__(256) k_ilu_usweep(int len, const int* __restri
   if (blockIdx.x == 0 && threadIdx.x == 0) tickets[0] = 0u;
 }
 
+// ------------------------------------------------------------------ both sweeps by one CTA
+// A factor whose vector fits one SM's shared memory and whose wavefronts are
+// narrow (a 2-D grid of 180 x 140 has 320 of them, at most 140 rows each) spends
+// its sweeps on hand-overs between SMs: 1.45 us a wavefront through L2.  Here one CTA
+// keeps the vector in shared memory, in place from right-hand side to solution, and
+// walks the wavefronts with a barrier between them: the rows of a wavefront are
+// packed in chunks of 32, a chunk a warp, and each warp loads the chunks of its
+// next wavefronts into registers ahead of time.  What bounds it is the chain of a
+// wavefront -- shared loads, the row's multiply-adds, (backward) the division off a
+// stored reciprocal, the store, the barrier -- and, a warp that waits for itself
+// issuing an instruction in 3-4 cycles, the number of its instructions.  So a
+// chunk is three or so 16-byte loads a lane from one address, places are byte
+// offsets, and nothing is predicated: a missing entry is 0 times a word that holds
+// 0 (subtracting +0 changes nothing), a missing row or chunk works on a word of
+// its own.  Measured on B200, one application at 181 x 140: 931 us across SMs, 210
+// with predicated rows of separately addressed arrays (rows placed in wavefront
+// order instead of natural order: the same, not the banks), 126 us.
+template <class T, int W>
+struct CtaChunk {  // one chunk in memory, by lane (bytes from its start)
+  static constexpr int kInts = (1 + W + 3) / 4;  // int4 a lane: row, W columns, unused
+  static constexpr int ints = 0;
+  static constexpr int vals = ints + kInts * 32 * 16;
+  static constexpr int rec = vals + W * 32 * (int)sizeof(T);  // U only: reciprocal (and the pivot, FP64)
+  static constexpr int kRec = 32 * (Recip<T>::keep_pivot ? 16 : 8);
+  template <bool UP>
+  static constexpr int bytes() {
+    return UP ? rec + kRec : rec;
+  }
+};
+
+template <class T, int W>
+struct CtaRow {
+  int at[4 * CtaChunk<T, W>::kInts];  // byte offsets of the row's word and of its columns' words
+  T val[W], piv;
+  typename Recip<T>::type rec;
+};
+
+template <bool UP, class T, int W>
+__device__ __forceinline__ void cta_load(const unsigned char* c, int lane, CtaRow<T, W>& e) {
+  using L = CtaChunk<T, W>;
+#pragma unroll
+  for (int k = 0; k < L::kInts; ++k) {
+    const int4 v = __ldg(reinterpret_cast<const int4*>(c + L::ints) + k * 32 + lane);
+    e.at[4 * k] = v.x;
+    e.at[4 * k + 1] = v.y;
+    e.at[4 * k + 2] = v.z;
+    e.at[4 * k + 3] = v.w;
+  }
+#pragma unroll
+  for (int j = 0; j < W; j += 2) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(c + L::vals) + j / 2 * 32 + lane);
+      e.val[j] = v.x;
+      e.val[j + 1] = v.y;
+    } else {
+      const float2 v = __ldg(reinterpret_cast<const float2*>(c + L::vals) + j / 2 * 32 + lane);
+      e.val[j] = v.x;
+      e.val[j + 1] = v.y;
+    }
+  }
+  if constexpr (UP) {
+    if constexpr (sizeof(T) == 8) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(c + L::rec) + lane);
+      e.rec = v.x;
+      e.piv = v.y;
+    } else {
+      e.rec = __ldg(reinterpret_cast<const double*>(c + L::rec) + lane);
+      e.piv = T(0);
+    }
+  }
+}
+
+template <bool UP, class T, int W>
+__device__ __forceinline__ void cta_row(const CtaRow<T, W>& e, unsigned char* x) {
+  auto word = [x](int at) -> T& { return *reinterpret_cast<T*>(x + at); };
+  T v[W];
+#pragma unroll
+  for (int j = 0; j < W; ++j) v[j] = word(e.at[1 + j]);
+  T acc = word(e.at[0]);
+#pragma unroll
+  for (int j = 0; j < W; ++j) acc = mul_sub_rn(e.val[j], v[j], acc);
+  if constexpr (UP) {
+    bool bad;
+    const T q = Recip<T>::div(acc, e.piv, e.rec, bad);
+    acc = bad ? Recip<T>::slow(acc, e.piv, e.rec) : q;
+  }
+  word(e.at[0]) = acc;
+}
+
+// One sweep: ptr (shared memory) the chunks before each of its wavefronts, chunk
+// number ptr[levels] the one without rows.  D wavefronts are loaded ahead.
+template <bool UP, class T, int W, int D, bool WIDE>
+__device__ __forceinline__ void cta_sweep(int levels, const unsigned char* chunks, const int* ptr, unsigned char* x,
+                                          int nw) {
+  constexpr int kBytes = CtaChunk<T, W>::template bytes<UP>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int none = ptr[levels];
+  CtaRow<T, W> e[D];
+  int begin = 0;  // of the next wavefront to load
+  auto ahead = [&](int l, CtaRow<T, W>& t) {
+    const int end = ptr[min(l + 1, levels)];
+    const int c = begin + warp < end ? begin + warp : none;
+    begin = end;
+    cta_load<UP>(chunks + (size_t)c * kBytes, lane, t);
+  };
+#pragma unroll
+  for (int u = 0; u < D; ++u) ahead(u, e[u]);
+  for (int l0 = 0; l0 < levels; l0 += D) {
+#pragma unroll
+    for (int u = 0; u < D; ++u) {
+      const int l = l0 + u;  // (past the last wavefront: the chunk without rows)
+      cta_row<UP>(e[u], x);
+      if constexpr (WIDE) {  // wavefronts wider than the sweeping warps
+        if (l < levels)
+          for (int c = ptr[l] + warp + nw; c < ptr[l + 1]; c += nw) {
+            CtaRow<T, W> t;
+            cta_load<UP>(chunks + (size_t)c * kBytes, lane, t);
+            cta_row<UP>(t, x);
+          }
+      }
+      ahead(l + D, e[u]);
+      asm volatile("bar.sync 1, %0;" ::"r"(nw * 32) : "memory");
+    }
+  }
+}
+
+template <class T, int W, bool WIDE>
+__global__ void __launch_bounds__(512, 1)
+    k_ilu_cta(int n, int nw, int levels_l, int levels_u, const unsigned char* __restrict__ chunks_l,
+              const unsigned char* __restrict__ chunks_u, const int* __restrict__ ptr, const T* y, T* z) {
+  constexpr int D = W <= 2 ? 4 : W <= 4 ? 3 : 2;
+  extern __shared__ __align__(16) unsigned char cta_smem[];
+  T* x = reinterpret_cast<T*>(cta_smem);
+  int* s_ptr = reinterpret_cast<int*>(x + n + 2);
+  for (int i = threadIdx.x; i < levels_l + levels_u + 2; i += blockDim.x) s_ptr[i] = ptr[i];
+  if (threadIdx.x == 0) {
+    x[n] = T(0);      // a missing entry's word
+    x[n + 1] = T(1);  // a missing row's
+  }
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = y[i];
+  __syncthreads();
+  if ((int)threadIdx.x < nw * 32) {  // the other warps only help to load and store the vector
+    cta_sweep<false, T, W, D, WIDE>(levels_l, chunks_l, s_ptr, cta_smem, nw);
+    cta_sweep<true, T, W, D, WIDE>(levels_u, chunks_u, s_ptr + levels_l + 1, cta_smem, nw);
+  }
+  __syncthreads();
+#pragma unroll 8
+  for (int i = threadIdx.x; i < n; i += blockDim.x) z[i] = x[i];
+}
+
+// Packs one sweep's chunks from the CSR factor (perm: rows by wavefront, whole
+// chunks; after them one chunk without rows).
+template <bool UP, class T, int W>
+__global__ void k_cta_pack(int n, int len, const int* __restrict__ perm, const int* __restrict__ rp,
+                           const int* __restrict__ ci, const int* __restrict__ dcol, const double* __restrict__ lu,
+                           unsigned char* __restrict__ out) {
+  using L = CtaChunk<T, W>;
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= len + 32) return;
+  const int lane = p & 31, row = p < len ? perm[p] : -1;
+  unsigned char* c = out + (size_t)(p >> 5) * L::template bytes<UP>();
+  const int kb = row < 0 ? 0 : UP ? dcol[row] + 1 : rp[row];
+  const int ke = row < 0 ? 0 : UP ? rp[row + 1] : dcol[row];
+  int* ints = reinterpret_cast<int*>(c + L::ints);
+  auto slot = [&](int q) -> int& { return ints[(q / 4 * 32 + lane) * 4 + q % 4]; };
+  slot(0) = (row < 0 ? n + 1 : row) * (int)sizeof(T);
+  T* vals = reinterpret_cast<T*>(c + L::vals);
+  for (int j = 0; j < W; ++j) {
+    const bool in = kb + j < ke;
+    slot(1 + j) = (in ? ci[kb + j] : n) * (int)sizeof(T);
+    vals[(j / 2 * 32 + lane) * 2 + j % 2] = in ? (T)lu[kb + j] : T(0);
+  }
+  for (int q = 1 + W; q < 4 * L::kInts; ++q) slot(q) = n * (int)sizeof(T);
+  if (UP) {
+    // (a row without a diagonal entry divides by 0, as the sweeps across SMs do)
+    const T d = row < 0 ? T(1) : dcol[row] < rp[row + 1] ? (T)lu[dcol[row]] : T(0);
+    if constexpr (sizeof(T) == 8) {
+      reinterpret_cast<double2*>(c + L::rec)[lane] = make_double2(Recip<T>::of(d), d);
+    } else {
+      reinterpret_cast<double*>(c + L::rec)[lane] = Recip<T>::of(d);
+    }
+  }
+}
+
+size_t cta_smem_bytes(int n, const Ilu0Data& d, size_t word) {
+  return ((size_t)n + 2) * word + (size_t)(d.levels_l + d.levels_u + 2) * sizeof(int);
+}
+
+// f(std::integral_constant<int, W>) for the factor's packed row width.
+template <class F>
+void with_cta_width(int W, F&& f) {
+  if (W == 2) f(std::integral_constant<int, 2>());
+  else if (W == 4) f(std::integral_constant<int, 4>());
+  else f(std::integral_constant<int, 8>());
+}
+
+// The chunks of both sweeps in T, from the factor.
+template <class T>
+void cta_pack(ab2_context* ctx, const ab2_matrix* A, const Ilu0Data& d, unsigned char** lo, unsigned char** up) {
+  with_cta_width(d.cta.width, [&](auto w) {
+    constexpr int W = decltype(w)::value;
+    using L = CtaChunk<T, W>;
+    *lo = dev_alloc<unsigned char>(ctx, (size_t)(d.len_l / 32 + 1) * L::template bytes<false>());
+    *up = dev_alloc<unsigned char>(ctx, (size_t)(d.len_u / 32 + 1) * L::template bytes<true>());
+    k_cta_pack<false, T, W><<<(d.len_l + 32 + 255) / 256, 256, 0, ctx->stream>>>(A->n, d.len_l, d.d_perm_l, A->d_rp,
+                                                                                 A->d_ci, A->d_dcol, d.d_lu, *lo);
+    check_launch(ctx, "cta_pack");
+    k_cta_pack<true, T, W><<<(d.len_u + 32 + 255) / 256, 256, 0, ctx->stream>>>(A->n, d.len_u, d.d_perm_u, A->d_rp,
+                                                                                A->d_ci, A->d_dcol, d.d_lu, *up);
+    check_launch(ctx, "cta_pack");
+  });
+}
+
+template <class T>
+void cta_apply(ab2_context* ctx, int n, const Ilu0Data& d, const T* y, T* z) {
+  const Ilu0Data::Cta& t = d.cta;
+  const unsigned char* lo = sizeof(T) == 8 ? t.lo : t.lo32;
+  const unsigned char* up = sizeof(T) == 8 ? t.up : t.up32;
+  const size_t smem = cta_smem_bytes(n, d, sizeof(T));
+  with_cta_width(t.width, [&](auto w) {
+    constexpr int W = decltype(w)::value;
+    auto* k = t.wide ? k_ilu_cta<T, W, true> : k_ilu_cta<T, W, false>;
+    AB2_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kCtaSmemMax));
+    k<<<1, 512, smem, ctx->stream>>>(n, t.warps, d.levels_l, d.levels_u, lo, up, t.ptr, y, z);
+  });
+  check_launch(ctx, "ilu_cta");
+}
+
 // Chebyshev step (ChebyshevPreconditioner.h:392-434 with y_cur the iterate):
 //   r = x - A y_cur ; z = D^-1 r ; p = first ? z : beta*p + z ; y_next = y_cur + a p
 template <class View, class T>
@@ -242,7 +478,9 @@ __global__ void k_pmult2(int n, const T* __restrict__ a, const T* x, T* y) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = mul_rn(a[i], x[i]);
 }
 
-void ilu_symbolic(const ab2_matrix* A, Ilu0Data& d) {
+// Fills d's wavefronts; ptr_u: the backward sweep's wavefront starts (as
+// d.lev_ptr_l), entries: the most entries of a row on one side of the diagonal.
+void ilu_symbolic(const ab2_matrix* A, Ilu0Data& d, std::vector<int>& ptr_u, int* entries) {
   host_profile(A);
   const int n = A->n;
   const int* rp = A->h_rp.data();
@@ -253,6 +491,8 @@ void ilu_symbolic(const ab2_matrix* A, Ilu0Data& d) {
     while (k < rp[i + 1] && ci[k] < i) ++k;
     dc[i] = k;
   }
+  *entries = 0;
+  for (int i = 0; i < n; ++i) *entries = std::max(*entries, std::max(dc[i] - rp[i], rp[i + 1] - dc[i] - 1));
   std::vector<int> lev_l(n, 0), lev_u(n, 0);
   int max_l = -1, max_u = -1;
   for (int i = 0; i < n; ++i) {
@@ -281,7 +521,7 @@ void ilu_symbolic(const ab2_matrix* A, Ilu0Data& d) {
       for (int i = n - 1; i >= 0; --i) perm[fill[lev[i]]++] = i;
     }
   };
-  std::vector<int> perm_u, ptr_u;
+  std::vector<int> perm_u;
   d.levels_l = max_l + 1;
   d.levels_u = max_u + 1;
   build(lev_l, d.levels_l, false, d.h_perm_l, d.lev_ptr_l);
@@ -312,6 +552,39 @@ int sweep_blocks(ab2_context* ctx, int len, int widest_chunks) {
   return std::max(1, std::min(blocks, ctx->num_sms * 8));
 }
 
+// Takes the one-CTA sweeps where the vector fits shared memory, rows have few
+// entries, and they are estimated faster: a wavefront costs 1.45 us across SMs
+// (two-entry rows; more with more), here 0.2 us and 0.25 us for every further pass of
+// the CTA's warps over it, plus 8 us to load and store the vector.  Measured, us an
+// application across SMs / here: 24 x 20 grid 119 / 17, 60 x 60 314 / 38, 181 x 140 944 /
+// 126, 500 x 40 1418 / 163; ragged rows of up to 8 entries, 1,500 rows 344 / 37, 20,011
+// rows (330 wavefronts of up to 4 passes) 1487 / 189.
+void cta_setup(ab2_context* ctx, const ab2_matrix* A, Ilu0Data& d, const std::vector<int>& ptr_u, int entries) {
+  const int n = A->n;
+  if (n == 0 || entries > kCtaMaxEntries || cta_smem_bytes(n, d, sizeof(double)) > (size_t)kCtaSmemMax) return;
+  Ilu0Data::Cta t;
+  const int warps = std::min(16, std::max(d.widest_l, d.widest_u));
+  t.warps = warps;
+  double here = 8.0;
+  for (const std::vector<int>* p : std::initializer_list<const std::vector<int>*>{&d.lev_ptr_l, &ptr_u})
+    for (size_t l = 0; l + 1 < p->size(); ++l) {
+      const int chunks = ((*p)[l + 1] - (*p)[l]) / 32;
+      here += 0.2 + 0.25 * ((chunks + warps - 1) / warps - 1);
+    }
+  if (here >= 1.45 * (d.levels_l + d.levels_u)) return;
+  t.width = entries <= 2 ? 2 : entries <= 4 ? 4 : 8;
+  t.wide = warps < std::max(d.widest_l, d.widest_u);
+  std::vector<int> ptr;
+  for (const std::vector<int>* p : std::initializer_list<const std::vector<int>*>{&d.lev_ptr_l, &ptr_u})
+    for (int v : *p) ptr.push_back(v / 32);
+  d.cta = t;
+  d.cta.ptr = dev_alloc<int>(ctx, ptr.size());
+  AB2_CUDA(cudaMemcpyAsync(d.cta.ptr, ptr.data(), sizeof(int) * ptr.size(), cudaMemcpyHostToDevice, ctx->stream));
+  cta_pack<double>(ctx, A, d, &d.cta.lo, &d.cta.up);
+  AB2_CUDA(cudaStreamSynchronize(ctx->stream));  // (the copy's source is a local)
+  d.cta.use = true;
+}
+
 }  // namespace
 
 void ilu_init(ab2_context* ctx, ab2_precond* pc, int schedule, const double* lu) {
@@ -330,9 +603,10 @@ void ilu_init(ab2_context* ctx, ab2_precond* pc, int schedule, const double* lu)
   if (schedule != AB2_ILU_WAVEFRONT && ilu_stencil_setup(ctx, A, d, lu != nullptr, schedule)) return;
   require(schedule != AB2_ILU_STENCIL && schedule != AB2_ILU_STENCIL_CLUSTER,
           "ILU0 tile schedule requested but the matrix is not a 3-D 7-point matrix in lexicographic order");
-  ilu_symbolic(A, d);
-  if (lu) return;
-  for (int l = 1; l < d.levels_l; ++l) {  // wavefront 0 rows have nothing left of the diagonal
+  std::vector<int> ptr_u;
+  int entries = 0;
+  ilu_symbolic(A, d, ptr_u, &entries);
+  for (int l = 1; !lu && l < d.levels_l; ++l) {  // wavefront 0 rows have nothing left of the diagonal
     const int a = d.lev_ptr_l[l], b = d.lev_ptr_l[l + 1];
     const int cnt = b - a;
     if (cnt == 0) continue;
@@ -340,11 +614,13 @@ void ilu_init(ab2_context* ctx, ab2_precond* pc, int schedule, const double* lu)
                                                                    d.d_lu);
     check_launch(ctx, "ilu_factor");
   }
+  if (schedule == AB2_ILU_AUTO) cta_setup(ctx, A, d, ptr_u, entries);
 }
 
 void ilu_drop_schedule(ab2_context* ctx, Ilu0Data& d) {
   for (void* p : {(void*)d.d_perm_l, (void*)d.d_perm_u, (void*)d.d_tmp, (void*)d.d_counters, (void*)d.d_err,
-                  (void*)d.d_bands, (void*)d.d_walk, (void*)d.d_walk32, (void*)d.d_tile_tickets})
+                  (void*)d.d_bands, (void*)d.d_walk, (void*)d.d_walk32, (void*)d.d_tile_tickets, (void*)d.cta.ptr,
+                  (void*)d.cta.lo, (void*)d.cta.up, (void*)d.cta.lo32, (void*)d.cta.up32})
     dev_free(ctx, p);
   double* lu = d.d_lu;
   d = Ilu0Data{};
@@ -541,6 +817,10 @@ void apply_t(ab2_context* ctx, const ab2_precond* pc, const T* x, T* y) {
         else ilu_stencil_apply_f32(ctx, d, x, y);
         break;
       }
+      if (d.cta.use) {
+        cta_apply<T>(ctx, n, d, x, y);
+        break;
+      }
       k_ilu_lsweep<T><<<sweep_blocks(ctx, d.len_l, d.widest_l), 256, 0, ctx->stream>>>(
           d.len_l, d.d_perm_l, A->d_rp, A->d_ci, A->d_dcol, w.lu, x, w.tmp, y, d.d_counters, d.d_err);
       check_launch(ctx, "ilu_lsweep");
@@ -612,6 +892,8 @@ void pc_enable_f32(ab2_context* ctx, ab2_precond* pc) {
   if (pc->kind == AB2_PC_ILU0) {
     if (pc->ilu.stencil) {
       ilu_stencil_enable_f32(ctx, pc->ilu);
+    } else if (pc->ilu.cta.use) {
+      cta_pack<float>(ctx, A, pc->ilu, &pc->ilu.cta.lo32, &pc->ilu.cta.up32);
     } else {
       pc->d_lu32 = dev_alloc<float>(ctx, (size_t)A->nnz);
       op_to_f32(ctx, A->nnz, pc->ilu.d_lu, pc->d_lu32);
@@ -718,6 +1000,11 @@ int ab2_precond_destroy(ab2_precond* pc) {
   dev_free(pc->ctx, pc->ilu.d_walk);
   dev_free(pc->ctx, pc->ilu.d_walk32);
   dev_free(pc->ctx, pc->ilu.d_tile_tickets);
+  {
+    const Ilu0Data::Cta& t = pc->ilu.cta;
+    for (void* p : {(void*)t.ptr, (void*)t.lo, (void*)t.up, (void*)t.lo32, (void*)t.up32})
+      dev_free(pc->ctx, p);
+  }
   dev_free(pc->ctx, pc->cheb.d_p);
   dev_free(pc->ctx, pc->cheb.d_y[0]);
   dev_free(pc->ctx, pc->cheb.d_y[1]);

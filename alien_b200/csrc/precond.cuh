@@ -37,6 +37,16 @@ struct Ilu0Data {
   // coefficients of both sweeps, the forward sweep's output, hand-over words.
   double* d_walk = nullptr;
   float* d_walk32 = nullptr;  // the same in FP32 (mixed-precision inner solves), built on demand
+  // Small factors of other matrices: both sweeps by one CTA (precond.cu).
+  struct Cta {
+    bool use = false;
+    int width = 0;               // packed entries of a row
+    int warps = 0;               // that run the sweeps
+    bool wide = false;           // some wavefront has more chunks than that
+    int* ptr = nullptr;          // 32-row chunks before each wavefront: levels_l + 1, then levels_u + 1
+    unsigned char *lo = nullptr, *up = nullptr;  // the sweeps' chunks
+    unsigned char *lo32 = nullptr, *up32 = nullptr;
+  } cta;
   bool walk_cluster = false;  // the name the walk is reported by (AB2_ILU_STENCIL_CLUSTER)
 };
 

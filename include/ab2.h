@@ -217,7 +217,8 @@ int ab2_dot_noalloc(const double* x, const double* y, int n, double* result, voi
  * STENCIL_CLUSTER: the same walk, for up to 346 planes along z (a request
  *   beyond that is refused).
  * AUTO: STENCIL_CLUSTER, else STENCIL when the matrix has that structure,
- *   else WAVEFRONT. */
+ *   else WAVEFRONT (small factors with narrow wavefronts then run both sweeps
+ *   in one CTA, the vector in its shared memory). */
 #define AB2_ILU_AUTO 0
 #define AB2_ILU_WAVEFRONT 1
 #define AB2_ILU_STENCIL 2

@@ -175,3 +175,80 @@ def test_ilu0_strip_walk_division_range(ctx, dims, scale):
         got = vx.download()
         np.testing.assert_array_equal(got, ref)
         np.testing.assert_array_equal(np.signbit(got)[~np.isnan(ref)], np.signbit(ref)[~np.isnan(ref)])
+
+
+def _csr(n, rows):
+    """CSR from {row: {col: value}}."""
+    rp, ci, vv = [0], [], []
+    for i in range(n):
+        for c in sorted(rows[i]):
+            ci.append(c)
+            vv.append(rows[i][c])
+        rp.append(len(ci))
+    return np.asarray(rp, np.int32), np.asarray(ci, np.int32), np.asarray(vv)
+
+
+def _random_rows(n, most, span, seed, dense_levels=False):
+    rng = np.random.default_rng(seed)
+    rows = []
+    for i in range(n):
+        r = {i: 4.0 + rng.uniform()}
+        # dense_levels: every row hangs on row 0 only
+        cols = [0] if dense_levels else rng.integers(max(0, i - span), i + 1, rng.integers(0, most + 1))
+        for c in cols:
+            if c != i:
+                r[int(c)] = -rng.uniform()
+        rows.append(r)
+    for i in range(n):  # the same on the other side of the diagonal
+        for c in list(rows[i]):
+            if c < i and len([k for k in rows[c] if k > c]) < most:
+                rows[c][i] = -rng.uniform()
+    return _csr(n, rows)
+
+
+# Both sweeps by one CTA (AUTO on small factors of matrices that are no 3-D grid)
+# against the sequential sweeps and the sweeps across SMs: narrow and wide
+# wavefronts, one to nine entries a side (nine is past what is packed), right-hand
+# sides outside the fast division's range, FP64 limits of shared memory.
+@pytest.mark.parametrize("kind", ["n1", "two", "eight", "nine", "wide", "grid", "limit", "past_limit", "nodiag"])
+def test_ilu0_one_cta_sweeps_bit_exact(ctx, kind):
+    if kind == "n1":
+        rp, ci, vv = _csr(1, [{0: 3.0}])
+    elif kind == "two":
+        rp, ci, vv = _random_rows(700, 2, 40, 1)
+    elif kind == "eight":
+        rp, ci, vv = _random_rows(900, 8, 60, 2)
+    elif kind == "nine":
+        n = 400
+        rows = [{c: (12.0 if c == i else -0.3 - 0.01 * (c % 7)) for c in range(max(0, i - 9), min(n, i + 10))}
+                for i in range(n)]
+        rp, ci, vv = _csr(n, rows)
+    elif kind == "wide":
+        rp, ci, vv = _random_rows(3000, 2, 10, 3, dense_levels=True)
+    elif kind == "nodiag":
+        rp, ci, vv = _csr(40, [{c: (2.0 if c == i else -0.5) for c in (i - 1, i, i + 1)
+                                if 0 <= c < 40 and not (i == 20 and c == 20)} for i in range(40)])
+    else:
+        nx, ny = {"grid": (61, 47), "limit": (165, 169), "past_limit": (170, 170)}[kind]
+        P = abi.diffusion(nx, ny, 1, sigma=1.0, smooth=2.0, seed=4)
+        rp, ci, vv = P.row_ptr, P.cols, P.vals
+    n = rp.size - 1
+    A = ctx.matrix(rp, ci, vv)
+    auto, across = abi.Precond(ctx, A, "ilu0"), abi.Precond(ctx, A, "ilu0", ilu_schedule="wavefront")
+    y0 = rnd(n, 7)
+    zeros = np.where(np.arange(n) % 3 == 0, y0, -0.0)
+    inf = y0.copy()
+    inf[n // 2] = np.inf
+    for y in (y0, zeros, y0 * 1e-290, y0 * 1e160, np.zeros(n), inf, y0):
+        out = []
+        for pc in (auto, across):
+            vx = ctx.vector(n)
+            pc.apply(ctx.vector(y), vx)
+            out.append(vx.download())
+        with np.errstate(all="ignore"):
+            ref = O.ilu0_apply(rp, ci, vv, y)
+        np.testing.assert_array_equal(out[0], ref)
+        np.testing.assert_array_equal(out[0], out[1])
+    v = ctx.vector(y0)
+    auto.apply(v, v)  # in place
+    np.testing.assert_array_equal(v.download(), O.ilu0_apply(rp, ci, vv, y0))
