@@ -392,14 +392,14 @@ void cta_apply(ab2_context* ctx, int n, const Ilu0Data& d, const T* y, T* z) {
 template <class View, class T>
 __global__ void __launch_bounds__(kThreads) k_cheb_step(int n, View A, const T* __restrict__ x, const T* __restrict__ ycur,
                                                         const T* __restrict__ inv, T* __restrict__ p,
-                                                        T* __restrict__ ynext, T a, T bcoef, int first) {
+                                                        T* __restrict__ ynext, T a, T bcoef, int first, int last) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= n) return;
   const T ay = A.row(row, ycur);
   const T r = fma_rn(T(-1), ay, x[row]);
   const T z = mul_rn(inv[row], r);
   const T pn = first ? z : add_rn(mul_rn(bcoef, p[row]), z);
-  p[row] = pn;
+  if (!last) p[row] = pn;
   ynext[row] = fma_rn(a, pn, ycur[row]);
 }
 
@@ -417,21 +417,48 @@ __global__ void k_cheb1_start(int n, const T* x, const T* __restrict__ inv, T in
   }
 }
 
+// The start and the first step in one pass (x and y different vectors): the
+// step forms w = (D^-1 x) / theta at every row it reads, so neither r, w nor y is
+// stored and read back in between (40 bytes a row stored or read less in FP64, of
+// 128).  last: nothing comes after, r and w are not stored.
+template <class View, class T>
+__global__ void __launch_bounds__(kThreads) k_cheb1_first(int n, View A, const T* __restrict__ x,
+                                                          const T* __restrict__ inv, T inv_theta, T* __restrict__ r,
+                                                          T* __restrict__ wnext, T* __restrict__ y, T c1, T c2,
+                                                          int last) {
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= n) return;
+  const T ir = inv[row];
+  const T r0 = mul_rn(ir, x[row]), w0 = mul_rn(inv_theta, r0);
+  auto w = [&](int c) { return mul_rn(inv_theta, mul_rn(__ldg(inv + c), __ldg(x + c))); };
+  const T my = mul_rn(ir, A.row_f(row, w));
+  const T rv = fma_rn(T(-1), my, r0);
+  const T wv = fma_rn(c2, rv, mul_rn(c1, w0));
+  if (!last) {
+    r[row] = rv;
+    wnext[row] = wv;
+  }
+  y[row] = fma_rn(T(1), wv, w0);
+}
+
 // _algo1 step (:342-354): r -= D^-1 A w ; w = c1 w + c2 r ; y += w, with the
-// rounding of pointwiseMult, axpy(-1), scal, axpy(c2), axpy(1).
+// rounding of pointwiseMult, axpy(-1), scal, axpy(c2), axpy(1).  last: r and w are
+// not stored.
 template <class View, class T>
 __global__ void __launch_bounds__(kThreads) k_cheb1_step(int n, View A, const T* __restrict__ inv, T* __restrict__ r,
                                                          const T* __restrict__ wcur, T* __restrict__ wnext,
-                                                         T* __restrict__ y, T c1, T c2) {
+                                                         T* __restrict__ y, T c1, T c2, int last) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= n) return;
   // mul_rn: the products are rounded on their own, as pointwiseMult and
   // scal round them; a plain '*' could be fused into the following update.
   const T my = mul_rn(inv[row], A.row(row, wcur));
   const T rv = fma_rn(T(-1), my, r[row]);
-  r[row] = rv;
   const T wv = fma_rn(c2, rv, mul_rn(c1, wcur[row]));
-  wnext[row] = wv;
+  if (!last) {
+    r[row] = rv;
+    wnext[row] = wv;
+  }
   y[row] = fma_rn(T(1), wv, y[row]);
 }
 
@@ -835,14 +862,25 @@ void apply_t(ab2_context* ctx, const ab2_precond* pc, const T* x, T* y) {
       if (c.saad) {
         T* r = w.p;
         T* wv[2] = {w.y0, w.y1};
-        k_cheb1_start<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, x, w.inv, (T)c.inv_theta, r, wv[0], y);
-        check_launch(ctx, "cheb1_start");
-        for (int k = 1; k < steps; ++k) {
+        const int blocks = (n + kThreads - 1) / kThreads;
+        int k = 1;
+        if (steps > 1 && x != y) {
+          with_view<T>(pc->A, pc->variant, [&](auto view) {
+            k_cheb1_first<<<blocks, kThreads, 0, ctx->stream>>>(n, view, x, w.inv, (T)c.inv_theta, r, wv[1], y,
+                                                                (T)c.a[1], (T)c.b[1], steps == 2);
+          });
+          check_launch(ctx, "cheb1_first");
+          k = 2;
+        } else {
+          k_cheb1_start<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, x, w.inv, (T)c.inv_theta, r, wv[0], y);
+          check_launch(ctx, "cheb1_start");
+        }
+        for (; k < steps; ++k) {
           const T* wcur = wv[(k - 1) & 1];
           T* wnext = wv[k & 1];
           with_view<T>(pc->A, pc->variant, [&](auto view) {
-            k_cheb1_step<<<(n + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(n, view, w.inv, r, wcur, wnext,
-                                                                                      y, (T)c.a[k], (T)c.b[k]);
+            k_cheb1_step<<<blocks, kThreads, 0, ctx->stream>>>(n, view, w.inv, r, wcur, wnext, y, (T)c.a[k], (T)c.b[k],
+                                                               k + 1 == steps);
           });
           check_launch(ctx, "cheb1_step");
         }
@@ -859,7 +897,7 @@ void apply_t(ab2_context* ctx, const ab2_precond* pc, const T* x, T* y) {
         T* next = (i == steps - 1) ? y : ys[i & 1];
         with_view<T>(pc->A, pc->variant, [&](auto view) {
           k_cheb_step<<<(n + kThreads - 1) / kThreads, kThreads, 0, ctx->stream>>>(n, view, xin, cur, w.inv, w.p, next,
-                                                                                   (T)c.a[i], (T)c.b[i], i == 0);
+                                                                                   (T)c.a[i], (T)c.b[i], i == 0, i + 1 == steps);
         });
         check_launch(ctx, "cheb_step");
         cur = next;

@@ -252,3 +252,25 @@ def test_ilu0_one_cta_sweeps_bit_exact(ctx, kind):
     v = ctx.vector(y0)
     auto.apply(v, v)  # in place
     np.testing.assert_array_equal(v.download(), O.ilu0_apply(rp, ci, vv, y0))
+
+
+@pytest.mark.parametrize("saad", [True, False])
+@pytest.mark.parametrize("order", [1, 2, 3, 5])
+@pytest.mark.parametrize("name", ["poisson16", "ragged", "convdiff_10x11x12"])
+def test_chebyshev_first_and_last_step(ctx, name, order, saad):
+    """The start fused into the first step (different vectors) and not (in
+    place), and the last step's skipped stores: the oracle's bits in both,
+    repeatedly."""
+    P = problems.get(name)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals)
+    pc = abi.Precond(ctx, A, "cheb", poly_factor=0.0, poly_order=order, poly_factor_max_iter=12, cheb_saad=saad)
+    tb = ctx.info.reduction_max_blocks
+    for seed in range(2):
+        x = rnd(P.n, seed)
+        exact = O.cheb_apply(P.row_ptr, P.cols, P.vals, x, 0.0, order, 12, dot_mode=O.DOT_DEVICE_TREE, tree_blocks=tb,
+                             saad=saad)
+        vx, vy = ctx.vector(x), ctx.vector(P.n)
+        pc.apply(vx, vy)
+        np.testing.assert_array_equal(vy.download(), exact)
+        pc.apply(vx, vx)
+        np.testing.assert_array_equal(vx.download(), exact)
