@@ -32,7 +32,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <initializer_list>
-#include <random>
 #include <type_traits>
 
 #include "ab2_internal.cuh"
@@ -462,6 +461,66 @@ __global__ void __launch_bounds__(kThreads) k_cheb1_step(int n, View A, const T*
   y[row] = fma_rn(T(1), wv, y[row]);
 }
 
+// x[i] = U(-1, 1) as a default-seeded std::mt19937 and a
+// std::uniform_real_distribution<double>(-1, 1) draw them in index order: two
+// 32-bit words a value, (a + 2^32 b) / 2^64 rounded once.  The generator is the
+// published one (M. Matsumoto, T. Nishimura, "Mersenne Twister", ACM TOMACS 8, 1998):
+// word k of a generation of 624 needs words k, k + 1 and k + 397 of the last one, or
+// word k - 227 of its own, so a generation is three rounds of up to 227 words for
+// one CTA (warps 0-7), while the other warps turn the last generation's words into
+// values.  One CTA because generation follows generation; the host drew 3.5 million values
+// in 15 ms and copied them in another 3, this takes 3.6 ms.
+constexpr int kMtN = 624, kMtM = 397;
+constexpr int kMtGen = 256, kMtOut = 320;  // threads of the two parts
+__global__ void __launch_bounds__(kMtGen + kMtOut, 1) k_mt_uniform(int n, double* __restrict__ x) {
+  __shared__ unsigned s_w[2][kMtN];
+  if (threadIdx.x == 0) {  // the seeding recurrence
+    unsigned w = 5489u;
+    s_w[0][0] = w;
+    for (int i = 1; i < kMtN; ++i) s_w[0][i] = w = 1812433253u * (w ^ (w >> 30)) + (unsigned)i;
+  }
+  const int gens = (n + kMtN / 2 - 1) / (kMtN / 2);
+  for (int g = 0; g <= gens; ++g) {
+    __syncthreads();
+    const unsigned* old = s_w[g & 1];
+    unsigned* now = s_w[(g + 1) & 1];
+    if (threadIdx.x < kMtGen) {
+      if (g == gens) continue;
+      const int t = threadIdx.x;
+      auto word = [&](unsigned hi, unsigned lo, unsigned far) {
+        const unsigned y = (hi & 0x80000000u) | (lo & 0x7FFFFFFFu);
+        return far ^ (y >> 1) ^ ((y & 1u) ? 0x9908B0DFu : 0u);
+      };
+      constexpr int kBack = kMtN - kMtM;  // 227
+      const unsigned a = t < kBack ? old[t] : 0u, a1 = t < kBack ? old[t + 1] : 0u, af = t < kBack ? old[t + kMtM] : 0u;
+      const unsigned b = t < kBack ? old[t + kBack] : 0u, b1 = t < kBack ? old[t + kBack + 1] : 0u;
+      const int k2 = t + 2 * kBack;
+      const bool third = t < kBack && k2 < kMtN;
+      const unsigned c = third ? old[k2] : 0u, c1 = third && k2 + 1 < kMtN ? old[k2 + 1] : 0u;
+      if (t < kBack) now[t] = word(a, a1, af);
+      asm volatile("bar.sync 1, %0;" ::"n"(kMtGen) : "memory");
+      if (t < kBack) now[t + kBack] = word(b, b1, now[t]);
+      asm volatile("bar.sync 1, %0;" ::"n"(kMtGen) : "memory");
+      if (third) now[k2] = word(c, k2 + 1 < kMtN ? c1 : now[0], now[k2 - kBack]);
+    } else if (g > 0) {  // generation g - 1's words are `old`
+      const int v = (int)threadIdx.x - kMtGen;
+      const int i = (g - 1) * (kMtN / 2) + v;
+      if (v < kMtN / 2 && i < n) {
+        auto temper = [](unsigned y) {
+          y ^= y >> 11;
+          y ^= (y << 7) & 0x9D2C5680u;
+          y ^= (y << 15) & 0xEFC60000u;
+          return y ^ (y >> 18);
+        };
+        const double sum = __dadd_rn((double)temper(old[2 * v]), __dmul_rn((double)temper(old[2 * v + 1]), 4294967296.0));
+        double u = __dmul_rn(sum, 5.421010862427522e-20);  // 2^-64
+        if (u >= 1.0) u = 0x1.fffffffffffffp-1;             // the largest double below 1
+        x[i] = __dadd_rn(__dmul_rn(u, 2.0), -1.0);
+      }
+    }
+  }
+}
+
 __global__ void k_sqrt(int n, const double* __restrict__ a, double* __restrict__ s) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) s[i] = sqrt(a[i]);
 }
@@ -674,12 +733,12 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
   op_fill(ctx, n, 0.0, c.d_p);
   // Both power methods draw their start vector from a default-seeded
   // std::mt19937 with U(-1,1), index order (computeBeta :124-129, computeAlpha :166-172).
-  std::vector<double> h(n);
+  auto start = [&] {
+    k_mt_uniform<<<1, kMtGen + kMtOut, 0, ctx->stream>>>(n, x);
+    check_launch(ctx, "mt_uniform");
+  };
   auto power = [&](bool shift, double b) {
-    std::mt19937 gen;
-    std::uniform_real_distribution<> dis(-1., 1.);
-    for (int i = 0; i < n; ++i) h[i] = dis(gen);
-    AB2_CUDA(cudaMemcpyAsync(x, h.data(), sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    start();
     op_dot(ctx, n, x, x, s);
     const double nrm = std::sqrt(read_scalar(ctx, s));
     op_scal(ctx, n, 1 / nrm, x);
@@ -709,10 +768,7 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
     double* w = c.d_xcopy;  // free until the first application
     k_sqrt<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, pc->d_inv, s);
     check_launch(ctx, "sqrt");
-    std::mt19937 gen;
-    std::uniform_real_distribution<> dis(-1., 1.);
-    for (int i = 0; i < n; ++i) h[i] = dis(gen);
-    AB2_CUDA(cudaMemcpyAsync(x, h.data(), sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
+    start();
     op_dot(ctx, n, x, x, s_out);
     const double nrm = std::sqrt(read_scalar(ctx, s_out));
     op_scal(ctx, n, 1 / nrm, x);

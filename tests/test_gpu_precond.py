@@ -274,3 +274,18 @@ def test_chebyshev_first_and_last_step(ctx, name, order, saad):
         np.testing.assert_array_equal(vy.download(), exact)
         pc.apply(vx, vx)
         np.testing.assert_array_equal(vx.download(), exact)
+
+
+@pytest.mark.parametrize("n", [1, 2, 311, 312, 313, 624, 1249, 40000])
+def test_chebyshev_start_vector_drawn_on_the_device(ctx, n):
+    """The power method's start vector (a default-seeded mt19937) around the
+    generator's block sizes: the oracle's bounds, bit for bit."""
+    rng = np.random.default_rng(n)
+    rp, ci, vals = _csr(n, [{c: (rng.uniform(2.5, 4.0) if c == i else -1.0) for c in (i - 1, i, i + 1) if 0 <= c < n}
+                            for i in range(n)])
+    A = ctx.matrix(rp, ci, vals)
+    pc = abi.Precond(ctx, A, "cheb", poly_factor=0.0, poly_order=3, poly_factor_max_iter=3)
+    with np.errstate(all="ignore"):  # (n = 1: D^-1 A is the identity, the shifted method divides 0 by 0)
+        bounds = O.cheb_bounds(rp, ci, vals, 0.0, 3, dot_mode=O.DOT_DEVICE_TREE,
+                               tree_blocks=ctx.info.reduction_max_blocks)
+    np.testing.assert_array_equal([pc.info.cheb_alpha, pc.info.cheb_beta], bounds)
