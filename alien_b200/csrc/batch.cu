@@ -103,8 +103,68 @@ __device__ __forceinline__ void cluster_sum(T (&acc)[NC], T (*s_part)[4], T (*s_
   }
 }
 
-template <class V64, class V32>
-__global__ void k_batch_cg(BatchArgs<V64, V32> a) {
+// U rows' sums at once, x[c] given by f(c): every load of all rows before the first
+// is used, each row summed as row_f sums it.  r[u] < 0: no row.
+template <class V, class T, int U, class F>
+__device__ __forceinline__ void rows_f(const V& A, const int (&r)[U], F&& f, T (&out)[U]) {
+#pragma unroll
+  for (int u = 0; u < U; ++u) out[u] = r[u] >= 0 ? A.row_f(r[u], f) : T(0);
+}
+template <class T, int S, int U, class F>
+__device__ __forceinline__ void rows_f(const EllViewS<T, S>& A, const int (&r)[U], F&& f, T (&out)[U]) {
+  int w[U], widest = 0;
+  const int* cp[U];
+  const T* vp[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int q = r[u] >= 0 ? r[u] : 0;
+    const int o = A.off[q / S];
+    w[u] = r[u] >= 0 ? A.off[q / S + 1] - o : 0;
+    const size_t base = (size_t)o * S + q % S;
+    cp[u] = A.ci + base;
+    vp[u] = A.v + base;
+    out[u] = T(0);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) widest = max(widest, w[u]);
+  for (int j = 0; j < widest; j += 8) {
+    int c[U][8];
+    T a[U][8], x[U][8];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const bool in = j + k < w[u];
+        c[u][k] = in ? __ldcs(cp[u] + (size_t)(j + k) * S) : -1;
+        a[u][k] = in ? __ldcs(vp[u] + (size_t)(j + k) * S) : T(0);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) x[u][k] = c[u][k] >= 0 ? f(c[u][k]) : T(0);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (c[u][k] >= 0) out[u] = mul_add_rn(a[u][k], x[u][k], out[u]);
+  }
+}
+
+// The kernel in three builds, the same arithmetic in the same order.  A thread
+// that takes its rows one after another is a chain of waits on L2 (47 rows each for
+// 192,721 rows on 8 x 512 threads); rows side by side take registers, and with
+// them clusters off the GPU.  Dense: one row of the SpMV and four of the update at a
+// time, 64 registers, two CTAs of 512 threads an SM.  Deep: two rows of the SpMV, 128
+// registers, one CTA of 512 an SM.  Any: one row, for CTAs of up to 1,024 threads.
+enum class Build { Any, Dense, Deep };
+template <Build B>
+constexpr int kSpmvRows = B == Build::Deep ? 2 : 1;
+template <Build B>
+constexpr int kUpdateRows = B == Build::Any ? 1 : 4;
+
+template <class V64, class V32, Build BUILD>
+__global__ void __launch_bounds__(BUILD == Build::Any ? 1024 : 512, BUILD == Build::Dense ? 2 : 1)
+    k_batch_cg(BatchArgs<V64, V32> a) {
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double s_part64[2][4];
   __shared__ float s_part32[2][4];
@@ -186,26 +246,55 @@ __global__ void k_batch_cg(BatchArgs<V64, V32> a) {
           const bool first = it == 0;
           auto pval = [&](int c) { return first ? a.z[c] : __fmaf_rn(beta, pold[c], a.z[c]); };
           float pq[1] = {0.f};
-          for (int i = lo + threadIdx.x; i < hi; i += T) {
-            const float qv = a.A32.row_f(i, pval);
-            const float pv = pval(i);
-            pcur[i] = pv;
-            a.q[i] = qv;
-            pq[0] = __fmaf_rn(pv, qv, pq[0]);
+          constexpr int US = kSpmvRows<BUILD>, UU = kUpdateRows<BUILD>;
+          for (int i0 = lo + threadIdx.x; i0 < hi; i0 += US * T) {
+            int row[US];
+            float qv[US], pv[US];
+#pragma unroll
+            for (int u = 0; u < US; ++u) {
+              row[u] = i0 + u * T < hi ? i0 + u * T : -1;
+              pv[u] = row[u] >= 0 ? pval(row[u]) : 0.f;
+            }
+            rows_f(a.A32, row, pval, qv);
+#pragma unroll
+            for (int u = 0; u < US; ++u)
+              if (row[u] >= 0) {
+                pcur[row[u]] = pv[u];
+                a.q[row[u]] = qv[u];
+                pq[0] = __fmaf_rn(pv[u], qv[u], pq[0]);
+              }
           }
           cluster_sum<1>(pq, s_part32, s_warp32, slot, cluster);
           slot ^= 1;
           if (pq[0] == 0.f) break;  // breakdown "alpha": keep the correction so far
           const float alpha = rho / pq[0];
           float rz[2] = {0.f, 0.f};
-          for (int i = lo + threadIdx.x; i < hi; i += T) {
-            a.d[i] = __fmaf_rn(alpha, pcur[i], a.d[i]);
-            const float rv = __fmaf_rn(-alpha, a.q[i], a.r[i]);
-            a.r[i] = rv;
-            const float zv = __fmul_rn(a.inv32[i], rv);
-            a.z[i] = zv;
-            rz[0] = __fmaf_rn(rv, zv, rz[0]);
-            rz[1] = __fmaf_rn(rv, rv, rz[1]);
+          for (int i0 = lo + threadIdx.x; i0 < hi; i0 += UU * T) {
+            float dv[UU], pv[UU], qv[UU], rv[UU], iv[UU];
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+              const int i = i0 + u * T;
+              if (i < hi) {
+                dv[u] = a.d[i];
+                pv[u] = pcur[i];
+                qv[u] = a.q[i];
+                rv[u] = a.r[i];
+                iv[u] = a.inv32[i];
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < UU; ++u) {
+              const int i = i0 + u * T;
+              if (i < hi) {
+                a.d[i] = __fmaf_rn(alpha, pv[u], dv[u]);
+                const float rn = __fmaf_rn(-alpha, qv[u], rv[u]);
+                a.r[i] = rn;
+                const float zv = __fmul_rn(iv[u], rn);
+                a.z[i] = zv;
+                rz[0] = __fmaf_rn(rn, zv, rz[0]);
+                rz[1] = __fmaf_rn(rn, rn, rz[1]);
+              }
+            }
           }
           cluster_sum<2>(rz, s_part32, s_warp32, slot, cluster);
           slot ^= 1;
@@ -307,6 +396,7 @@ struct ab2_batch {
   int tuned = 0;
   double tune_ms = 0, setup_ms = 0, solve_ms = 0;
   std::vector<ab2_batch_trial> trials;
+  std::vector<double> work;  // rows^1.5 of the first k systems, largest first
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
@@ -358,15 +448,42 @@ bool launch_batch(ab2_batch* B, V64 a64, V32 a32, int csize, int threads, const 
   cfg.stream = ctx->stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (csize > 8)  // 16-CTA clusters are beyond the portable size
-    AB2_CUDA(cudaFuncSetAttribute(k_batch_cg<V64, V32>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  // Dense or deep: with the work of a system taken as rows^1.5 (iterations grow
+  // with the side of a 2-D grid), deep where the largest system is more than two
+  // thirds of what each of the dense build's clusters has to do on average -- it
+  // then ends the launch, and its own pace counts -- else dense.  Measured on B200
+  // (8 x 512, ms; before, dense, deep; total work over the largest's): 24 systems of up
+  // to 200,000 rows (3.8) 431, 339, 220; 96 (14) 611, 524, 311; 96 of up to 50,000 (20)
+  // 92, 83, 49; 192 of up to 100,000 (34) 253, 215, 194; 512 of up to 200,000 (75)
+  // 1234, 987, 1088.
+  auto fit = [&](auto* k) {
+    if (csize > 8)  // 16-CTA clusters are beyond the portable size
+      AB2_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    int c = 0;
+    AB2_CUDA(cudaOccupancyMaxActiveClusters(&c, (void*)k, &cfg));
+    return c;
+  };
+  auto* kernel = k_batch_cg<V64, V32, Build::Any>;
   int nclusters = 0;
-  AB2_CUDA(cudaOccupancyMaxActiveClusters(&nclusters, (void*)k_batch_cg<V64, V32>, &cfg));
+  if (threads <= 512) {
+    kernel = k_batch_cg<V64, V32, Build::Dense>;
+    nclusters = fit(kernel);
+    if (1.5 * B->work[1] * nclusters > B->work[nsys_run]) {
+      auto* deep = k_batch_cg<V64, V32, Build::Deep>;
+      const int c = fit(deep);
+      if (c >= 1) {
+        kernel = deep;
+        nclusters = c;
+      }
+    }
+  } else {
+    nclusters = fit(kernel);
+  }
   if (nclusters < 1) return false;
   nclusters = std::min(nclusters, nsys_run);
   cfg.gridDim = dim3((unsigned)(nclusters * csize));
   AB2_CUDA(cudaMemsetAsync(B->d_ticket, 0, sizeof(unsigned int), ctx->stream));
-  AB2_CUDA(cudaLaunchKernelEx(&cfg, k_batch_cg<V64, V32>, args));
+  AB2_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
   check_launch(ctx, "batch_cg");
   return true;
 }
@@ -546,6 +663,8 @@ int ab2_batch_create(ab2_context* ctx, const ab2_matrix* A, int nsys, const int*
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
       return sys_offsets[a + 1] - sys_offsets[a] > sys_offsets[b + 1] - sys_offsets[b];
     });
+    B->work.assign(1, 0.0);
+    for (int i : order) B->work.push_back(B->work.back() + std::pow((double)(sys_offsets[i + 1] - sys_offsets[i]), 1.5));
     B->d_off = dev_alloc<int>(ctx, (size_t)nsys + 1);
     B->d_order = dev_alloc<int>(ctx, (size_t)nsys);
     AB2_CUDA(cudaMemcpyAsync(B->d_off, sys_offsets, sizeof(int) * ((size_t)nsys + 1), cudaMemcpyHostToDevice,

@@ -123,3 +123,21 @@ def test_batch_rejects_bad_input(ctx, batch):
         with pytest.raises(abi.AB2Error) as e:
             abi.Batch(ctx, *args, **kw)
         assert e.value.code == abi.AB2_ERR_BAD_ARG
+
+
+# Many systems of a size run on the kernel's dense build, a few on its deep one
+# (rows taken side by side): the same bits as the oracle in both, on systems with
+# fewer rows than a CTA has threads, ragged last rows and widths past one group of
+# slots.
+@pytest.mark.parametrize("nsys,cluster,threads", [(700, 1, 64), (300, 2, 128), (3, 2, 128), (1, 4, 256), (2, 1, 512)])
+def test_batch_dense_and_deep_builds(ctx, nsys, cluster, threads):
+    B = abi.batch_problem(nsys=nsys, min_rows=60, max_rows=90 if nsys > 100 else 3000, seed=11)
+    for slice_rows in (32, 64):
+        S, st, x = run(ctx, B, tol=1e-8, spmv_variant=abi.SPMV_ELL, cluster_size=cluster, threads=threads,
+                       ell_slice=slice_rows)
+        P = B.problem
+        o = O.batch_solve(P.row_ptr, P.cols, P.vals, B.sys_offsets, P.b, tol=1e-8, cluster_size=cluster,
+                          threads=threads, lanes_per_row=1)
+        np.testing.assert_array_equal(x, o.x)
+        np.testing.assert_array_equal(S.results()[2], o.inner)
+        S.close()
