@@ -252,6 +252,25 @@ double read_scalar(ab2_context* ctx, const double* d) {
   return ctx->h_pinned[0];
 }
 
+// A double of the pinned staging memory (device-writable) that nothing else uses.
+static double* host_result(ab2_context* ctx) { return ctx->h_pinned + 63; }
+static double wait_result(ab2_context* ctx) {
+  AB2_CUDA(cudaStreamSynchronize(ctx->stream));
+  return *static_cast<volatile double*>(host_result(ctx));
+}
+double dot_value(ab2_context* ctx, int n, const double* x, const double* y) {
+  op_dot(ctx, n, x, y, host_result(ctx), 0);
+  return wait_result(ctx);
+}
+double norm0_value(ab2_context* ctx, int n, const double* x) {
+  op_norm0(ctx, n, x, host_result(ctx), 0);
+  return wait_result(ctx);
+}
+double norm1_value(ab2_context* ctx, int n, const double* x) {
+  op_norm1(ctx, n, x, host_result(ctx), 0);
+  return wait_result(ctx);
+}
+
 }  // namespace ab2
 
 using namespace ab2;
@@ -440,36 +459,28 @@ int ab2_dot(ab2_context* ctx, const ab2_vector* x, const ab2_vector* y, double* 
   if (!ctx || !x || !result || check_vec(y, x->n)) return AB2_ERR_BAD_ARG;
   PhaseScope phase_scope(ctx, "CSR-DOT");
   return guard(ctx, [&] {
-    RedSlot s = red_slot(ctx, 0);
-    op_dot(ctx, x->n, x->d, y->d, s.result, 0);
-    *result = read_scalar(ctx, s.result);
+    *result = dot_value(ctx, x->n, x->d, y->d);
   });
 }
 int ab2_norm2(ab2_context* ctx, const ab2_vector* x, double* result) {
   if (!ctx || !x || !result) return AB2_ERR_BAD_ARG;
   PhaseScope phase_scope(ctx, "CSR-NORM2");
   return guard(ctx, [&] {
-    RedSlot s = red_slot(ctx, 0);
-    op_dot(ctx, x->n, x->d, x->d, s.result, 0);
-    *result = std::sqrt(read_scalar(ctx, s.result));
+    *result = std::sqrt(dot_value(ctx, x->n, x->d, x->d));
   });
 }
 int ab2_norm1(ab2_context* ctx, const ab2_vector* x, double* result) {
   if (!ctx || !x || !result) return AB2_ERR_BAD_ARG;
   PhaseScope phase_scope(ctx, "CSR-NORM1");
   return guard(ctx, [&] {
-    RedSlot s = red_slot(ctx, 0);
-    op_norm1(ctx, x->n, x->d, s.result, 0);
-    *result = read_scalar(ctx, s.result);
+    *result = norm1_value(ctx, x->n, x->d);
   });
 }
 int ab2_norm0(ab2_context* ctx, const ab2_vector* x, double* result) {
   if (!ctx || !x || !result) return AB2_ERR_BAD_ARG;
   PhaseScope phase_scope(ctx, "CSR-NORM0");
   return guard(ctx, [&] {
-    RedSlot s = red_slot(ctx, 0);
-    op_norm0(ctx, x->n, x->d, s.result, 0);
-    *result = read_scalar(ctx, s.result);
+    *result = norm0_value(ctx, x->n, x->d);
   });
 }
 

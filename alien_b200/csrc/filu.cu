@@ -306,17 +306,14 @@ void neumann_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* 
   for (int i = 0; i < n; ++i) h[(size_t)i] = dis(gen);
   double* x = nd.d_t[0];
   double* y = nd.d_t[1];
-  double* s = red_slot(ctx, 0).result;
   AB2_CUDA(cudaMemcpyAsync(x, h.data(), sizeof(double) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
   op_spmv(ctx, A, x, y, pc->variant);
-  op_dot(ctx, n, y, y, s);
-  double nk = std::sqrt(read_scalar(ctx, s));
+  double nk = std::sqrt(dot_value(ctx, n, y, y));
   double factor = 0.0;
   for (int it = 0; it < o->poly_factor_max_iter; ++it) {
     op_copy(ctx, n, y, x);
     op_spmv(ctx, A, x, y, pc->variant);
-    op_dot(ctx, n, y, y, s);
-    const double nrm = std::sqrt(read_scalar(ctx, s));
+    const double nrm = std::sqrt(dot_value(ctx, n, y, y));
     factor = nrm / nk;
     nk = nrm;
   }

@@ -1408,11 +1408,8 @@ double gnn_loss_grad(ab2_gnn* G, const double* r, const double* e) {
   op_axpy(ctx, n, -1.0, e, G->d_d);
   op_spmv(ctx, A, G->d_d, G->d_Ad, AB2_SPMV_AUTO);
   op_spmv(ctx, A, e, G->d_Ae, AB2_SPMV_AUTO);
-  double* s = red_slot(ctx, 6).result;
-  op_dot(ctx, n, e, G->d_Ae, s, 6);
-  const double eAe = read_scalar(ctx, s);
-  op_dot(ctx, n, G->d_d, G->d_Ad, s, 6);
-  const double dAd = read_scalar(ctx, s);
+  const double eAe = dot_value(ctx, n, e, G->d_Ae);
+  const double dAd = dot_value(ctx, n, G->d_d, G->d_Ad);
   require(eAe > 0, "gnn training pair: e^T A e must be positive");
   op_scal(ctx, n, 2.0 / eAe, G->d_Ad);  // dz
   const int wg = warp_grid(ctx, n);
@@ -1702,8 +1699,7 @@ int ab2_fcg_solve(ab2_context* ctx, const ab2_matrix* A, ab2_gnn* G, const ab2_p
     RedSlot red = red_slot(ctx, 7);
     const int rg = red_grid(ctx, n);
     auto dot = [&](const double* u, const double* v) {
-      op_dot(ctx, n, u, v, red.result, 7);
-      return read_scalar(ctx, red.result);
+      return dot_value(ctx, n, u, v);
     };
     bool use_gnn = G != nullptr;      // the network preconditions the next step
     bool gnn_retired = G == nullptr;  // STICKY fallback has taken over

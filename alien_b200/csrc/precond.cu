@@ -726,8 +726,6 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
   c.d_xcopy = dev_alloc<double>(ctx, (size_t)n);
   double* x = dev_alloc<double>(ctx, (size_t)n);
   double* y = c.d_y[0];
-  double* s = red_slot(ctx, 0).result;
-  double* s_out = s;
   c.saad = o->cheb_saad != 0;
   op_fill(ctx, n, 0.0, y);
   op_fill(ctx, n, 0.0, c.d_p);
@@ -739,21 +737,17 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
   };
   auto power = [&](bool shift, double b) {
     start();
-    op_dot(ctx, n, x, x, s);
-    const double nrm = std::sqrt(read_scalar(ctx, s));
+    const double nrm = std::sqrt(dot_value(ctx, n, x, x));
     op_scal(ctx, n, 1 / nrm, x);
     double est = 0.0;
     for (int it = 0; it < o->poly_factor_max_iter; ++it) {
       op_spmv(ctx, A, x, y, pc->variant);
       op_pmult(ctx, n, pc->d_inv, y, y);
       if (shift) op_axpy(ctx, n, -b, x, y);
-      op_dot(ctx, n, y, x, s);
-      const double xax = read_scalar(ctx, s);
-      op_dot(ctx, n, x, x, s);
-      const double xdx = read_scalar(ctx, s);
+      const double xax = dot_value(ctx, n, y, x);
+      const double xdx = dot_value(ctx, n, x, x);
       est = xax / xdx;
-      op_dot(ctx, n, y, y, s);
-      const double nr = std::sqrt(read_scalar(ctx, s));
+      const double nr = std::sqrt(dot_value(ctx, n, y, y));
       op_scal(ctx, n, 1 / nr, y);
       op_copy(ctx, n, y, x);
     }
@@ -769,8 +763,7 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
     k_sqrt<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, pc->d_inv, s);
     check_launch(ctx, "sqrt");
     start();
-    op_dot(ctx, n, x, x, s_out);
-    const double nrm = std::sqrt(read_scalar(ctx, s_out));
+    const double nrm = std::sqrt(dot_value(ctx, n, x, x));
     op_scal(ctx, n, 1 / nrm, x);
     std::vector<double> ta, tb;
     double bprev = 0.0;
@@ -780,11 +773,9 @@ void cheb_init(ab2_context* ctx, ab2_precond* pc, const ab2_precond_options* o) 
       op_spmv(ctx, A, t, w, pc->variant);
       op_pmult(ctx, n, s, w, w);
       if (j > 0) op_axpy(ctx, n, -bprev, vp, w);
-      op_dot(ctx, n, w, x, s_out);
-      const double aj = read_scalar(ctx, s_out);
+      const double aj = dot_value(ctx, n, w, x);
       op_axpy(ctx, n, -aj, x, w);
-      op_dot(ctx, n, w, w, s_out);
-      const double bj = std::sqrt(read_scalar(ctx, s_out));
+      const double bj = std::sqrt(dot_value(ctx, n, w, w));
       ta.push_back(aj);
       if (bj == 0.0 || j + 1 == m) break;
       tb.push_back(bj);
