@@ -51,39 +51,49 @@ constexpr int kRedThreads = 256;
 template <int NC, Combine C, class T>
 __device__ __forceinline__ void sum_partials(int G, const T* partials, T* out) {
   constexpr int kRound = 2 * kRedThreads, kRounds = 3;
-  __shared__ T s_stage[kRound];
   const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    const T* p = partials + (size_t)c * G;
-    T v = reduce_identity<C, T>();
-    for (int base = 0; base < G; base += kRound * kRounds) {
-      T t[kRounds][2];
-#pragma unroll
-      for (int k = 0; k < kRounds; ++k)
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int b = base + k * kRound + u * kRedThreads + (int)threadIdx.x;
-          t[k][u] = b < G ? __ldcg(p + b) : T(0);
-        }
-#pragma unroll
-      for (int k = 0; k < kRounds; ++k) {
-        const int at = base + k * kRound;
-        if (at >= G) break;
-        __syncthreads();  // the round before has been summed
-        s_stage[threadIdx.x] = t[k][0];
-        s_stage[kRedThreads + threadIdx.x] = t[k][1];
-        __syncthreads();
-        if (threadIdx.x < 32) {
-          const int m = G - at < kRound ? G - at : kRound;
-#pragma unroll 8
-          for (int b = lane; b < m; b += 32) v = combine<C, T>(v, s_stage[b]);
-        }
-      }
-    }
-    if (threadIdx.x < 32) {
+  if constexpr (NC > 2) {  // many components: a warp each, fetching for itself
+    for (int c = threadIdx.x >> 5; c < NC; c += kRedThreads / 32) {
+      T v = reduce_identity<C, T>();
+#pragma unroll 16
+      for (int b = lane; b < G; b += 32) v = combine<C, T>(v, __ldcg(partials + (size_t)c * G + b));
       v = warp_reduce<C, T>(v);
       if (lane == 0) out[c] = v;
+    }
+  } else {
+    __shared__ T s_stage[kRound];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const T* p = partials + (size_t)c * G;
+      T v = reduce_identity<C, T>();
+      for (int base = 0; base < G; base += kRound * kRounds) {
+        T t[kRounds][2];
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int b = base + k * kRound + u * kRedThreads + (int)threadIdx.x;
+            t[k][u] = b < G ? __ldcg(p + b) : T(0);
+          }
+#pragma unroll
+        for (int k = 0; k < kRounds; ++k) {
+          const int at = base + k * kRound;
+          if (at >= G) break;
+          __syncthreads();  // the round before has been summed
+          s_stage[threadIdx.x] = t[k][0];
+          s_stage[kRedThreads + threadIdx.x] = t[k][1];
+          __syncthreads();
+          if (threadIdx.x < 32) {
+            const int m = G - at < kRound ? G - at : kRound;
+#pragma unroll 8
+            for (int b = lane; b < m; b += 32) v = combine<C, T>(v, s_stage[b]);
+          }
+        }
+      }
+      if (threadIdx.x < 32) {
+        v = warp_reduce<C, T>(v);
+        if (lane == 0) out[c] = v;
+      }
     }
   }
   __syncthreads();

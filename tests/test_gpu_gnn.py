@@ -241,3 +241,45 @@ def test_gradient_blocks_ragged(ctx, shape):
         err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
         cos = a @ b / max(np.linalg.norm(a) * np.linalg.norm(b), 1e-30)
         assert err < 5e-2 and cos > 0.998, (name, err, cos)
+
+
+@pytest.mark.parametrize("m", [1, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("n", [1, 2, 255, 1000, 606_209])
+def test_fcg_window_sums(ctx, m, n):
+    """The direction window at each of its kernels' widths and across them, n odd
+    and even (the direction's 16-byte pairs) and up to a thread's second element
+    (a pass of the reduction grid is 1184 x 256 = 303,104 elements), against the
+    same recurrences in NumPy.  The matrix is unsymmetric, so every coefficient of
+    the window counts.  20 steps of a matrix of condition below 10 with sums of at
+    most 6e5 terms: rounding stays below 20 x 10 x 1e-13."""
+    k = np.arange(n)
+    a = 4.0 + (k % 7) * 0.25
+    up, lo = -1.0 - (k % 3) * 0.25, -0.5 - (k % 5) * 0.1
+    cols = np.stack([k - 1, k, k + 1], 1)
+    vals = np.stack([lo, a, up], 1)
+    keep = (cols >= 0) & (cols < n)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+
+    def mul(v):
+        w = a * v
+        w[1:] += lo[1:] * v[:-1]
+        w[:-1] += up[:-1] * v[1:]
+        return w
+
+    b = np.cos(0.37 * k) + 0.1
+    steps = min(20, max(1, n // 4))
+    x, r, win = np.zeros(n), b.copy(), []
+    for _ in range(steps):
+        z = r / a
+        p = z - sum((z @ q) / d * pk for pk, q, d in win)
+        q = mul(p)
+        d = p @ q
+        al = (p @ r) / d
+        x += al * p
+        r -= al * q
+        win = (win + [(p, q, d)])[-m:]
+    A = ctx.matrix(rp, cols[keep].astype(np.int32), vals[keep])
+    vb, vx = ctx.vector(b), ctx.vector(n)
+    res = abi.fcg_solve(ctx, A, vb, vx, fallback=abi.Precond(ctx, A, "diag"), tol=1e-30, max_iter=steps, truncation=m)
+    assert res.iterations == steps
+    assert np.linalg.norm(vx.download() - x) <= 2e-11 * np.linalg.norm(x)
