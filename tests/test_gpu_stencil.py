@@ -185,3 +185,30 @@ def test_explicit_zeros_in_the_profile_stay_terms(ctx):
     np.testing.assert_array_equal(got, exp)
     assert np.all(np.isnan(got[rows]))
     A.close()
+
+
+SWEEPS = [  # a pass of the reduction grid is 1184 x 256 = 303,104 rows
+    ((64, 64, 64), False, [5]), ((68, 68, 68), False, [5]), ((100, 100, 68), False, [5]),
+    ((104, 104, 100), False, [5]), ((108, 106, 106), True, [1, 2, 3, 4, 5, 8]), ((109, 106, 106), True, [6]),
+]
+
+
+@pytest.mark.parametrize("dims,use_graph,iters", SWEEPS)
+@pytest.mark.parametrize("form", ["plain", "scaled"])
+def test_fp32_jacobi_update_sweeps(ctx, dims, use_graph, iters, form):
+    """The FP32 Jacobi-CG update with one to five passes of the grid a thread (four
+    are in flight), and the graph's loop stopped after each of the bodies of a turn,
+    bit for bit against the oracle."""
+    P = abi.diffusion(*dims, sigma=1.0, smooth=1.0, seed=3)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals, BANDS)
+    for it in iters:
+        kw = dict(solver="cg", precond="diag", tol=1e-10, max_outer=1, inner_tol=1e-9, inner_max_iter=it)
+        M = abi.Mixed(ctx, A, use_graph=use_graph, jacobi_form=form, **kw)
+        x = ctx.vector(P.n)
+        st = M.solve(ctx.vector(P.b), x)
+        o = O.mixed_solve(P.row_ptr, P.cols, P.vals, P.b, dot_mode=O.DOT_DEVICE_TREE,
+                          tree_blocks=ctx.info.reduction_max_blocks, jacobi_scaled=form == "scaled", **kw)
+        assert st.inner_iterations == o.inner_iterations == it
+        np.testing.assert_array_equal(x.download(), o.x)
+        M.close()
+    A.close()
