@@ -249,19 +249,40 @@ __device__ __forceinline__ void ldsm_x4_t(unsigned (&r)[4], const void* p) {
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_u32(p)));
 }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
-// (acc0, acc1) += g * (lo(w), hi(w)) as one packed FP32 FMA (fma.rn.f32x2):
-// a BF16 value is the high half of its FP32 value, so the halves of w unpack
-// with a shift and a mask; each product is exact and each sum rounds once.
-__device__ __forceinline__ void fma2_bf16_pair(float& acc0, float& acc1, float g, unsigned w) {
-  const float lo = __uint_as_float(w << 16), hi = __uint_as_float(w & 0xffff0000u);
-  asm("{\n\t.reg .b64 a, x, y;\n\t"
-      "mov.b64 a, {%0, %1};\n\t"
-      "mov.b64 x, {%2, %3};\n\t"
-      "mov.b64 y, {%4, %4};\n\t"
-      "fma.rn.f32x2 a, y, x, a;\n\t"
-      "mov.b64 {%0, %1}, a;\n\t}"
-      : "+f"(acc0), "+f"(acc1)
-      : "f"(lo), "f"(hi), "f"(g));
+// Two FP32 values in one 64-bit register pair, and acc += g * (lo(w), hi(w)) as
+// one packed FP32 FMA (fma.rn.f32x2): a BF16 value is the high half of its FP32
+// value, so the halves of w unpack with a shift and a mask; each product is exact
+// and each sum rounds once.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 make_f32x2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void split_f32x2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 unpack_f32x2(unsigned w) {
+  return make_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ void fma_f32x2(f32x2& acc, f32x2 g, f32x2 x) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(g), "l"(x));
+}
+__device__ __forceinline__ f32x2 add_f32x2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned pack_f32x2(f32x2 v) {  // rounded to BF16
+  float lo, hi;
+  split_f32x2(v, lo, hi);
+  return pack_bf16(lo, hi);
+}
+// max(x, 0) of two BF16 values (NaN: 0, as fmaxf)
+__device__ __forceinline__ unsigned relu_bf16x2(unsigned w) {
+  unsigned r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(w), "r"(0u));
+  return r;
 }
 // Shared-memory words at 32-bit shared addresses.
 __device__ __forceinline__ float lds_f32(unsigned a) {
@@ -269,13 +290,6 @@ __device__ __forceinline__ float lds_f32(unsigned a) {
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
   return v;
 }
-__device__ __forceinline__ void lds_f32x2(unsigned a, float& x, float& y) {
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(a));
-}
-__device__ __forceinline__ void sts_f32(unsigned a, float v) {
-  asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-// 16 bytes of shared memory at a 32-bit shared address.
 __device__ __forceinline__ uint4 lds128(unsigned a) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
@@ -486,58 +500,66 @@ __global__ void __launch_bounds__(kLayerWarps * 32) k_gnn_layer(const LayerArgs 
 // -nx, -1, +1, +nx, +nx ny where inside the grid): 128 consecutive nodes a
 // tile, so each direction's neighbour rows form one contiguous block of h and
 // nothing is gathered by index.  A persistent CTA (one an SM) walks tiles with
-// its warps in three roles that hand tiles on through mbarriers, so one
-// tile's MMA and epilogue overlap the next tile's aggregation:
-//   - control (one thread): issues each tile's inputs by bulk copy
-//     (cp.async.bulk, no multicast) two tiles ahead into a two-stage ring --
-//     the tile's own rows with one row either side (the +-1 neighbours), the
-//     four +-nx / +-nx ny blocks, and the edge features in direction order
-//     (NaN where no neighbour) -- and, once a tile's A operand is complete and
-//     an accumulator buffer is free, eight tcgen05.mma (M = 128, N = 64,
-//     K = 16) into that buffer (two 128 x 64 FP32 accumulators in tensor
-//     memory); B is W (64 x 128 BF16), staged once per CTA;
-//   - aggregation (16 warps): the gates sigmoid(u e + c) once per (node,
-//     direction), then m = sum_d g_d h_nbr(d), four threads a node and two
-//     8-feature chunks a thread
-//     (BF16 x BF16 products, FP32 sums in the CSR column order, rounded to
-//     BF16 as the tensor-core aggregation of k_gnn_layer is; absent neighbours
-//     read a row of zeros), held in registers until the tensor core has
-//     released A, then [h ; m] written as A (128 x 128 BF16, 128-byte swizzle);
-//   - epilogue (4 warps, one a tensor-memory lane quarter): a row a thread,
-//     bias, relu, BF16, stored to h (LAST: the decoder's z instead).
+// its warps in four roles that hand on through mbarriers:
+//   - copies (one thread): a step's inputs (64 nodes, half a tile) by bulk copy
+//     (cp.async.bulk, no multicast) into a ring of three stages -- the step's own
+//     rows with one row either side (the +-1 neighbours), the four +-nx / +-nx ny
+//     blocks, and the edge features in direction order (NaN where no neighbour);
+//   - aggregation (16 warps, each four nodes a step and a lane one 8-feature chunk
+//     of one node): the gates sigmoid(u e + c) once per (node, direction), a lane
+//     each, handed round by shuffles, m = sum_d g_d h_nbr(d) (BF16 x BF16 products,
+//     FP32 sums in the CSR column order, rounded to BF16 as the tensor-core
+//     aggregation of k_gnn_layer is; 0 for absent neighbours), then [h ; m] written
+//     as A (128 x 128 BF16, 128-byte swizzle) into one of two buffers;
+//   - MMA (one thread): once a tile's A operand is complete and an accumulator is
+//     free, eight tcgen05.mma (M = 128, N = 64, K = 16) into it (two 128 x 64 FP32
+//     accumulators in tensor memory); B is W (64 x 128 BF16), staged once per CTA;
+//   - epilogue (4 warps, one a tensor-memory lane quarter): a row a thread, bias,
+//     BF16, relu, turned through shared memory so that h is stored in whole
+//     sectors (LAST: the decoder's z instead).
+// Beside the MMA the work a tile is about 8,000 warp instructions and 3,000 turns of
+// the shared-memory port (inputs copied in, seven rows read a node, A written and
+// read, the output turned), and that port at three quarters of its rate is what
+// bounds it: 1.72 million nodes take 180 us a layer (the last one 190), 227 (192)
+// before, when the aggregation warps went in step through a tile (gates, a barrier,
+// sums, a wait for the one A buffer) and the epilogue stored a row a thread, 16 bytes
+// at a time.  Also measured there: the neighbour rows by registers from global
+// memory instead of the ring 219 to 293 us (too few bytes in flight for L2's
+// latency), the last reader refilling a stage behind an atomic and a fence instead of
+// a warp of its own 300, the epilogue's first warp issuing the MMA 222.
 // Every wait is bounded: on expiry the kernel sets *err, every role stops at
 // its next tile, and the CTA waits (bounded) for the copies and the MMA it
 // issued and frees its tensor memory before it returns.
 constexpr int kTcAggWarps = 16;
 constexpr int kTcEpiWarps = 4;
-constexpr int kTcAggThreads = kTcAggWarps * 32;
-constexpr int kTcEpiThreads = kTcEpiWarps * 32;
-constexpr int kTcThreads = kTcAggThreads + kTcEpiThreads + 32;  // + the control warp
+constexpr int kTcThreads = (kTcAggWarps + kTcEpiWarps + 2) * 32;  // + the MMA's and the copies' warps
 constexpr int kTcTile = 128;
+constexpr int kTcHalf = kTcAggWarps * 4;                     // nodes the aggregation warps take at a time: a step
+constexpr int kTcStages = 3;
 constexpr unsigned kTcRowB = kH * 2;                         // bytes of one h row
 constexpr unsigned kTcW = 0;                                 // B: 2 regions x 64 rows x 128 B
-constexpr unsigned kTcA = kTcW + 2 * kH * kTcRowB;           // A: 2 regions x 128 rows x 128 B
+constexpr unsigned kTcA = kTcW + 2 * kH * kTcRowB;           // A: 2 buffers x 2 regions x 128 rows x 128 B
 constexpr unsigned kTcARegion = kTcTile * kTcRowB;
-constexpr unsigned kTcStage0 = kTcA + 2 * kTcARegion;
-constexpr unsigned kTcXOff = 0;                              // rows b-1 .. b+128
-constexpr unsigned kTcYmOff = kTcXOff + (kTcTile + 2) * kTcRowB;
-constexpr unsigned kTcYpOff = kTcYmOff + kTcARegion;
-constexpr unsigned kTcZmOff = kTcYpOff + kTcARegion;
-constexpr unsigned kTcZpOff = kTcZmOff + kTcARegion;
-constexpr unsigned kTcEfOff = kTcZpOff + kTcARegion;         // 128 x 6 floats
-constexpr unsigned kTcEfBytes = kTcTile * 6 * 4;
+constexpr unsigned kTcABuf = 2 * kTcARegion;
+constexpr unsigned kTcStage = kTcA + 2 * kTcABuf;            // a step's inputs:
+constexpr unsigned kTcBlockB = kTcHalf * kTcRowB;
+constexpr unsigned kTcXOff = 0;                              //   rows b-1 .. b+64
+constexpr unsigned kTcYmOff = kTcXOff + (kTcHalf + 2) * kTcRowB;
+constexpr unsigned kTcYpOff = kTcYmOff + kTcBlockB;
+constexpr unsigned kTcZmOff = kTcYpOff + kTcBlockB;
+constexpr unsigned kTcZpOff = kTcZmOff + kTcBlockB;
+constexpr unsigned kTcEfOff = kTcZpOff + kTcBlockB;          //   64 x 6 floats
+constexpr unsigned kTcEfBytes = kTcHalf * 6 * 4;
 constexpr unsigned kTcStageB = kTcEfOff + kTcEfBytes;
-constexpr unsigned kTcStage1 = kTcStage0 + kTcStageB;
-constexpr unsigned kTcBias = kTcStage1 + kTcStageB;          // bias, wd: 2 x 64 floats
-constexpr unsigned kTcGate = kTcBias + 2 * kH * 4;           // gates (BF16 values as FP32): 2 tiles x 128 x 6
-constexpr unsigned kTcGateB = kTcTile * 6 * 4;
-constexpr unsigned kTcZero = kTcGate + 2 * kTcGateB;         // one row of zeros (absent neighbours)
-constexpr unsigned kTcBar = kTcZero + kTcRowB;               // 8 mbarriers, tensor-memory address, abort flag
-constexpr unsigned kTcSmem = kTcBar + 80 + 1024;             // + slack to align the base to 1024 bytes
+constexpr unsigned kTcOut = kTcStage + kTcStages * kTcStageB;  // the epilogue's half rows: 8 warps x 32 x 64 B
+constexpr unsigned kTcOutB = 32 * kTcRowB / 2;
+constexpr unsigned kTcBias = kTcOut + kTcEpiWarps * kTcOutB;  // bias, wd: 2 x 64 floats
+constexpr unsigned kTcBar = kTcBias + 2 * kH * 4;            // 14 mbarriers, tensor-memory address, abort flag
+constexpr unsigned kTcSmem = kTcBar + 128 + 1024;            // + slack to align the base to 1024 bytes
 constexpr unsigned kTcCols = 2 * kH;                         // tensor-memory columns: two accumulators
 static_assert(kTcSmem <= 227 * 1024, "grid layer: shared memory");
-static_assert(kTcStage0 % 1024 == 0 && kTcA % 1024 == 0 && kTcStageB % 16 == 0, "grid layer: alignment");
-static_assert(kTcAggThreads == kTcTile * 4, "grid layer: four aggregation threads a node");
+static_assert(kTcA % 1024 == 0 && kTcABuf % 1024 == 0 && kTcStageB % 16 == 0, "grid layer: alignment");
+static_assert(2 * kTcHalf == kTcTile && kTcHalf % 8 == 0, "grid layer: two steps a tile, one swizzle for both");
 
 struct GridLayerArgs {
   LayerArgs a;
@@ -545,20 +567,6 @@ struct GridLayerArgs {
   const float* dir_ef;   // [ceil(n/128) * 128][6] edge features by direction, NaN = none
   int* err;              // set when a bounded wait gives up
 };
-
-// Named barrier `id` over `count` threads that ORs a flag across them.
-__device__ __forceinline__ int bar_or(int id, int count, int v) {
-  int r;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.s32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
-      "selp.s32 %0, 1, 0, q;\n\t}"
-      : "=r"(r)
-      : "r"(v), "r"(id), "r"(count)
-      : "memory");
-  return r;
-}
 
 template <bool LAST>
 __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLayerArgs ga) {
@@ -569,12 +577,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLaye
   const unsigned sb = tc::smem_u32(sm);
   float* s_bias = reinterpret_cast<float*>(sm + kTcBias);
   float* s_wd = s_bias + kH;
-  // mbarriers: inputs of stage 0/1 landed; A written; A released by the
-  // tensor core; accumulator 0/1 complete; accumulator 0/1 read
-  const unsigned bar_full = sb + kTcBar, bar_afull = bar_full + 16, bar_aempty = bar_full + 24;
-  const unsigned bar_accf = bar_full + 32, bar_acce = bar_full + 48;
-  volatile unsigned* s_tmem = reinterpret_cast<volatile unsigned*>(sm + kTcBar + 64);
-  volatile int* s_abort = reinterpret_cast<volatile int*>(sm + kTcBar + 68);
+  // mbarriers, two of each: A written; A released by the tensor core; accumulator
+  // complete; accumulator read; then one a stage: inputs landed; inputs read
+  const unsigned bar_afull = sb + kTcBar, bar_aempty = bar_afull + 16;
+  const unsigned bar_accf = bar_afull + 32, bar_acce = bar_afull + 48, bar_full = bar_afull + 64;
+  const unsigned bar_read = bar_full + 8 * kTcStages;
+  volatile unsigned* s_tmem = reinterpret_cast<volatile unsigned*>(sm + kTcBar + 112);
+  volatile int* s_abort = reinterpret_cast<volatile int*>(sm + kTcBar + 116);
+  const unsigned kFull = 0xffffffffu;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n = a.n;
   const int ntiles = (n + kTcTile - 1) / kTcTile;
@@ -595,21 +605,22 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLaye
     s_bias[t] = a.P[kOffB + a.layer * kH + t];
     s_wd[t] = a.P[kOffWd + t];
   }
-  if (tid < (int)kTcRowB / 16) reinterpret_cast<uint4*>(sm + kTcZero)[tid] = make_uint4(0u, 0u, 0u, 0u);
   if (tid == 0) {
-    tc::mbar_init(bar_full, 1);
-    tc::mbar_init(bar_full + 8, 1);
-    tc::mbar_init(bar_afull, kTcAggThreads);
-    tc::mbar_init(bar_aempty, 1);
-    tc::mbar_init(bar_accf, 1);
-    tc::mbar_init(bar_accf + 8, 1);
-    tc::mbar_init(bar_acce, kTcEpiThreads);
-    tc::mbar_init(bar_acce + 8, kTcEpiThreads);
+    for (int k = 0; k < 2; ++k) {
+      tc::mbar_init(bar_afull + 8 * k, kTcAggWarps);
+      tc::mbar_init(bar_aempty + 8 * k, 1);
+      tc::mbar_init(bar_accf + 8 * k, 1);
+      tc::mbar_init(bar_acce + 8 * k, kTcEpiWarps);
+    }
+    for (int k = 0; k < kTcStages; ++k) {
+      tc::mbar_init(bar_full + 8 * k, 1);
+      tc::mbar_init(bar_read + 8 * k, kTcAggWarps);
+    }
     *s_abort = 0;
     tc::fence_mbar_init();
   }
   if (warp == 0) {
-    tc::tmem_alloc(sb + kTcBar + 64, kTcCols);
+    tc::tmem_alloc(sb + kTcBar + 112, kTcCols);
     tc::tmem_relinquish();
   }
   tc::fence_proxy_async_smem();  // W (generic stores) is read by the tensor core
@@ -621,80 +632,94 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLaye
   if (warp < kTcAggWarps) {
     // ================================================================ aggregation
     const float u = a.P[kOffU + a.layer], cg = a.P[kOffC + a.layer];
-    int failed = 0;
+    const int ch = lane & 7, group = lane & 24;       // this lane's chunk; the first lane of its node
+    const int ln0 = warp * 4 + (lane >> 3);           // its node in a tile's first half
+    // chunk ch of row ln0 of A's first region, and of a stage's rows
+    unsigned char* const dst0 = sm + kTcA + ln0 * kTcRowB + ((ch ^ (ln0 & 7)) << 4);
+    const unsigned src0 = sb + kTcStage + ln0 * kTcRowB + ch * 16;
+    int stage = 0;
+    unsigned phase = 0;
+    bool ok = true;
+    // One step: h and m of its nodes into A (beyond the last node whatever the stage
+    // holds: a row of A reaches its own row of the result only, which is not stored).
+    auto step = [&](int i, unsigned char* dst, bool wait_a, unsigned a_phase) {
+      ok = tc::mbar_try_wait(bar_full + 8 * stage, phase) ||
+           tc::mbar_wait(bar_full + 8 * stage, phase, kWaitCycles, s_abort);
+      if (__any_sync(kFull, !ok)) return false;
+      const unsigned st = src0 + stage * kTcStageB;
+      const float e = ch < 6 ? lds_f32(sb + kTcStage + stage * kTcStageB + kTcEfOff + ln0 * 24 + ch * 4)
+                             : __int_as_float(0x7fc00000);
+      const unsigned all = __ballot_sync(kFull, e == e);
+      uint4 w[6];
+      const uint4 own = lds128(st + kTcXOff + kTcRowB);
+      if (all == 0x3f3f3f3fu) {  // four nodes with all six neighbours
+        w[0] = lds128(st + kTcZmOff);
+        w[1] = lds128(st + kTcYmOff);
+        w[2] = lds128(st + kTcXOff);
+        w[3] = lds128(st + kTcXOff + 2 * kTcRowB);
+        w[4] = lds128(st + kTcYpOff);
+        w[5] = lds128(st + kTcZpOff);
+      } else {
+        const unsigned there = all >> group;
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        w[0] = there & 1 ? lds128(st + kTcZmOff) : zero;
+        w[1] = there & 2 ? lds128(st + kTcYmOff) : zero;
+        w[2] = there & 4 ? lds128(st + kTcXOff) : zero;
+        w[3] = there & 8 ? lds128(st + kTcXOff + 2 * kTcRowB) : zero;
+        w[4] = there & 16 ? lds128(st + kTcYpOff) : zero;
+        w[5] = there & 32 ? lds128(st + kTcZpOff) : zero;
+      }
+      const float gate = e == e ? bf16r(sigmoidf(fmaf(u, e, cg))) : 0.f;
+      f32x2 acc[4] = {0ull, 0ull, 0ull, 0ull};
+#pragma unroll
+      for (int d = 0; d < 6; ++d) {
+        const float g = __shfl_sync(kFull, gate, group + d);
+        const f32x2 g2 = make_f32x2(g, g);
+        fma_f32x2(acc[0], g2, unpack_f32x2(w[d].x));
+        fma_f32x2(acc[1], g2, unpack_f32x2(w[d].y));
+        fma_f32x2(acc[2], g2, unpack_f32x2(w[d].z));
+        fma_f32x2(acc[3], g2, unpack_f32x2(w[d].w));
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar_read + 8 * stage);
+      if (++stage == kTcStages) {
+        stage = 0;
+        phase ^= 1u;
+      }
+      const uint4 m = make_uint4(pack_f32x2(acc[0]), pack_f32x2(acc[1]), pack_f32x2(acc[2]), pack_f32x2(acc[3]));
+      if (wait_a) {  // this A buffer is free once the tensor core has read the tile before the last
+        const unsigned bar = bar_aempty + 8 * ((i >> 1) & 1);
+        ok = tc::mbar_try_wait(bar, a_phase) || tc::mbar_wait(bar, a_phase, kWaitCycles, s_abort);
+        if (__any_sync(kFull, !ok)) return false;
+      }
+      *reinterpret_cast<uint4*>(dst) = own;
+      *reinterpret_cast<uint4*>(dst + kTcARegion) = m;
+      if (a.m_out) {
+        const long long node = tile_base(i >> 1) + (i & 1) * kTcHalf + ln0;
+        if (node < n) reinterpret_cast<uint4*>(a.m_out + node * kH)[ch] = m;
+      }
+      return true;
+    };
     for (int c = 0; c < count; ++c) {
-      const int s = c & 1;
-      const long long b = tile_base(c);
-      if (!tc::mbar_wait(bar_full + 8 * s, (unsigned)(c >> 1) & 1u, kWaitCycles, s_abort)) {
-        failed = 1;
+      unsigned char* const dst = dst0 + (c & 1) * kTcABuf;
+      if (!step(2 * c, dst, c >= 2, (unsigned)((c >> 1) - 1) & 1u) ||
+          !step(2 * c + 1, dst + kTcHalf * kTcRowB, false, 0u)) {
         give_up();
-      }
-      // gates, once per (node, direction), rounded to BF16 (0 where no neighbour)
-      {
-        const unsigned ef = sb + (s ? kTcStage1 : kTcStage0) + kTcEfOff, gt = sb + kTcGate + s * kTcGateB;
-        for (int q = tid; q < kTcTile * 6; q += kTcAggThreads) {
-          const float e = lds_f32(ef + 4 * q);
-          sts_f32(gt + 4 * q, e == e ? bf16r(sigmoidf(fmaf(u, e, cg))) : 0.f);
-        }
-      }
-      if (bar_or(1, kTcAggThreads, failed)) break;
-      const int ln = tid >> 2, qq = tid & 3;  // node, and its chunks qq and qq + 4
-      const unsigned sst = sb + (s ? kTcStage1 : kTcStage0) + ln * kTcRowB;  // this node's row of each block
-      unsigned src[6] = {sst + kTcZmOff, sst + kTcYmOff, sst + kTcXOff, sst + kTcXOff + 2 * kTcRowB, sst + kTcYpOff,
-                         sst + kTcZpOff};
-      float g[6], e[6];
-      {
-        const unsigned efa = sb + (s ? kTcStage1 : kTcStage0) + kTcEfOff + ln * 24;
-        const unsigned gta = sb + kTcGate + s * kTcGateB + ln * 24;
-#pragma unroll
-        for (int d = 0; d < 6; d += 2) {
-          lds_f32x2(efa + 4 * d, e[d], e[d + 1]);
-          lds_f32x2(gta + 4 * d, g[d], g[d + 1]);
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < 6; ++d) src[d] = e[d] == e[d] ? src[d] : sb + kTcZero;
-      uint4 hv[2], mv[2];
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int ch = 4 * ((ln & 1) ^ jj) + qq;  // the 8 threads of a quarter-warp touch 8 distinct banks
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int d = 0; d < 6; ++d) {
-          const uint4 w = lds128(src[d] + ch * 16);
-          fma2_bf16_pair(acc[0], acc[1], g[d], w.x);
-          fma2_bf16_pair(acc[2], acc[3], g[d], w.y);
-          fma2_bf16_pair(acc[4], acc[5], g[d], w.z);
-          fma2_bf16_pair(acc[6], acc[7], g[d], w.w);
-        }
-        mv[jj] = pack8(acc);
-        hv[jj] = b + ln < n ? lds128(sst + kTcXOff + kTcRowB + ch * 16) : make_uint4(0u, 0u, 0u, 0u);
-      }
-      // A is free once the tensor core has read the previous tile's
-      if (c > 0 && !tc::mbar_wait(bar_aempty, (unsigned)(c - 1) & 1u, kWaitCycles, s_abort)) {
-        failed = 1;
-        give_up();
-      }
-#pragma unroll
-      for (int jj = 0; jj < 2; ++jj) {
-        const int ch = 4 * ((ln & 1) ^ jj) + qq;
-        const unsigned pos = ln * kTcRowB + ((ch ^ (ln & 7)) << 4);
-        *reinterpret_cast<uint4*>(sm + kTcA + pos) = hv[jj];
-        *reinterpret_cast<uint4*>(sm + kTcA + kTcARegion + pos) = mv[jj];
-        if (a.m_out && b + ln < n) reinterpret_cast<uint4*>(a.m_out + (b + ln) * kH)[ch] = mv[jj];
+        break;
       }
       tc::fence_proxy_async_smem();
-      tc::mbar_arrive(bar_afull);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar_afull + 8 * (c & 1));
     }
   } else if (warp < kTcAggWarps + kTcEpiWarps) {
     // ================================================================ epilogue
     const int q = warp & 3;  // the tensor-memory lane quarter this warp may read
-    const int row = 32 * q + lane;
+    unsigned char* out = sm + kTcOut + q * kTcOutB;
     for (int c = 0; c < count; ++c) {
       const int bsel = c & 1;
-      const long long gi = tile_base(c) + row;
-      int failed = !tc::mbar_wait(bar_accf + 8 * bsel, (unsigned)(c >> 1) & 1u, kWaitCycles, s_abort);
-      if (__any_sync(0xffffffffu, failed)) {
+      const long long base = tile_base(c) + 32 * q, gi = base + lane;
+      const bool ok = tc::mbar_wait(bar_accf + 8 * bsel, (unsigned)(c >> 1) & 1u, kWaitCycles, s_abort);
+      if (__any_sync(kFull, !ok)) {
         give_up();
         break;
       }
@@ -707,31 +732,38 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLaye
         tc::tmem_ld32(ta + 32 * h, v);
         if (h == 1) {
           tc::fence_before_sync();
-          tc::mbar_arrive(bar_acce + 8 * bsel);  // the accumulator is read
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(bar_acce + 8 * bsel);  // the accumulator is read
         }
-        if (gi < n) {
+        // bias, BF16, relu (after the rounding: the same values)
+        unsigned o[16];
 #pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 bb = reinterpret_cast<const float4*>(s_bias)[8 * h + j4];
-            const float bv[4] = {bb.x, bb.y, bb.z, bb.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v[4 * j4 + e] = fmaxf(v[4 * j4 + e] + bv[e], 0.f);
-            if constexpr (LAST) {
-              const float4 ww = reinterpret_cast<const float4*>(s_wd)[8 * h + j4];
-              const float wv[4] = {ww.x, ww.y, ww.z, ww.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) y = fmaf(wv[e], bf16r(v[4 * j4 + e]), y);
-            }
+        for (int j4 = 0; j4 < 8; ++j4) {
+          const ulonglong2 bb = reinterpret_cast<const ulonglong2*>(s_bias)[8 * h + j4];
+          o[2 * j4] = relu_bf16x2(pack_f32x2(add_f32x2(make_f32x2(v[4 * j4], v[4 * j4 + 1]), bb.x)));
+          o[2 * j4 + 1] = relu_bf16x2(pack_f32x2(add_f32x2(make_f32x2(v[4 * j4 + 2], v[4 * j4 + 3]), bb.y)));
+          if constexpr (LAST) {
+            const float4 ww = reinterpret_cast<const float4*>(s_wd)[8 * h + j4];
+            const float2 x = unpack_bf16(o[2 * j4]), z = unpack_bf16(o[2 * j4 + 1]);
+            y = fmaf(ww.x, x.x, y);
+            y = fmaf(ww.y, x.y, y);
+            y = fmaf(ww.z, z.x, y);
+            y = fmaf(ww.w, z.y, y);
           }
-          if (a.h_out) {
+        }
+        if (a.h_out) {  // half rows: chunk c8 of row r at c8 ^ (r / 2 & 3)
 #pragma unroll
-            for (int c8 = 0; c8 < 4; ++c8) {
-              float f8[8];
+          for (int c8 = 0; c8 < 4; ++c8)
+            *reinterpret_cast<uint4*>(out + lane * (kTcRowB / 2) + ((c8 ^ (lane >> 1 & 3)) << 4)) =
+                make_uint4(o[4 * c8], o[4 * c8 + 1], o[4 * c8 + 2], o[4 * c8 + 3]);
+          __syncwarp();
 #pragma unroll
-              for (int e = 0; e < 8; ++e) f8[e] = v[8 * c8 + e];
-              reinterpret_cast<uint4*>(a.h_out + gi * kH)[4 * h + c8] = pack8(f8);
-            }
+          for (int k = 0; k < 4; ++k) {  // eight half rows at a time
+            const int r = 8 * k + (lane >> 2), c8 = lane & 3;
+            const uint4 t = *reinterpret_cast<const uint4*>(out + r * (kTcRowB / 2) + ((c8 ^ (r >> 1 & 3)) << 4));
+            if (base + r < n) reinterpret_cast<uint4*>(a.h_out + (base + r) * kH)[4 * h + c8] = t;
           }
+          __syncwarp();  // the staging is refilled
         }
       }
       if constexpr (LAST) {
@@ -742,64 +774,92 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_gnn_layer_grid(const GridLaye
         }
       }
     }
-  } else if (lane == 0) {
-    // ================================================================ control
-    // in flight, for the drain after a failure: the parity of each stage's
-    // last issued phase and of the last MMA commit (-1: none)
-    int last_in[2] = {-1, -1}, last_mma = -1;
-    auto issue = [&](int c) {
-      const int s = c & 1;
-      const long long b = tile_base(c);
-      const unsigned st = sb + (s ? kTcStage1 : kTcStage0);
-      const long long first[5] = {b - 1, b - ga.nx, b + ga.nx, b - ga.sxy, b + ga.sxy};
-      const int rows[5] = {kTcTile + 2, kTcTile, kTcTile, kTcTile, kTcTile};
-      const unsigned dst[5] = {kTcXOff, kTcYmOff, kTcYpOff, kTcZmOff, kTcZpOff};
-      long long lo[5], hi[5];
-      unsigned bytes = kTcEfBytes;
-      for (int k = 0; k < 5; ++k) {
-        lo[k] = first[k] < 0 ? 0 : first[k];
-        hi[k] = first[k] + rows[k] > n ? n : first[k] + rows[k];
-        if (hi[k] > lo[k]) bytes += (unsigned)(hi[k] - lo[k]) * kTcRowB;
+  } else if (warp == kTcAggWarps + kTcEpiWarps) {
+    // ================================================================ MMA
+    if (lane == 0) {
+      int last = -1;  // the last tile whose MMA was issued, for the drain after a failure
+      bool ok = true;
+      for (int c = 0; c < count; ++c) {
+        const int bsel = c & 1;
+        const unsigned phase = (unsigned)(c >> 1) & 1u;
+        // A of tile c written; the epilogue has read this accumulator's previous tile
+        ok = tc::mbar_wait(bar_afull + 8 * bsel, phase, kWaitCycles, s_abort) &&
+             (c < 2 || tc::mbar_wait(bar_acce + 8 * bsel, phase ^ 1u, kWaitCycles, s_abort));
+        if (!ok) {
+          give_up();
+          break;
+        }
+        tc::fence_after_sync();
+        constexpr uint32_t idesc = tc::idesc_bf16_f32(kTcTile, kH);
+        const unsigned abuf = sb + kTcA + bsel * kTcABuf;
+#pragma unroll
+        for (int k = 0; k < kIn / 16; ++k) {
+          const unsigned aoff = (k >> 2) * kTcARegion + (k & 3) * 32, boff = (k >> 2) * (kH * kTcRowB) + (k & 3) * 32;
+          tc::mma_bf16_ss(tmem + bsel * kH, tc::sdesc_sw128(abuf + aoff), tc::sdesc_sw128(sb + kTcW + boff), idesc,
+                          k > 0);
+        }
+        tc::mma_commit(bar_aempty + 8 * bsel);
+        tc::mma_commit(bar_accf + 8 * bsel);
+        last = c;
       }
-      tc::mbar_expect_tx(bar_full + 8 * s, bytes);
-      for (int k = 0; k < 5; ++k)
-        if (hi[k] > lo[k])
-          tc::bulk_g2s(st + dst[k] + (unsigned)(lo[k] - first[k]) * kTcRowB, a.h_in + lo[k] * kH,
-                       (unsigned)(hi[k] - lo[k]) * kTcRowB, bar_full + 8 * s);
-      tc::bulk_g2s(st + kTcEfOff, ga.dir_ef + b * 6, kTcEfBytes, bar_full + 8 * s);
-      last_in[s] = (c >> 1) & 1;
+      if (!ok && last >= 0)  // drain: no MMA of this CTA's may still run at exit
+        tc::mbar_wait(bar_aempty + 8 * (last & 1), (unsigned)(last >> 1) & 1u, kWaitCycles, nullptr);
+    }
+  } else if (lane == 0) {
+    // ================================================================ input copies
+    const long long sy = (long long)ga.nx * kH, sz = (long long)ga.sxy * kH;
+    // the inputs of step i (half i & 1 of tile i / 2) into its stage
+    auto issue = [&](int i, int stage) {
+      const long long b = tile_base(i >> 1) + (i & 1) * kTcHalf;
+      const unsigned st = sb + kTcStage + stage * kTcStageB, bar = bar_full + 8 * stage;
+      if (b >= ga.sxy && b + ga.sxy + kTcHalf <= n) {  // every row of every block exists (sxy >= nx >= 1)
+        tc::mbar_expect_tx(bar, kTcStageB);
+        const bf16* h = a.h_in + b * kH;
+        tc::bulk_g2s(st + kTcZmOff, h - sz, kTcBlockB, bar);
+        tc::bulk_g2s(st + kTcYmOff, h - sy, kTcBlockB, bar);
+        tc::bulk_g2s(st + kTcXOff, h - kH, kTcBlockB + 2 * kTcRowB, bar);
+        tc::bulk_g2s(st + kTcYpOff, h + sy, kTcBlockB, bar);
+        tc::bulk_g2s(st + kTcZpOff, h + sz, kTcBlockB, bar);
+      } else {
+        const long long first[5] = {b - 1, b - ga.nx, b + ga.nx, b - ga.sxy, b + ga.sxy};
+        const unsigned dst[5] = {kTcXOff, kTcYmOff, kTcYpOff, kTcZmOff, kTcZpOff};
+        long long lo[5];
+        int rows[5];
+        unsigned bytes = kTcEfBytes;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+          const long long end = first[k] + (k == 0 ? kTcHalf + 2 : kTcHalf);
+          lo[k] = first[k] < 0 ? 0 : first[k];
+          rows[k] = (int)((end > n ? n : end) - lo[k]);
+          if (rows[k] > 0) bytes += (unsigned)rows[k] * kTcRowB;
+        }
+        tc::mbar_expect_tx(bar, bytes);
+#pragma unroll
+        for (int k = 0; k < 5; ++k)
+          if (rows[k] > 0)
+            tc::bulk_g2s(st + dst[k] + (unsigned)(lo[k] - first[k]) * kTcRowB, a.h_in + lo[k] * kH,
+                         (unsigned)rows[k] * kTcRowB, bar);
+      }
+      tc::bulk_g2s(st + kTcEfOff, ga.dir_ef + b * 6, kTcEfBytes, bar);
     };
-    for (int c = 0; c < 2 && c < count; ++c) issue(c);
-    bool ok = true;
-    for (int c = 0; c < count && ok; ++c) {
-      const int bsel = c & 1;
-      ok = tc::mbar_wait(bar_afull, (unsigned)c & 1u, kWaitCycles, s_abort);  // A of tile c written
-      if (ok && c + 2 < count) issue(c + 2);  // stage c & 1 read by every aggregation thread
-      if (ok && c >= 2)  // the epilogue has read this accumulator's previous tile
-        ok = tc::mbar_wait(bar_acce + 8 * bsel, (unsigned)((c >> 1) - 1) & 1u, kWaitCycles, s_abort);
-      if (!ok) {
+    int i = 0, stage = 0;
+    unsigned phase = 0;
+    for (; i < 2 * count; ++i) {
+      if (i >= kTcStages && !tc::mbar_wait(bar_read + 8 * stage, phase ^ 1u, kWaitCycles, s_abort)) {
         give_up();
         break;
       }
-      tc::fence_after_sync();
-      constexpr uint32_t idesc = tc::idesc_bf16_f32(kTcTile, kH);
-#pragma unroll
-      for (int k = 0; k < kIn / 16; ++k) {
-        const unsigned aoff = (k >> 2) * kTcARegion + (k & 3) * 32, boff = (k >> 2) * (kH * kTcRowB) + (k & 3) * 32;
-        tc::mma_bf16_ss(tmem + bsel * kH, tc::sdesc_sw128(sb + kTcA + aoff), tc::sdesc_sw128(sb + kTcW + boff), idesc,
-                        k > 0);
+      issue(i, stage);
+      if (++stage == kTcStages) {
+        stage = 0;
+        phase ^= 1u;
       }
-      tc::mma_commit(bar_aempty);
-      tc::mma_commit(bar_accf + 8 * bsel);
-      last_mma = c & 1;
     }
-    if (!ok) {  // drain: nothing of this CTA's may still write its shared or tensor memory at exit
-      for (int s = 0; s < 2; ++s)
-        if (last_in[s] >= 0) tc::mbar_wait(bar_full + 8 * s, (unsigned)last_in[s], kWaitCycles, nullptr);
-      if (last_mma >= 0) tc::mbar_wait(bar_aempty, (unsigned)last_mma, kWaitCycles, nullptr);
-    }
+    // the last copies have landed, whether or not a failure left them unread
+    for (int k = i - 1; k >= 0 && k >= i - kTcStages; --k)
+      tc::mbar_wait(bar_full + 8 * (k % kTcStages), (unsigned)(k / kTcStages) & 1u, kWaitCycles, nullptr);
   }
-  __syncwarp();  // the control warp reconverges before the CTA barrier
+  __syncwarp();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 0) {
