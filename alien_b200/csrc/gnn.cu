@@ -517,10 +517,9 @@ __global__ void __launch_bounds__(kLayerWarps * 32) k_gnn_layer(const LayerArgs 
 //   - epilogue (4 warps, one a tensor-memory lane quarter): a row a thread, bias,
 //     BF16, relu, turned through shared memory so that h is stored in whole
 //     sectors (LAST: the decoder's z instead).
-// Beside the MMA the work a tile is about 8,000 warp instructions and 3,000 turns of
+// Beside the MMA the work a tile is about 7,500 warp instructions and 3,000 turns of
 // the shared-memory port (inputs copied in, seven rows read a node, A written and
-// read, the output turned), and that port at three quarters of its rate is what
-// bounds it: 1.72 million nodes take 180 us a layer (the last one 190), 227 (192)
+// read, the output turned), and that port, 81 % busy, is what bounds it: 1.72 million nodes take 180 us a layer (the last one 190), 227 (192)
 // before, when the aggregation warps went in step through a tile (gates, a barrier,
 // sums, a wait for the one A buffer) and the epilogue stored a row a thread, 16 bytes
 // at a time.  Also measured there: the neighbour rows by registers from global
