@@ -41,6 +41,18 @@ __device__ __forceinline__ T reduce_identity() {
   return C == Combine::Sum ? T(0) : -T(1) / T(0);
 }
 
+// One thread's arrival for its block at the counter of a reduction over `blocks`
+// blocks: true in the last one.  What its block wrote is released before it, what
+// all the others wrote is acquired behind it -- by this thread, so that the block
+// barrier after it hands both on (a fence of another thread's behind the barrier
+// pairs with nothing).
+__device__ __forceinline__ bool last_arrival(unsigned int* counter, unsigned int blocks) {
+  fence_gpu();
+  const bool last = atomicAdd(counter, 1u) == blocks - 1;
+  if (last) fence_gpu();
+  return last;
+}
+
 // The last step of every grid reduction, by one whole block of 256 threads: out[c]
 // = partials[c * G + 0 .. G) summed as one warp would, lane l taking l, l + 32, ...
 // in order, then the shuffle tree.  All 256 threads fetch (up to 6 words each in
@@ -123,15 +135,10 @@ __device__ __forceinline__ bool grid_reduce(T (&acc)[NC], T* partials, unsigned 
       v = warp_reduce<C, T>(v);
       if (lane == 0) partials[(size_t)c * gridDim.x + blockIdx.x] = v;
     }
-    if (lane == 0) {
-      fence_gpu();
-      unsigned int ticket = atomicAdd(counter, 1u);
-      s_last = (ticket == gridDim.x - 1);
-    }
+    if (lane == 0) s_last = last_arrival(counter, gridDim.x);
   }
   __syncthreads();
   if (!s_last) return false;
-  fence_gpu();
   sum_partials<NC, C, T>((int)gridDim.x, partials, out);
   if (threadIdx.x == 0) {
     *counter = 0u;  // ready for the next launch that uses this slot
@@ -176,15 +183,10 @@ __device__ __forceinline__ bool grid_reduce_v(T (&acc)[V][NC], T* partials, unsi
           x = warp_reduce<C, T>(x);
           if (lane == 0) partials[(size_t)c * G + v * gridDim.x + blockIdx.x] = x;
         }
-      if (lane == 0) {
-        fence_gpu();
-        unsigned int ticket = atomicAdd(counter, 1u);
-        s_last = (ticket == gridDim.x - 1);
-      }
+      if (lane == 0) s_last = last_arrival(counter, gridDim.x);
     }
     __syncthreads();
     if (!s_last) return false;
-    fence_gpu();
     sum_partials<NC, C, T>(G, partials, out);
     if (threadIdx.x == 0) {
       *counter = 0u;  // ready for the next launch that uses this slot
@@ -237,14 +239,9 @@ __device__ __forceinline__ bool grid_reduce_r(const T (&acc)[R][NC], int G, T* p
     if (lane == 0) fence_gpu();
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    fence_gpu();
-    unsigned int ticket = atomicAdd(counter, 1u);
-    s_last = (ticket == gridDim.x - 1);
-  }
+  if (threadIdx.x == 0) s_last = last_arrival(counter, gridDim.x);
   __syncthreads();
   if (!s_last) return false;
-  fence_gpu();
   sum_partials<NC, Combine::Sum, T>(G, partials, out);
   if (threadIdx.x == 0) {
     *counter = 0u;  // ready for the next launch that uses this slot
