@@ -265,6 +265,7 @@ SIGNATURES: dict[str, tuple] = {
     "ab2_selftest_bounded_wait": (_I, [_P, _IP, _DP]),
     "ab2_selftest_mbarrier_wait": (_I, [_P, _IP, _DP]),
     "ab2_context_inject_alloc_failure": (_I, [_P, C.c_longlong]),
+    "ab2_context_inject_lost_arrival": (_I, [_P, C.c_longlong]),
     "ab2_rng_u64": (C.c_uint64, [C.c_uint64, C.c_uint64, C.c_uint64]),
     "ab2_rng_uniform": (_D, [C.c_uint64, C.c_uint64, C.c_uint64]),
 }
@@ -371,6 +372,10 @@ class Context:
     def inject_alloc_failure(self, nth: int) -> None:
         """The nth device allocation from now on fails as AB2_ERR_OOM (0: off)."""
         self.check(lib().ab2_context_inject_alloc_failure(self.h, nth), "inject_alloc_failure")
+
+    def inject_lost_arrival(self, nth: int) -> None:
+        """The next one-launch CG loop loses an arrival at its nth grid barrier and ends as AB2_ERR_TIMEOUT (0: off)."""
+        self.check(lib().ab2_context_inject_lost_arrival(self.h, nth), "inject_lost_arrival")
 
     # -- objects
     def matrix(self, row_ptr, cols, vals, formats: int = FMT_CSR | FMT_ELL) -> "Matrix":

@@ -44,7 +44,8 @@ namespace ab2 {
 namespace {
 
 constexpr int kCtlThreads = 256;
-constexpr long long kLoopWaitCycles = 4000000000LL;  // a grid barrier's bound, ~2 s
+constexpr long long kLoopWaitCycles = 4000000000LL;      // a grid barrier's bound, ~2 s
+constexpr long long kLoopWaitCyclesLost = 40000000LL;  // ... in a launch that is made to lose an arrival, ~20 ms
 
 template <class T>
 __device__ __forceinline__ void record(SolveStateT<T>* st, T v) {
@@ -635,6 +636,13 @@ struct Pair2<float> {
   using type = float2;
 };
 
+// A grid barrier's bound, and the arrival count at which block 0 keeps its own back
+// (0: never): the failure the bound is there for, made without a fault.
+struct LoopWait {
+  long long cycles;
+  unsigned int lost;
+};
+
 // The partials of this block's logical blocks (acc[v]: logical block v of the
 // thread's slot), reduced as grid_reduce does.
 template <int NC, int V, class T>
@@ -697,20 +705,21 @@ __device__ __forceinline__ void loop_sums(int G, const T* partials, T* s_stage, 
 // blocks with partials in distributed shared memory, 9.9 (16 SMs' FP64 units).
 template <int NC, int V, class T>
 __device__ __forceinline__ bool loop_exchange(T (&acc)[V][NC], T* partials, unsigned int* count, unsigned int& target,
-                                              T (&s_warp)[V][2][32], int G, T* s_stage, T (&s_sum)[2], int& s_ok,
-                                              T (&out)[NC]) {
+                                              LoopWait wait, T (&s_warp)[V][2][32], int G, T* s_stage, T (&s_sum)[2],
+                                              int& s_ok, T (&out)[NC]) {
   loop_partials<NC, V>(acc, s_warp, G, partials);
   __syncthreads();
   target += gridDim.x;
   if (threadIdx.x == 0) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    if (blockIdx.x != 0 || target != wait.lost)
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
     const long long t0 = clock64();
     int ok = 1;
     for (unsigned it = 1;; ++it) {
       unsigned int c;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
       if ((int)(c - target) >= 0) break;
-      if ((it & 255) == 0 && clock64() - t0 > kLoopWaitCycles) {
+      if ((it & 255) == 0 && clock64() - t0 > wait.cycles) {
         ok = 0;
         break;
       }
@@ -726,7 +735,7 @@ __device__ __forceinline__ bool loop_exchange(T (&acc)[V][NC], T* partials, unsi
 template <class View, class T, int V, int M>
 __global__ void __launch_bounds__(1024, 1)
     k_cgj_loop(int n, View A, typename Pair2<T>::type* zp, T* r, const T* __restrict__ inv, const T* __restrict__ w,
-               SolveStateT<T>* st, Red<T> red_a, Red<T> red_b, int G) {
+               SolveStateT<T>* st, Red<T> red_a, Red<T> red_b, int G, LoopWait wait) {
   using P2 = typename Pair2<T>::type;
   __shared__ T s_warp[V][2][32];
   __shared__ T s_sum[2];
@@ -737,7 +746,7 @@ __global__ void __launch_bounds__(1024, 1)
   // odd: which of two partials buffers (alternate ones, so that none is written while it is read)
   auto exchange = [&](auto& acc, auto& out, int odd) {
     return loop_exchange<sizeof(out) / sizeof(T), V>(acc, odd ? red_b.partials : red_a.partials, &st->barrier, target,
-                                                     s_warp, G, s_stage, s_sum, s_ok, out);
+                                                     wait, s_warp, G, s_stage, s_sum, s_ok, out);
   };
   const int slots = blockDim.x >> 8, slot = threadIdx.x >> 8, lt = threadIdx.x & 255;
   int row[V][M];  // this thread's rows, n where it has none
@@ -1241,10 +1250,15 @@ void Krylov<T>::launch_loop() {
   const T* inv = diag_inv();
   const T* weight = stop_weight;
   Red<T> ra = red_of<T>(ctx, 2), rb = red_of<T>(ctx, 3);
+  LoopWait wait{kLoopWaitCycles, 0u};
+  if (ctx->lose_arrival_at > 0) {  // (once)
+    wait = LoopWait{kLoopWaitCyclesLost, (unsigned int)(ctx->lose_arrival_at * f.blocks)};
+    ctx->lose_arrival_at = 0;
+  }
   with_op([&](auto view) {
     using View = decltype(view);
     int nn = n;
-    void* args[] = {&nn, &view, &zp, &r, (void*)&inv, (void*)&weight, &d_st, &ra, &rb, &g};
+    void* args[] = {&nn, &view, &zp, &r, (void*)&inv, (void*)&weight, &d_st, &ra, &rb, &g, &wait};
     const void* k = f.V == 1 ? (const void*)k_cgj_loop<View, T, 1, 1>
                     : f.M == 1 ? (const void*)k_cgj_loop<View, T, 2, 1>
                     : f.M == 2 ? (const void*)k_cgj_loop<View, T, 2, 2>

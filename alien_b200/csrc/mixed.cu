@@ -295,7 +295,9 @@ int ab2_mixed_solve(ab2_mixed* M, const ab2_vector* b, ab2_vector* x, ab2_mixed_
           error = AB2_ERR_TIMEOUT;
           break;
         }
-        if (st.error && st.iter == 0) {  // the inner solve could not start: nothing to add
+        // Nothing to add of an inner solve that could not start, or whose wait ran out
+        // (its blocks may have left at different points: d is no iterate).
+        if (st.error == AB2_ERR_TIMEOUT || (st.error && st.iter == 0)) {
           error = st.error;
           break;
         }

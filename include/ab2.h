@@ -539,6 +539,12 @@ int ab2_selftest_mbarrier_wait(ab2_context* ctx, int* expired, double* seconds);
 /* Host-side fault injection: the nth device allocation on ctx from now on
  * fails as AB2_ERR_OOM (once); 0 turns it off. */
 int ab2_context_inject_alloc_failure(ab2_context* ctx, long long nth);
+/* The same for the grid barriers of the one-launch CG loop: in the next such loop
+ * on ctx (a solve of CG with AB2_PC_DIAG or AB2_PC_NONE, or a mixed solve's inner
+ * one) one block never arrives at the nth barrier, every wait of that launch is
+ * bounded by ~20 ms instead of ~2 s, and the solve reports AB2_ERR_TIMEOUT; 0
+ * turns it off. */
+int ab2_context_inject_lost_arrival(ab2_context* ctx, long long nth);
 
 #ifdef __cplusplus
 }

@@ -51,6 +51,46 @@ def test_mbarrier_wait_gives_up_and_context_stays_usable(ctx):
     A.close()
 
 
+# A grid barrier of the one-launch CG loop that one block never reaches: its first,
+# those of the first iteration, one well into the solve.
+@pytest.mark.parametrize("nth", [1, 2, 3, 30])
+def test_lost_arrival_ends_a_one_launch_cg_solve_as_a_timeout(ctx, nth):
+    P = abi.poisson(20, 21, 22, seed=0)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals)
+    S = abi.Solver(ctx, A, solver="cg", precond="diag", tol=1e-8, max_iter=200)
+    b = ctx.vector(P.b)
+    ref = ctx.vector(P.n)
+    good = S.solve(b, ref)
+    assert good.succeeded and good.iterations > 15
+    ctx.inject_lost_arrival(nth)
+    st = S.solve(b, ctx.vector(P.n))
+    assert st.error == abi.AB2_ERR_TIMEOUT and not st.succeeded
+    x = ctx.vector(P.n)
+    st = S.solve(b, x)  # the next one is whole again
+    assert st.succeeded and st.error == 0 and st.iterations == good.iterations
+    np.testing.assert_array_equal(x.download(), ref.download())
+    S.close()
+    A.close()
+
+
+# The same inside mixed precision: x keeps what the refinement steps before the
+# failed one made of it, whatever the failed inner solve has left behind.
+@pytest.mark.parametrize("nth", [1, 3, 30])
+def test_lost_arrival_ends_a_mixed_solve_as_a_timeout(ctx, nth):
+    P = abi.poisson(20, 21, 22, seed=0)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals, abi.FMT_CSR | abi.FMT_ELL | abi.FMT_F32)
+    M = abi.Mixed(ctx, A, solver="cg", precond="diag", tol=1e-12, inner_tol=1e-5)
+    b, x = ctx.vector(P.b), ctx.vector(P.n)
+    ctx.inject_lost_arrival(nth)
+    st = M.solve(b, x)
+    assert st.error == abi.AB2_ERR_TIMEOUT and not st.succeeded and st.outer_iterations == 0
+    np.testing.assert_array_equal(x.download(), np.zeros(P.n))
+    st = M.solve(b, x)
+    assert st.succeeded and st.error == 0
+    M.close()
+    A.close()
+
+
 def _tridiag(n, diag0):
     rp, ci, vv = [0], [], []
     for i in range(n):
