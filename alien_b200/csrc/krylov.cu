@@ -234,6 +234,7 @@ __global__ void k_cg_xfix(int n, const T* __restrict__ p, const SolveStateT<T>* 
 template <class View, class T, int VB = 1>
 __global__ void __launch_bounds__(kCtlThreads) k_cg_spmv(int n, View A, const T* __restrict__ p, T* __restrict__ q,
                                                          SolveStateT<T>* st, Red<T> red) {
+  if (st->done) return;  // (a body past the end)
   T acc[VB][1] = {};
   const int lstride = gridDim.x * blockDim.x;  // between a thread's logical threads
   for (int base = blockIdx.x * blockDim.x + threadIdx.x; base < n; base += VB * lstride) {
@@ -335,6 +336,7 @@ template <bool UNIT>
 __global__ void __launch_bounds__(kCtlThreads) k_cg_spmv_x4(int n, StencilView<float, true, UNIT> A,
                                                             const float* __restrict__ p, float* __restrict__ q,
                                                             SolveStateT<float>* st, Red<float> red, int G) {
+  if (st->done) return;  // (a body past the end)
   const int S = G * kCtlThreads;  // rows per sweep of the logical grid
   const int t4 = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   const size_t N = (size_t)n;
@@ -1292,17 +1294,17 @@ void Krylov<T>::build_graph() {
   // an iteration: 82.6 us with one body a turn, 79.3 with four); bodies past the end
   // return or write what nothing reads (the host-driven loop queues them too).  A
   // preconditioned body is too dear to run past the end.
-  const int bodies = fused_diag ? 4 : 1;
+  turn_bodies = fused_diag ? 4 : 1;
   int launched = 0;
   try {
-    for (int i = 0; i < bodies; ++i) launched = enqueue_body(handle, 1);
+    for (int i = 0; i < turn_bodies; ++i) launched = enqueue_body(handle, 1);
   } catch (...) {
     cudaGraph_t dummy;
     cudaStreamEndCapture(ctx->stream, &dummy);
     throw;
   }
   AB2_CUDA(cudaStreamEndCapture(ctx->stream, &body));
-  ctx->launches -= launched * bodies;  // captured, not launched
+  ctx->launches -= launched * turn_bodies;  // captured, not launched
   body_launches = launched;
   AB2_CUDA(cudaGraphInstantiate(&exec, graph, 0));
 }
@@ -1385,7 +1387,10 @@ void Krylov<T>::solve(const T* b, T* x, T tol, int max_iter) {
   }
   AB2_CUDA(cudaMemcpyAsync(h_st, d_st, sizeof(SolveStateT<T>), cudaMemcpyDeviceToHost, ctx->stream));
   AB2_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (use_graph) ctx->launches += (long long)h_st->bodies * body_launches;
+  if (use_graph) {  // whole turns of the graph's loop
+    const long long turns = (h_st->bodies + turn_bodies - 1) / turn_bodies;
+    ctx->launches += turns * turn_bodies * body_launches;
+  }
 }
 
 template <class T>

@@ -50,6 +50,7 @@ struct Krylov {
   cudaGraphExec_t exec = nullptr;
   cudaGraphConditionalHandle handle = 0;
   int body_launches = 0;
+  int turn_bodies = 1;  // loop bodies in a turn of the graph's loop
   bool fused_diag = false;  // CG with Diag or no preconditioner: the two-kernel body
   bool one_launch = false;  // ... and its whole loop in one cooperative launch
   // Operator override (set before init): the symmetric unit-diagonal 7-point

@@ -294,3 +294,20 @@ def test_one_launch_cg_breakdown_and_null_rhs(ctx):
         np.testing.assert_array_equal(z.download(), np.full(n, 3.0))
         S.close()
     assert res[0] == res[1]
+
+
+@pytest.mark.parametrize("iters", [1, 3, 4, 5])
+def test_launch_count_holds_the_whole_turns_of_the_graph_loop(ctx, iters):
+    """Beyond the one-launch loop's sizes a turn of the graph runs four bodies of
+    two kernels, whether or not the last ones are past the end; before it b.b, the
+    state, the residual and the start, after it the true residual."""
+    P = abi.poisson(104, 104, 104, seed=0)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals)
+    S = abi.Solver(ctx, A, solver="cg", precond="diag", tol=1e-14, max_iter=iters)
+    b, x = ctx.vector(P.b), ctx.vector(P.n)
+    before = ctx.launches
+    st = S.solve(b, x)
+    assert st.iterations == iters
+    assert ctx.launches - before == 4 + (iters + 3) // 4 * 4 * 2 + 1
+    S.close()
+    A.close()
