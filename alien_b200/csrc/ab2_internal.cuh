@@ -74,6 +74,7 @@ struct ab2_matrix {
   ab2_context* ctx = nullptr;
   int n = 0;
   long long nnz = 0;
+  int widest_row = 0;         // the most entries of a row
   int formats = 0;
   long long device_bytes = 0;
   // CSR (always present: ILU0, invdiag and L/U products use it)

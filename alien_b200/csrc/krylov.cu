@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(1024, 1)
 
 // How a system of n rows fits the one-launch loop: threads a block, blocks, and
 // the rows of a thread (V logical blocks of the reduction grid, M rows each).
-// Where the line lies: up to three rows a logical thread in FP64 (909,000 rows on 148
+// Where the line lies for short rows: up to three rows a logical thread in FP64 (909,000 rows on 148
 // SMs), four in FP32, beyond which the graph loop's two bandwidth-bound kernels are
 // as fast.  Measured on B200, us an iteration, graph loop / one launch: 7-point
 // bands FP64 32^3 15.2 / 6.6, 64^3 21.8 / 11.9, 491,111 rows 24.7 / 18.1, 96^3 32.4 /
@@ -904,6 +904,28 @@ CgLoopFit cg_loop_fit(const ab2_context* ctx, int n, bool fp32) {
   f.V = v;
   f.M = m == 1 ? 1 : m == 2 ? 2 : 4;
   return f;
+}
+
+// Whether its rows are short enough for it.  One thread sums a row, and in the
+// one-launch loop an SM has half as many threads to wait with, each operand is a
+// pair (z, p) past L1, and a row of the wide ELL view works out of spilled
+// registers; so wide rows, and in FP32, where the graph loop reads p once for
+// all, many entries, belong to the graph loop.  Measured on B200, us an iteration,
+// graph loop / one launch, k entries in every row, columns scattered over n^(2/3)
+// rows: FP32 ELL 600,000 rows k = 12 40.4 / 39.6, 16 44.2 / 51.5, 300,000 rows k = 16
+// 30.8 / 26.5, 24 35.1 / 36.7, 32 38.4 / 44.8, 100,000 rows k = 32 23.8 / 22.2, 64 31.8 /
+// 37.2; FP64 ELL 600,000 rows k = 32 115 / 101, 100,000 rows k = 32 29.1 / 25.7, 64 39.6 /
+// 42.3; FP32 CSR 600,000 rows k = 32 183 / 174, 100,000 rows k = 32 41.9 / 41.2, 64 53.6 /
+// 62.3; FP64 CSR 300,000 rows k = 64 216 / 161.  One row of L entries among rows of 7
+// (2,000 rows): ELL FP64 L = 64 23.2 / 23.0, 128 28.9 / 40.1, FP32 21.3 / 20.5, 24.7 /
+// 36.8; CSR FP64 L = 1,900 244 / 220, FP32 L = 512 45.8 / 41.1, 1,900 99.7 / 139.
+bool cg_loop_pays(const ab2_matrix* A, ViewKind kind, bool fp32) {
+  if (kind == ViewKind::Stencil) return true;
+  const bool ell = kind == ViewKind::Ell;
+  const int any_size = ell ? (fp32 ? 16 : 32) : (fp32 ? 32 : 2048);  // widest row at any size ...
+  const int small = ell ? 72 : (fp32 ? 512 : 2048);                  // ... of few entries
+  if (A->widest_row > any_size) return A->widest_row <= small && A->nnz <= 3200000;
+  return !(ell && fp32) || A->nnz <= 8000000;
 }
 
 // ------------------------------------------------------------------ BiCGStab
@@ -1319,7 +1341,9 @@ void Krylov<T>::init(ab2_context* c, const ab2_matrix* a, const ab2_precond* p, 
   variant = spmv_variant;
   use_graph = graph_loop;
   fused_diag = solver == AB2_SOLVER_CG && pc && (pc->kind == AB2_PC_DIAG || pc->kind == AB2_PC_NONE);
-  one_launch = use_graph && fused_diag && cg_loop_fit(ctx, A->n, sizeof(T) == 4).V > 0;
+  const ViewKind view = unit_bands ? ViewKind::Stencil : view_kind<T>(A, variant);
+  one_launch = use_graph && fused_diag && cg_loop_fit(ctx, A->n, sizeof(T) == 4).V > 0 &&
+               cg_loop_pays(A, view, sizeof(T) == 4);
   // (the one-launch loop keeps r, and z and p side by side)
   const int nw = one_launch ? 2 : fused_diag ? 5 : solver == AB2_SOLVER_CG ? (sizeof(T) == sizeof(double) ? 5 : 4) : 8;
   for (int i = 0; i < nw; ++i) {

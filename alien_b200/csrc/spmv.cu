@@ -33,13 +33,17 @@ namespace ab2 {
 namespace {
 
 // ----------------------------------------------------------------- set-up kernels
-__global__ void k_validate(int n, const int* __restrict__ rp, const int* __restrict__ ci, int* bad) {
+// out[0]: what is wrong (bits), out[1]: the most entries of a row.
+__global__ void k_validate(int n, const int* __restrict__ rp, const int* __restrict__ ci, int* out) {
+  int* bad = out;
+  int widest = 0;
   for (int row = blockIdx.x * blockDim.x + threadIdx.x; row < n; row += gridDim.x * blockDim.x) {
     const int a = rp[row], b = rp[row + 1];
     if (b < a) {
       atomicOr(bad, 1);
       continue;
     }
+    widest = max(widest, b - a);
     int prev = -1;
     for (int k = a; k < b; ++k) {
       const int c = ci[k];
@@ -48,6 +52,8 @@ __global__ void k_validate(int n, const int* __restrict__ rp, const int* __restr
       prev = c;
     }
   }
+  widest = __reduce_max_sync(0xffffffffu, widest);
+  if ((threadIdx.x & 31) == 0) atomicMax(out + 1, widest);
 }
 
 __global__ void k_dcol(int n, const int* __restrict__ rp, const int* __restrict__ ci, int* __restrict__ dcol) {
@@ -677,14 +683,16 @@ int ab2_matrix_create_csr(ab2_context* ctx, int n, const int* row_ptr, const int
     AB2_CUDA(cudaMemcpyAsync(A->d_v, vals, sizeof(double) * nnz, cudaMemcpyHostToDevice, ctx->stream));
     if (n > 0) {
       // Device-side profile check: every later kernel indexes x by these columns.
-      int* d_bad = dev_alloc<int>(ctx, 1);
-      AB2_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(int), ctx->stream));
-      k_validate<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, A->d_rp, A->d_ci, d_bad);
+      int* d_found = dev_alloc<int>(ctx, 2);
+      AB2_CUDA(cudaMemsetAsync(d_found, 0, 2 * sizeof(int), ctx->stream));
+      k_validate<<<grid_for(n), kThreads, 0, ctx->stream>>>(n, A->d_rp, A->d_ci, d_found);
       check_launch(ctx, "validate");
-      int bad = 0;
-      AB2_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+      int found[2] = {0, 0};
+      AB2_CUDA(cudaMemcpyAsync(found, d_found, sizeof(found), cudaMemcpyDeviceToHost, ctx->stream));
       AB2_CUDA(cudaStreamSynchronize(ctx->stream));
-      dev_free(ctx, d_bad);
+      dev_free(ctx, d_found);
+      const int bad = found[0];
+      A->widest_row = found[1];
       if (bad & 1) throw Error{AB2_ERR_BAD_ARG, "row_ptr is not non-decreasing"};
       if (bad & 2) throw Error{AB2_ERR_BAD_ARG, "column index out of range"};
       if (bad & 4) throw Error{AB2_ERR_BAD_ARG, "columns must be strictly increasing inside each row"};

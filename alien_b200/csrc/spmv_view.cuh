@@ -257,23 +257,35 @@ StencilView<T, SYM, UNIT> stencil_view(const ab2_matrix* A, const T* bands) {
                                    FastDiv((unsigned)A->st_ny)};
 }
 
-// Calls f(view) with the view the variant selects: the 7-point bands when
-// chosen and present in T, ELL when chosen and present, else CSR.
+// The view the variant selects: the 7-point bands when chosen and present in T,
+// ELL when chosen and present, else CSR.
+enum class ViewKind { Stencil, Ell, Csr };
+template <class T>
+ViewKind view_kind(const ab2_matrix* A, int variant) {
+  const bool f32 = sizeof(T) == 4;
+  const int v = resolve_variant(A, variant);
+  if (v == AB2_SPMV_STENCIL && (f32 ? A->d_st_v32 != nullptr : A->d_st_v != nullptr)) return ViewKind::Stencil;
+  if ((v == AB2_SPMV_ELL || v == AB2_SPMV_STENCIL) && (f32 ? A->d_ell_v32 != nullptr : A->d_ell_v != nullptr))
+    return ViewKind::Ell;
+  return ViewKind::Csr;
+}
+
+// Calls f(view) with that view.
 // kStencil = false leaves the band views out (callers whose kernels are never
 // given a 7-point matrix, so that they are not instantiated for it).
 template <class T, bool kStencil = true, class F>
 void with_view(const ab2_matrix* A, int variant, F&& f) {
   const bool f32 = sizeof(T) == 4;
-  const int v = resolve_variant(A, variant);
+  const ViewKind kind = view_kind<T>(A, variant);
   const T* ev = (const T*)(f32 ? (const void*)A->d_ell_v32 : (const void*)A->d_ell_v);
   const T* cv = (const T*)(f32 ? (const void*)A->d_v32 : (const void*)A->d_v);
   const T* sv = (const T*)(f32 ? (const void*)A->d_st_v32 : (const void*)A->d_st_v);
-  if (kStencil && v == AB2_SPMV_STENCIL && sv) {
+  if (kStencil && kind == ViewKind::Stencil) {
     if constexpr (kStencil) {
       if (A->st_bands == 4) f(stencil_view<T, true>(A, sv));
       else f(stencil_view<T, false>(A, sv));
     }
-  } else if ((v == AB2_SPMV_ELL || v == AB2_SPMV_STENCIL) && ev) {
+  } else if (ev && kind != ViewKind::Csr) {
     f(EllView<T>{A->d_ell_off, A->d_ell_ci, ev});
   } else {
     require(cv != nullptr, "matrix values missing in the requested precision");

@@ -311,3 +311,38 @@ def test_launch_count_holds_the_whole_turns_of_the_graph_loop(ctx, iters):
     assert ctx.launches - before == 4 + (iters + 3) // 4 * 4 * 2 + 1
     S.close()
     A.close()
+
+
+# Rows too wide for the one-launch loop take the graph loop: told apart by the
+# launches of a solve of 20 iterations, either side of each width limit.
+@pytest.mark.parametrize("variant,fp32,limit", [(abi.SPMV_ELL, False, 72), (abi.SPMV_CSR_SCALAR, False, 2048),
+                                                (abi.SPMV_ELL, True, 72), (abi.SPMV_CSR_SCALAR, True, 512)])
+def test_wide_rows_take_the_graph_loop(ctx, variant, fp32, limit):
+    n, iters = 5000, 20
+    for widest, one_launch in ((7, True), (limit, True), (limit + 1, False)):
+        row = np.concatenate([np.arange(n), np.full(widest - 1, n // 2)])
+        col = np.concatenate([np.arange(n), np.delete(np.arange(n), n // 2)[: widest - 1]])
+        order = np.lexsort((col, row))
+        row, col = row[order], col[order]
+        rp = np.zeros(n + 1, np.int32)
+        rp[1:] = np.cumsum(np.bincount(row, minlength=n))
+        vals = np.where(row == col, np.linspace(2.0, 9.0, n)[row], -1e-3)
+        A = ctx.matrix(rp, col.astype(np.int32), vals, abi.FMT_CSR | abi.FMT_ELL | abi.FMT_F32)
+        b = ctx.vector(np.random.default_rng(widest).uniform(-1, 1, n))
+        out = []
+        for graph in (True, False):
+            x = ctx.vector(n)
+            if fp32:
+                S = abi.Mixed(ctx, A, solver="cg", precond="none", tol=1e-30, max_outer=1, inner_tol=1e-12,
+                              inner_max_iter=iters, spmv_variant=variant, use_graph=graph)
+            else:
+                S = abi.Solver(ctx, A, solver="cg", precond="none", tol=1e-30, max_iter=iters, spmv_variant=variant,
+                               use_graph=graph)
+            before = ctx.launches
+            S.solve(b, x)
+            if graph:
+                assert (ctx.launches - before < 2 * iters) == one_launch
+            out.append(x.download())
+            S.close()
+        np.testing.assert_array_equal(out[0], out[1])
+        A.close()
