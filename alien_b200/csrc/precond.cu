@@ -418,8 +418,8 @@ __global__ void k_cheb1_start(int n, const T* x, const T* __restrict__ inv, T in
 
 // The start and the first step in one pass (x and y different vectors): the
 // step forms w = (D^-1 x) / theta at every row it reads, so neither r, w nor y is
-// stored and read back in between (40 bytes a row stored or read less in FP64, of
-// 128).  last: nothing comes after, r and w are not stored.
+// stored and read back in between (FP64 and four bands: 128 bytes a row in two
+// passes, 72 in one).  last: nothing comes after, r and w are not stored.
 template <class View, class T>
 __global__ void __launch_bounds__(kThreads) k_cheb1_first(int n, View A, const T* __restrict__ x,
                                                           const T* __restrict__ inv, T inv_theta, T* __restrict__ r,
@@ -438,6 +438,20 @@ __global__ void __launch_bounds__(kThreads) k_cheb1_first(int n, View A, const T
     wnext[row] = wv;
   }
   y[row] = fma_rn(T(1), wv, w0);
+}
+
+// Whether the start goes into the first step.  Every entry then gathers two words, x
+// and 1/a, instead of one.  With bands the neighbours are at hand: always.  With
+// column indices only where the launch counts more than the gathers.  Measured on
+// B200, us an application of order 2, two passes / one, k entries a row scattered
+// over n^(2/3) rows: ELL 5,000 rows k = 24 9.7 / 8.5, 32 9.5 / 10.5; 50,000 rows k = 24
+// 11.9 / 10.6; 100,000 rows k = 12 11.1 / 9.5, 24 14.7 / 14.7; 200,000 rows k = 5 12.6 /
+// 10.7, 7 12.7 / 12.7, 9 14.7 / 15.8; 2,000,000 rows k = 7 72 / 97, 24 179 / 290; CSR 200,000
+// rows k = 7 14.8 / 14.8, 9 16.8 / 18.8.
+template <class T>
+bool cheb_fuses_start(const ab2_matrix* A, int variant) {
+  if (view_kind<T>(A, variant) == ViewKind::Stencil) return true;
+  return A->widest_row <= 24 && A->nnz <= 1400000;
 }
 
 // _algo1 step (:342-354): r -= D^-1 A w ; w = c1 w + c2 r ; y += w, with the
@@ -911,7 +925,7 @@ void apply_t(ab2_context* ctx, const ab2_precond* pc, const T* x, T* y) {
         T* wv[2] = {w.y0, w.y1};
         const int blocks = (n + kThreads - 1) / kThreads;
         int k = 1;
-        if (steps > 1 && x != y) {
+        if (steps > 1 && x != y && cheb_fuses_start<T>(pc->A, pc->variant)) {
           with_view<T>(pc->A, pc->variant, [&](auto view) {
             k_cheb1_first<<<blocks, kThreads, 0, ctx->stream>>>(n, view, x, w.inv, (T)c.inv_theta, r, wv[1], y,
                                                                 (T)c.a[1], (T)c.b[1], steps == 2);

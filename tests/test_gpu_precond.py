@@ -289,3 +289,46 @@ def test_chebyshev_start_vector_drawn_on_the_device(ctx, n):
         bounds = O.cheb_bounds(rp, ci, vals, 0.0, 3, dot_mode=O.DOT_DEVICE_TREE,
                                tree_blocks=ctx.info.reduction_max_blocks)
     np.testing.assert_array_equal([pc.info.cheb_alpha, pc.info.cheb_beta], bounds)
+
+
+# The start goes into Saad's first step where that pays (bands, or few and narrow
+# rows): seen by an application's launches, either side of the limits, with the
+# oracle's bits in both forms.
+@pytest.mark.parametrize("n,per_row,widest,fused", [(900, 3, 24, True), (900, 3, 25, False), (200000, 7, 7, True),
+                                                    (200001, 7, 7, False)])
+def test_chebyshev_start_fused_where_it_pays(ctx, n, per_row, widest, fused):
+    rows = np.repeat(np.arange(n), per_row)
+    cols = (rows + np.tile(np.arange(per_row) - per_row // 2, n)) % n
+    if widest > per_row:
+        rows = np.concatenate([rows, np.full(widest - per_row, 5)])
+        cols = np.concatenate([cols, np.arange(100, 100 + widest - per_row)])
+    order = np.lexsort((cols, rows))
+    rows, cols = rows[order], cols[order]
+    rp = np.zeros(n + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    vals = np.where(rows == cols, np.linspace(widest + 1.0, widest + 2.0, n)[rows], -0.5)
+    assert np.bincount(rows).max() == widest and (vals.size <= 1400000) == (n <= 200000)
+    A = ctx.matrix(rp, cols.astype(np.int32), vals)
+    pc = abi.Precond(ctx, A, "cheb", poly_factor=0.0, poly_order=3, poly_factor_max_iter=4, cheb_saad=True)
+    x = rnd(n, 3)
+    vx, vy = ctx.vector(x), ctx.vector(n)
+    before = ctx.launches
+    pc.apply(vx, vy)
+    assert ctx.launches - before == (2 if fused else 3)
+    exact = O.cheb_apply(rp, cols.astype(np.int32), vals, x, 0.0, 3, 4, dot_mode=O.DOT_DEVICE_TREE,
+                         tree_blocks=ctx.info.reduction_max_blocks, saad=True)
+    np.testing.assert_array_equal(vy.download(), exact)
+    A.close()
+
+
+def test_chebyshev_start_fused_with_bands(ctx):
+    P = abi.diffusion(70, 60, 50, sigma=1.0, smooth=2.0, seed=5)  # 1.45 million entries
+    x = rnd(P.n, 3)
+    for formats, launches in ((abi.FMT_CSR | abi.FMT_ELL | abi.FMT_STENCIL, 2), (abi.FMT_CSR | abi.FMT_ELL, 3)):
+        A = ctx.matrix(P.row_ptr, P.cols, P.vals, formats)
+        pc = abi.Precond(ctx, A, "cheb", poly_factor=0.0, poly_order=3, poly_factor_max_iter=4, cheb_saad=True)
+        vx, vy = ctx.vector(x), ctx.vector(P.n)
+        before = ctx.launches
+        pc.apply(vx, vy)
+        assert ctx.launches - before == launches
+        A.close()
