@@ -264,6 +264,7 @@ SIGNATURES: dict[str, tuple] = {
     "ab2_matrix_market_error": (C.c_char_p, []),
     "ab2_selftest_bounded_wait": (_I, [_P, _IP, _DP]),
     "ab2_selftest_mbarrier_wait": (_I, [_P, _IP, _DP]),
+    "ab2_selftest_batch_build": (_I, [_P, _IP]),
     "ab2_context_inject_alloc_failure": (_I, [_P, C.c_longlong]),
     "ab2_context_inject_lost_arrival": (_I, [_P, C.c_longlong]),
     "ab2_rng_u64": (C.c_uint64, [C.c_uint64, C.c_uint64, C.c_uint64]),
@@ -973,6 +974,12 @@ class Batch:
         i = BatchInfo()
         self.ctx.check(lib().ab2_batch_get_info(self.h, C.byref(i)), "batch_info")
         return i
+
+    def selftest_build(self) -> int:
+        """The kernel build the last launch ran: 0 any, 1 dense, 2 deep (-1: none yet)."""
+        n = C.c_int()
+        self.ctx.check(lib().ab2_selftest_batch_build(self.h, C.byref(n)), "selftest_batch_build")
+        return n.value
 
     def trials(self) -> list[tuple[int, int, int, float, int, int]]:
         """(spmv_variant, cluster_size, threads, ms, ell_slice, lanes_per_row) per autotuning trial."""

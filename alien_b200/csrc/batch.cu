@@ -155,15 +155,22 @@ __device__ __forceinline__ void rows_f(const EllViewS<T, S>& A, const int (&r)[U
 // 192,721 rows on 8 x 512 threads); rows side by side take registers, and with
 // them clusters off the GPU.  Dense: one row of the SpMV and four of the update at a
 // time, 64 registers, two CTAs of 512 threads an SM.  Deep: two rows of the SpMV, 128
-// registers, one CTA of 512 an SM.  Any: one row, for CTAs of up to 1,024 threads.
+// registers, one CTA of 512 an SM (formats with one lane a row only).  Any: one row, for
+// CTAs of up to 1,024 threads.
 enum class Build { Any, Dense, Deep };
 template <Build B>
 constexpr int kSpmvRows = B == Build::Deep ? 2 : 1;
 template <Build B>
 constexpr int kUpdateRows = B == Build::Any ? 1 : 4;
 
+// Threads and CTAs an SM that a build is compiled for (576: 56 registers, so that more
+// of the small CTAs fit than with 64; 1,000 systems of 50 to 200 rows, CTAs of 64 threads,
+// four lanes a row: 1.08 ms with 64, 0.99 with 56).
+template <class V32, Build B>
+constexpr int kMaxThreads = B == Build::Any ? 1024 : lanes_per_row<V32>::value > 1 ? 576 : 512;
+
 template <class V64, class V32, Build BUILD>
-__global__ void __launch_bounds__(BUILD == Build::Any ? 1024 : 512, BUILD == Build::Dense ? 2 : 1)
+__global__ void __launch_bounds__(kMaxThreads<V32, BUILD>, BUILD == Build::Dense ? 2 : 1)
     k_batch_cg(BatchArgs<V64, V32> a) {
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ double s_part64[2][4];
@@ -396,12 +403,36 @@ struct ab2_batch {
   int tuned = 0;
   double tune_ms = 0, setup_ms = 0, solve_ms = 0;
   std::vector<ab2_batch_trial> trials;
-  std::vector<double> work;  // rows^1.5 of the first k systems, largest first
+  std::vector<int> rows;  // of the systems, largest first
+  int last_build = -1;    // the kernel's build in the last launch (Build)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 };
 
 namespace ab2 {
 namespace {
+
+// Deep or dense, for a format with a row a thread (rows: of the systems, largest
+// first; cdeep: clusters of the deep build that the GPU holds, half the dense one's).
+// An iteration takes a cluster its rows a thread, and never less than one; iterations
+// grow with the side of a 2-D grid, sqrt(rows).  With that as a system's work, deep
+// where the largest system is at least 1 / c of what each deep cluster has to do on
+// average -- it then ends the launch, and its own pace counts.  How much faster deep
+// makes that pace depends on the rows a thread r of the largest system: c = 3 from 4
+// rows on, 2 from 2 on, and below that, where there is nothing to take side by
+// side, 1.  Measured on B200, ELL, ms (before the builds; dense; deep; total work over
+// the largest's): 8 x 512, 24 systems of up to 200,000 rows (r = 49; 3.8) 431, 339, 220;
+// 96 (14) 611, 524, 311; 192 of up to 100,000 (34) 253, 215, 194; 512 of up to 200,000 (75)
+// 1234, 987, 1088; 40 of 100 to 400 rows (r = 0.1; 28) 0.41, 0.41, 0.49; 16 x 512, 64 of
+// 2,000 to 20,000 (r = 2.4; 20) 20.1, 20.1, 26.6; 24 of 5,000 to 50,000 (r = 6.1) deep 32.9 for
+// 47.7.
+bool batch_is_deep(const int* rows, int nsys, int threads, int cdeep) {
+  if (cdeep < 1) return false;
+  auto work = [&](int n) { return std::sqrt((double)n) * std::max(1.0, (double)n / threads); };
+  const double r = (double)rows[0] / threads, c = r >= 4 ? 3 : r >= 2 ? 2 : 1;
+  double total = 0;
+  for (int i = 0; i < nsys; ++i) total += work(rows[i]);
+  return total <= c * cdeep * work(rows[0]);
+}
 
 // Launches the persistent kernel over the first nsys_run systems of the
 // largest-first order.  Returns false (nothing launched) when not even one
@@ -448,14 +479,6 @@ bool launch_batch(ab2_batch* B, V64 a64, V32 a32, int csize, int threads, const 
   cfg.stream = ctx->stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // Dense or deep: with the work of a system taken as rows^1.5 (iterations grow
-  // with the side of a 2-D grid), deep where the largest system is more than two
-  // thirds of what each of the dense build's clusters has to do on average -- it
-  // then ends the launch, and its own pace counts -- else dense.  Measured on B200
-  // (8 x 512, ms; before, dense, deep; total work over the largest's): 24 systems of up
-  // to 200,000 rows (3.8) 431, 339, 220; 96 (14) 611, 524, 311; 96 of up to 50,000 (20)
-  // 92, 83, 49; 192 of up to 100,000 (34) 253, 215, 194; 512 of up to 200,000 (75)
-  // 1234, 987, 1088.
   auto fit = [&](auto* k) {
     if (csize > 8)  // 16-CTA clusters are beyond the portable size
       AB2_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -463,28 +486,35 @@ bool launch_batch(ab2_batch* B, V64 a64, V32 a32, int csize, int threads, const 
     AB2_CUDA(cudaOccupancyMaxActiveClusters(&c, (void*)k, &cfg));
     return c;
   };
+  constexpr int kLanes = lanes_per_row<V32>::value;
   auto* kernel = k_batch_cg<V64, V32, Build::Any>;
   int nclusters = 0;
+  Build build = Build::Any;
   if (threads <= 512) {
-    kernel = k_batch_cg<V64, V32, Build::Dense>;
-    nclusters = fit(kernel);
-    if (1.5 * B->work[1] * nclusters > B->work[nsys_run]) {
+    // (up to a row a thread there is nothing for the dense build to take side by side:
+    // 1 x 512, 300 systems of 100 to 400 rows, 0.40 ms dense, 0.36 as one row a time)
+    if (kLanes > 1 || B->rows[0] > csize * threads) {
+      build = Build::Dense;
+      kernel = k_batch_cg<V64, V32, Build::Dense>;
+    }
+    if constexpr (kLanes == 1) {
       auto* deep = k_batch_cg<V64, V32, Build::Deep>;
-      const int c = fit(deep);
-      if (c >= 1) {
+      const int cdeep = fit(deep);
+      if (batch_is_deep(B->rows.data(), nsys_run, csize * threads, cdeep)) {
+        build = Build::Deep;
         kernel = deep;
-        nclusters = c;
+        nclusters = cdeep;
       }
     }
-  } else {
-    nclusters = fit(kernel);
   }
+  if (build != Build::Deep) nclusters = fit(kernel);
   if (nclusters < 1) return false;
   nclusters = std::min(nclusters, nsys_run);
   cfg.gridDim = dim3((unsigned)(nclusters * csize));
   AB2_CUDA(cudaMemsetAsync(B->d_ticket, 0, sizeof(unsigned int), ctx->stream));
   AB2_CUDA(cudaLaunchKernelEx(&cfg, kernel, args));
   check_launch(ctx, "batch_cg");
+  B->last_build = (int)build;
   return true;
 }
 
@@ -663,8 +693,8 @@ int ab2_batch_create(ab2_context* ctx, const ab2_matrix* A, int nsys, const int*
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
       return sys_offsets[a + 1] - sys_offsets[a] > sys_offsets[b + 1] - sys_offsets[b];
     });
-    B->work.assign(1, 0.0);
-    for (int i : order) B->work.push_back(B->work.back() + std::pow((double)(sys_offsets[i + 1] - sys_offsets[i]), 1.5));
+    B->rows.clear();
+    for (int i : order) B->rows.push_back(sys_offsets[i + 1] - sys_offsets[i]);
     B->d_off = dev_alloc<int>(ctx, (size_t)nsys + 1);
     B->d_order = dev_alloc<int>(ctx, (size_t)nsys);
     AB2_CUDA(cudaMemcpyAsync(B->d_off, sys_offsets, sizeof(int) * ((size_t)nsys + 1), cudaMemcpyHostToDevice,
@@ -779,6 +809,12 @@ int ab2_batch_get_info(const ab2_batch* B, ab2_batch_info* info) {
   info->trials = (int)B->trials.size();
   info->ell_slice = B->variant == AB2_SPMV_ELL ? B->slice : 0;
   info->lanes_per_row = B->variant == AB2_SPMV_CSR_SCALAR ? B->lpr : 0;
+  return AB2_OK;
+}
+
+int ab2_selftest_batch_build(const ab2_batch* B, int* build) {
+  if (!B || !build) return AB2_ERR_BAD_ARG;
+  *build = B->last_build;
   return AB2_OK;
 }
 

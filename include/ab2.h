@@ -536,6 +536,10 @@ int ab2_selftest_bounded_wait(ab2_context* ctx, int* expired, double* seconds);
  * a wait on a barrier phase that nothing completes gives up after its clock
  * budget; *expired = 1 when it did. */
 int ab2_selftest_mbarrier_wait(ab2_context* ctx, int* expired, double* seconds);
+/* The build of the batched kernel that the last launch on this batch ran: 0 one row
+ * of a thread at a time, 1 dense (more clusters), 2 deep (rows of a thread side by side),
+ * -1 before the first launch.  The results do not depend on it. */
+int ab2_selftest_batch_build(const ab2_batch* batch, int* build);
 /* Host-side fault injection: the nth device allocation on ctx from now on
  * fails as AB2_ERR_OOM (once); 0 turns it off. */
 int ab2_context_inject_alloc_failure(ab2_context* ctx, long long nth);

@@ -141,3 +141,35 @@ def test_batch_dense_and_deep_builds(ctx, nsys, cluster, threads):
         np.testing.assert_array_equal(x, o.x)
         np.testing.assert_array_equal(S.results()[2], o.inner)
         S.close()
+
+
+ANY, DENSE, DEEP = 0, 1, 2
+
+
+# Which build a batch's launch runs: deep where the largest system ends the launch,
+# dense where the clusters count, neither without rows to take side by side or with CTAs
+# past 512 threads; several lanes a row are never deep.
+@pytest.mark.parametrize("nsys,rows,cluster,threads,lanes,build", [
+    (40, (100, 400), 4, 256, 0, DEEP), (40, (100, 400), 8, 512, 0, ANY), (40, (100, 400), 8, 512, 1, ANY),
+    (300, (100, 400), 4, 256, 0, ANY), (300, (100, 400), 1, 256, 0, DEEP), (1000, (50, 200), 1, 256, 0, ANY),
+    (600, (1000, 3000), 4, 256, 0, DENSE), (600, (1000, 3000), 4, 256, 1, DENSE),
+    (1000, (50, 200), 1, 128, 0, DEEP), (64, (2000, 20000), 16, 512, 0, DENSE), (64, (2000, 20000), 8, 512, 0, DEEP),
+    (24, (5000, 50000), 16, 512, 0, DEEP), (300, (100, 400), 1, 256, 4, DENSE), (3, (300, 6000), 1, 128, 2, DENSE), (24, (300, 6000), 8, 1024, 0, ANY)])
+def test_batch_build(ctx, nsys, rows, cluster, threads, lanes, build):
+    B = abi.batch_problem(nsys=nsys, min_rows=rows[0], max_rows=rows[1], seed=3)
+    kw = dict(spmv_variant=abi.SPMV_CSR_SCALAR, lanes_per_row=lanes) if lanes else dict(spmv_variant=abi.SPMV_ELL,
+                                                                                        ell_slice=32)
+    P = B.problem
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals, F32)
+    S = abi.Batch(ctx, A, B.sys_offsets, tol=1e-8, cluster_size=cluster, threads=threads, max_outer=2,
+                  inner_max_iter=40, **kw)
+    assert S.selftest_build() == -1
+    x = ctx.vector(P.n)
+    S.solve(ctx.vector(P.b), x)
+    assert S.selftest_build() == build
+    o = O.batch_solve(P.row_ptr, P.cols, P.vals, B.sys_offsets, P.b, tol=1e-8, max_outer=2, inner_max_iter=40,
+                      cluster_size=cluster, threads=threads, lanes_per_row=max(lanes, 1))
+    np.testing.assert_array_equal(S.results()[2], o.inner)
+    np.testing.assert_array_equal(x.download(), o.x)
+    S.close()
+    A.close()
