@@ -425,18 +425,19 @@ namespace {
 // 1234, 987, 1088; 40 of 100 to 400 rows (r = 0.1; 28) 0.41, 0.41, 0.49; 16 x 512, 64 of
 // 2,000 to 20,000 (r = 2.4; 20) 20.1, 20.1, 26.6; 24 of 5,000 to 50,000 (r = 6.1) deep 32.9 for
 // 47.7.
-bool batch_is_deep(const int* rows, int nsys, int threads, int cdeep) {
+bool batch_is_deep(const std::vector<int>& rows, int threads, int cdeep) {
   if (cdeep < 1) return false;
   auto work = [&](int n) { return std::sqrt((double)n) * std::max(1.0, (double)n / threads); };
   const double r = (double)rows[0] / threads, c = r >= 4 ? 3 : r >= 2 ? 2 : 1;
   double total = 0;
-  for (int i = 0; i < nsys; ++i) total += work(rows[i]);
+  for (int n : rows) total += work(n);
   return total <= c * cdeep * work(rows[0]);
 }
 
 // Launches the persistent kernel over the first nsys_run systems of the
-// largest-first order.  Returns false (nothing launched) when not even one
-// cluster of this shape fits on the GPU.
+// largest-first order, in the build that the whole batch calls for (so that both
+// parts of an autotuning trial time what the solve will run).  Returns false
+// (nothing launched) when not even one cluster of this shape fits on the GPU.
 template <class V64, class V32>
 bool launch_batch(ab2_batch* B, V64 a64, V32 a32, int csize, int threads, const double* b, double* x, int max_outer,
                   int inner_max_iter, int nsys_run) {
@@ -500,7 +501,7 @@ bool launch_batch(ab2_batch* B, V64 a64, V32 a32, int csize, int threads, const 
     if constexpr (kLanes == 1) {
       auto* deep = k_batch_cg<V64, V32, Build::Deep>;
       const int cdeep = fit(deep);
-      if (batch_is_deep(B->rows.data(), nsys_run, csize * threads, cdeep)) {
+      if (batch_is_deep(B->rows, csize * threads, cdeep)) {
         build = Build::Deep;
         kernel = deep;
         nclusters = cdeep;

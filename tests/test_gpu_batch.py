@@ -173,3 +173,19 @@ def test_batch_build(ctx, nsys, rows, cluster, threads, lanes, build):
     np.testing.assert_array_equal(x.download(), o.x)
     S.close()
     A.close()
+
+
+def test_autotuner_times_the_build_that_the_solve_runs(ctx):
+    """Both parts of a trial, every system and the largest alone, run the build that
+    the whole batch's launch runs (the last launch of the tuning is a long-pole one)."""
+    for nsys, rows, cluster, threads, build in ((600, (1000, 3000), 4, 256, DENSE), (24, (5000, 50000), 16, 512, DEEP)):
+        B = abi.batch_problem(nsys=nsys, min_rows=rows[0], max_rows=rows[1], seed=3)
+        P = B.problem
+        A = ctx.matrix(P.row_ptr, P.cols, P.vals, F32)
+        S = abi.Batch(ctx, A, B.sys_offsets, tol=1e-8, cluster_size=cluster, threads=threads,
+                      spmv_variant=abi.SPMV_ELL, max_outer=1, inner_max_iter=4)
+        assert S.info.tuned and S.selftest_build() == build
+        S.solve(ctx.vector(P.b), ctx.vector(P.n))
+        assert S.selftest_build() == build
+        S.close()
+        A.close()
