@@ -967,6 +967,9 @@ bool ilu_stencil_setup(ab2_context* ctx, const ab2_matrix* A, Ilu0Data& d, bool 
   // The 7-point geometry: kept by the matrix (AB2_FMT_STENCIL) or checked here.
   int nx = A->st_nx, ny = A->st_ny, nz = A->st_nz;
   if (nx == 0 && !stencil_geometry(ctx, A, &nx, &ny, &nz)) return false;
+  d.walk_cluster = schedule != AB2_ILU_STENCIL && nz <= kClusterPlanes;
+  require(schedule != AB2_ILU_STENCIL_CLUSTER || d.walk_cluster,
+          "ILU0 cluster schedule requested with more planes along z than it is offered for");
   d.st_nx = nx;
   d.st_ny = ny;
   d.st_nz = nz;
@@ -1009,9 +1012,6 @@ bool ilu_stencil_setup(ab2_context* ctx, const ab2_matrix* A, Ilu0Data& d, bool 
   dev_free(ctx, d.d_bands);
   d.d_bands = nullptr;
   set_walk_smem<double>();
-  d.walk_cluster = schedule != AB2_ILU_STENCIL && nz <= kClusterPlanes;
-  require(schedule != AB2_ILU_STENCIL_CLUSTER || d.walk_cluster,
-          "ILU0 cluster schedule requested with more planes along z than it is offered for");
   d.stencil = true;
   d.levels_l = d.levels_u = (int)(nx + ny + nz - 2);
   return true;

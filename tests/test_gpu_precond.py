@@ -332,3 +332,22 @@ def test_chebyshev_start_fused_with_bands(ctx):
         pc.apply(vx, vy)
         assert ctx.launches - before == launches
         A.close()
+
+
+def test_ilu0_cluster_schedule_is_refused_before_any_set_up(ctx):
+    """Past the planes it is offered for, the request ends with the grid's shape known:
+    nothing is factorised or packed for it."""
+    P = abi.diffusion(6, 5, 347, sigma=1.0, smooth=2.0, seed=3)
+    A = ctx.matrix(P.row_ptr, P.cols, P.vals, abi.FMT_CSR | abi.FMT_ELL | abi.FMT_STENCIL)
+    launches = []
+    for schedule in ("stencil", "stencil_cluster"):
+        before = ctx.launches
+        if schedule == "stencil":
+            abi.Precond(ctx, A, "ilu0", ilu_schedule=schedule)
+        else:
+            with pytest.raises(abi.AB2Error) as e:
+                abi.Precond(ctx, A, "ilu0", ilu_schedule=schedule)
+            assert e.value.code == abi.AB2_ERR_BAD_ARG
+        launches.append(ctx.launches - before)
+    assert launches[0] - launches[1] >= 7  # extract, fill, factor, pack, both sweeps' coefficients, hand-over words
+    A.close()
