@@ -380,6 +380,9 @@ __device__ __forceinline__ float quiet_nan<float>() {
 __device__ __forceinline__ bool waiting(double v) { return __double2hiint(v) == (int)(kSentinel >> 32); }
 __device__ __forceinline__ bool waiting(float v) { return is_sentinel(v); }
 
+__device__ __forceinline__ bool sign_bit(double v) { return __double2hiint(v) < 0; }
+__device__ __forceinline__ bool sign_bit(float v) { return __float_as_int(v) < 0; }
+
 // A bounded wait's give-up test, asked every 256 polls.
 __device__ __forceinline__ bool give_up(unsigned it, long long t0, int* err) {
   if ((it & 255) != 0) return false;
@@ -674,11 +677,19 @@ __global__ void __launch_bounds__(kWalkWarps * 32, 1)
         n[1] = Recip<T>::div(num(1, n[0], xb1), c.p[1], c.r[1], bad[1]);
         n[2] = Recip<T>::div(num(2, xl1, n[0]), c.p[2], c.r[2], bad[2]);
         n[3] = Recip<T>::div(num(3, n[2], n[1]), c.p[3], c.r[3], bad[3]);
-        if (__any_sync(0xffffffffu, bad[0] | bad[1] | bad[2] | bad[3])) {  // the step again, with plain divisions
-          n[0] = Recip<T>::slow(num(0, xl0, xb0), c.p[0], c.r[0]);
-          n[1] = Recip<T>::slow(num(1, n[0], xb1), c.p[1], c.r[1]);
-          n[2] = Recip<T>::slow(num(2, xl1, n[0]), c.p[2], c.r[2]);
-          n[3] = Recip<T>::slow(num(3, n[2], n[1]), c.p[3], c.r[3]);
+        if (__any_sync(0xffffffffu, bad[0] | bad[1] | bad[2] | bad[3])) {
+          // A dividend of +0 over a positive pivot in range has come out as the division's
+          // +0 (empty regions of a right-hand side are full of them); with anything else
+          // among the bad ones, the step again with plain divisions.
+          auto zero = [&](int q, T x) { return x == T(0) && !sign_bit(x) && c.r[q] > R(0); };
+          const bool hard = (bad[0] && !zero(0, num(0, xl0, xb0))) | (bad[1] && !zero(1, num(1, n[0], xb1))) |
+                            (bad[2] && !zero(2, num(2, xl1, n[0]))) | (bad[3] && !zero(3, num(3, n[2], n[1])));
+          if (__any_sync(0xffffffffu, hard)) {
+            n[0] = Recip<T>::slow(num(0, xl0, xb0), c.p[0], c.r[0]);
+            n[1] = Recip<T>::slow(num(1, n[0], xb1), c.p[1], c.r[1]);
+            n[2] = Recip<T>::slow(num(2, xl1, n[0]), c.p[2], c.r[2]);
+            n[3] = Recip<T>::slow(num(3, n[2], n[1]), c.p[3], c.r[3]);
+          }
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[q] = n[q];

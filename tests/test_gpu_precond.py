@@ -351,3 +351,26 @@ def test_ilu0_cluster_schedule_is_refused_before_any_set_up(ctx):
         launches.append(ctx.launches - before)
     assert launches[0] - launches[1] >= 7  # extract, fill, factor, pack, both sweeps' coefficients, hand-over words
     A.close()
+
+
+# Exact zeros in the sweeps: point sources, empty regions, all of it, of both signs,
+# and zeros over pivots outside the fast division's range, down to the sign bit.
+@pytest.mark.parametrize("dims", [(33, 18, 21), (40, 31, 1)])
+@pytest.mark.parametrize("scale", [1.0, 1e-140])
+def test_ilu0_zero_dividends(ctx, dims, scale):
+    P = abi.diffusion(*dims, sigma=1.0, smooth=2.0, seed=7)
+    vals = P.vals * scale
+    A = ctx.matrix(P.row_ptr, P.cols, vals)
+    pc = abi.Precond(ctx, A, "ilu0")
+    vz = ctx.vector(P.n)
+    point = np.zeros(P.n)
+    point[P.n // 2] = 1.0
+    last = np.zeros(P.n)
+    last[-1] = -3.0
+    half = rnd(P.n, 5)
+    half[P.n // 3:] = -0.0
+    for y in (point, last, -last, half, np.zeros(P.n), np.full(P.n, -0.0), np.where(np.arange(P.n) % 2 == 0, 0.0, -0.0)):
+        pc.apply(ctx.vector(y), vz)
+        np.testing.assert_array_equal(vz.download().view(np.int64),
+                                      O.ilu0_apply(P.row_ptr, P.cols, vals, y).view(np.int64))
+    A.close()
