@@ -374,3 +374,59 @@ def test_ilu0_zero_dividends(ctx, dims, scale):
         np.testing.assert_array_equal(vz.download().view(np.int64),
                                       O.ilu0_apply(P.row_ptr, P.cols, vals, y).view(np.int64))
     A.close()
+
+
+def _layers(layers, per_layer, entries, seed):
+    """Rows in layers, each hanging on `entries` rows of the layer before it and as
+    many of the one after it (fewer in the outer layers): one wavefront a layer."""
+    rng = np.random.default_rng(seed)
+    n = layers * per_layer
+    rows, cols = [np.arange(n)], [np.arange(n)]
+    for step in (-1, 1):
+        r = np.repeat(np.arange(n).reshape(layers, per_layer)[(1 if step < 0 else 0):(None if step < 0 else -1)], entries)
+        first = np.stack([rng.choice(per_layer, entries, replace=False) for _ in range(r.size // entries)]).ravel()
+        rows.append(r)
+        cols.append((r // per_layer + step) * per_layer + first)
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    order = np.lexsort((cols, rows))
+    rows, cols = rows[order], cols[order]
+    rp = np.zeros(n + 1, np.int32)
+    rp[1:] = np.cumsum(np.bincount(rows, minlength=n))
+    vals = np.where(rows == cols, 2.0 * entries + 1.0, -rng.uniform(0.1, 1.0, rows.size))
+    return rp, cols.astype(np.int32), vals
+
+
+# The one-CTA sweeps told from the sweeps across SMs by an application's launches
+# (one, two): wavefronts of more rows than the CTA's warps take at a time (its WIDE
+# builds) with 2, 4 and 8 entries a side, and a vector that fits shared memory to the
+# byte (28 x 970: 225,280) or misses it by eight (159 x 175).
+@pytest.mark.parametrize("kind,launches", [("wide2", 1), ("wide4", 1), ("wide8", 1), ("wide9", 2), ("wide3_odd", 1),
+                                           ("fits", 1), ("misses", 2)])
+def test_ilu0_one_cta_sweeps_run_where_they_should(ctx, kind, launches):
+    if kind.startswith("wide"):
+        rp, ci, vv = _layers(20, 1300 if kind != "wide3_odd" else 513, int(kind[4]), seed=int(kind[4]))
+    else:
+        P = abi.diffusion(*((28, 970) if kind == "fits" else (159, 175)), 1, sigma=1.0, smooth=2.0, seed=4)
+        rp, ci, vv = P.row_ptr, P.cols, P.vals
+    n = rp.size - 1
+    A = ctx.matrix(rp, ci, vv, abi.FMT_CSR | abi.FMT_ELL | abi.FMT_F32)
+    pc = abi.Precond(ctx, A, "ilu0")
+    np.testing.assert_array_equal(pc.ilu0_values(), O.ilu0_factor(rp, ci, vv))
+    vz = ctx.vector(n)
+    y0 = rnd(n, 11)
+    for y in (y0, np.where(np.arange(n) % 3 == 0, y0, -0.0), y0 * 1e-290, y0):
+        vy = ctx.vector(y)
+        before = ctx.launches
+        pc.apply(vy, vz)
+        assert ctx.launches - before == launches
+        np.testing.assert_array_equal(vz.download(), O.ilu0_apply(rp, ci, vv, y))
+    # the same in FP32, inside the mixed solver
+    kw = dict(solver="bicgs", precond="ilu0", tol=1e-10, max_outer=10, inner_tol=1e-4, inner_max_iter=500)
+    M = abi.Mixed(ctx, A, **kw)
+    x = ctx.vector(n)
+    st = M.solve(ctx.vector(y0), x)
+    o = O.mixed_solve(rp, ci, vv, y0, dot_mode=O.DOT_DEVICE_TREE, tree_blocks=ctx.info.reduction_max_blocks, **kw)
+    assert (st.outer_iterations, st.inner_iterations) == (o.outer_iterations, o.inner_iterations)
+    np.testing.assert_array_equal(x.download(), o.x)
+    M.close()
+    A.close()
