@@ -1114,6 +1114,10 @@ def main():
         world, rank, local = dist.ranks()
         if rank != 0:
             return 0
+        if not O.ref_available():
+            print(json.dumps({"impl": "reference", "unavailable": "Alien's templates are not built here (oracle/_ref; "
+                              "the reference's headers are absent): make -f oracle/Makefile"}))
+            return 0
         P = O.problem_diffusion(n1, n1, n1, sigma=1.0, smooth=4.0, seed=rank)
         return reference_main(a, world, rank, P, make_config(P))
 

@@ -36,3 +36,14 @@ def test_reference_arm_prints_one_complete_json_line():
     e2e = d["e2e"]
     assert e2e["value"] == d["value"] and e2e["unit"] == "s"
     assert e2e["h2d_bytes_per_step"] == 0 and e2e["d2h_bytes_per_step"] == 0
+
+
+def test_reference_arm_says_so_where_the_templates_are_not_built(tmp_path):
+    """One JSON line that names the reason, and exit code 0."""
+    code = ("import sys, pathlib; sys.argv = ['bench.py', '--impl', 'reference', '--n', '16']; sys.path.insert(0, '.');"
+            "from oracle import oracle; oracle.REF_SO = pathlib.Path('absent.so'); import bench; sys.exit(bench.main())")
+    out = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=600, check=True)
+    lines = [ln for ln in out.stdout.splitlines() if ln.startswith("{")]
+    assert len(lines) == 1
+    d = json.loads(lines[0])
+    assert d["impl"] == "reference" and d["unavailable"]
