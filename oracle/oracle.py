@@ -71,9 +71,13 @@ def build() -> None:
     subprocess.run(["make", "-s", "-f", str(HERE / "Makefile")], check=True)
 
 
+class ReferenceNotBuilt(ImportError):
+    """The library of Alien's own templates is absent (it needs the reference's headers)."""
+
+
 def _load(path: Path, prefix: str) -> C.CDLL:
     if not path.exists():
-        raise ImportError(f"{path} missing: run make -f oracle/Makefile")
+        raise (ReferenceNotBuilt if path == REF_SO else ImportError)(f"{path} missing: run make -f oracle/Makefile")
     L = C.CDLL(str(path))
     f = getattr(L, f"{prefix}_solve")
     f.restype = C.c_int
