@@ -9,12 +9,13 @@
 //   4 x { g_ij = sigmoid(u e_ij + c), e_ij = log|a_ij| - (log a_ii + log a_jj)/2 ;
 //         m_i = sum_j g_ij h_j ; h <- relu(W [h; m] + b) }                       (128 -> 64)
 //   z_i = s (wd . h5_i + bd + ws x0_i) / sqrt(a_ii)       (ws: the Jacobi skip)
-// Activations are stored in BF16 ([n][64], 128 B per node).  Each layer is
-// one fused kernel: neighbour gather, BF16 x BF16 -> FP32 tensor-core MMAs
-// (mma.sync m16n8k16; a warp computes 16 nodes x 64 outputs over K = 128) and
-// the bias/relu epilogue; the first layer recomputes h1 from x0 instead of
-// reading it, the last one applies the decoder in its epilogue, so inference
-// moves about 2 x 128 B per node and layer.  Training: hand-written backward kernels (loss
+// Activations are stored in BF16 ([n][64], 128 B per node); h1 by a kernel of its
+// own.  Each layer is one fused kernel, neighbour sums, dense layer on the tensor
+// cores (BF16 x BF16 -> FP32) and bias/relu epilogue, of two: on 3-D 7-point graphs
+// the grid layer (k_gnn_layer_grid: neighbours by bulk copy, tcgen05.mma), on others
+// the gather layer (k_gnn_layer: neighbours by index, mma.sync m16n8k16, a warp 16
+// nodes x 64 outputs over K = 128).  The last one applies the decoder in its
+// epilogue, so inference moves about 2 x 128 B per node and layer.  Training: hand-written backward kernels (loss
 // (z-e)^T A (z-e) / e^T A e on (residual, error) pairs), per-block partial
 // sums reduced in a fixed order (deterministic), Adam on FP32 master weights
 // with BF16 copies for the forward.
@@ -550,7 +551,7 @@ constexpr unsigned kTcZpOff = kTcZmOff + kTcBlockB;
 constexpr unsigned kTcEfOff = kTcZpOff + kTcBlockB;          //   64 x 6 floats
 constexpr unsigned kTcEfBytes = kTcHalf * 6 * 4;
 constexpr unsigned kTcStageB = kTcEfOff + kTcEfBytes;
-constexpr unsigned kTcOut = kTcStage + kTcStages * kTcStageB;  // the epilogue's half rows: 8 warps x 32 x 64 B
+constexpr unsigned kTcOut = kTcStage + kTcStages * kTcStageB;  // the epilogue's half rows: 4 warps x 32 x 64 B
 constexpr unsigned kTcOutB = 32 * kTcRowB / 2;
 constexpr unsigned kTcBias = kTcOut + kTcEpiWarps * kTcOutB;  // bias, wd: 2 x 64 floats
 constexpr unsigned kTcBar = kTcBias + 2 * kH * 4;            // 14 mbarriers, tensor-memory address, abort flag
@@ -558,6 +559,7 @@ constexpr unsigned kTcSmem = kTcBar + 128 + 1024;            // + slack to align
 constexpr unsigned kTcCols = 2 * kH;                         // tensor-memory columns: two accumulators
 static_assert(kTcSmem <= 227 * 1024, "grid layer: shared memory");
 static_assert(kTcA % 1024 == 0 && kTcABuf % 1024 == 0 && kTcStageB % 16 == 0, "grid layer: alignment");
+static_assert(kTcBias - kTcOut == 4 * 32 * 64, "grid layer: one staging buffer an epilogue warp");
 static_assert(2 * kTcHalf == kTcTile && kTcHalf % 8 == 0, "grid layer: two steps a tile, one swizzle for both");
 
 struct GridLayerArgs {
