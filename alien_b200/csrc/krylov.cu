@@ -882,12 +882,14 @@ __global__ void __launch_bounds__(1024, 1)
 
 // How a system of n rows fits the one-launch loop: threads a block, blocks, and
 // the rows of a thread (V logical blocks of the reduction grid, M rows each).
-// Where the line lies for short rows: up to three rows a logical thread in FP64 (909,000 rows on 148
-// SMs), four in FP32, beyond which the graph loop's two bandwidth-bound kernels are
-// as fast.  Measured on B200, us an iteration, graph loop / one launch: 7-point
+// Where the line lies for short rows: up to three rows a logical thread in FP64
+// (909,000 rows on 148 SMs), four in FP32, beyond which the graph loop's two
+// bandwidth-bound kernels are as fast.  Measured on B200, us an iteration, graph loop / one launch: 7-point
 // bands FP64 32^3 15.2 / 6.6, 64^3 21.8 / 11.9, 491,111 rows 24.7 / 18.1, 96^3 32.4 /
 // 28.6, 104^3 40.3 / 40.3 (ELL 43.6 / 47.8); FP32 (scaled Jacobi) 32^3 19.9 / 6.9, 96^3
-// 26.6 / 20.3, 104^3 28.4 / 23.8, 128 x 96 x 96 28.0 / 24.6.
+// 26.6 / 20.3, 104^3 28.4 / 23.8, 128 x 96 x 96 28.0 / 24.6.  Contexts that solve at the
+// same time take turns at it (all of it needs every SM): 491,111 rows, four threads with
+// a context each, 16.7 / 18.3 us an iteration over all, two 20.5 / 18.4.
 struct CgLoopFit {
   int threads = 0, blocks = 0, V = 0, M = 0;  // V = 0: too large
 };
@@ -918,10 +920,14 @@ CgLoopFit cg_loop_fit(const ab2_context* ctx, int n, bool fp32) {
 // 42.3; FP32 CSR 600,000 rows k = 32 183 / 174, 100,000 rows k = 32 41.9 / 41.2, 64 53.6 /
 // 62.3; FP64 CSR 300,000 rows k = 64 216 / 161.  One row of L entries among rows of 7
 // (2,000 rows): ELL FP64 L = 64 23.2 / 23.0, 128 28.9 / 40.1, FP32 21.3 / 20.5, 24.7 /
-// 36.8; CSR FP64 L = 1,900 244 / 220, FP32 L = 512 45.8 / 41.1, 1,900 99.7 / 139.
+// 36.8; CSR FP64 L = 1,900 244 / 220, FP32 L = 512 45.8 / 41.1, 1,900 99.7 / 139.  FP64 CSR
+// with rows of thousands of entries among ragged ones: 150,000 rows 476 / 393, 400,000
+// 1093 / 703, 100,000 and one of 20,000 1973 / 1977, but 800,000 (four rows a thread)
+// 1418 / 1504.
 bool cg_loop_pays(const ab2_matrix* A, ViewKind kind, bool fp32) {
   if (kind == ViewKind::Stencil) return true;
   const bool ell = kind == ViewKind::Ell;
+  if (!ell && !fp32 && A->n <= 600000) return true;
   const int any_size = ell ? (fp32 ? 16 : 32) : (fp32 ? 32 : 2048);  // widest row at any size ...
   const int small = ell ? 72 : (fp32 ? 512 : 2048);                  // ... of few entries
   if (A->widest_row > any_size) return A->widest_row <= small && A->nnz <= 3200000;

@@ -315,11 +315,14 @@ def test_launch_count_holds_the_whole_turns_of_the_graph_loop(ctx, iters):
 
 # Rows too wide for the one-launch loop take the graph loop: told apart by the
 # launches of a solve of 20 iterations, either side of each width limit.
-@pytest.mark.parametrize("variant,fp32,limit", [(abi.SPMV_ELL, False, 72), (abi.SPMV_CSR_SCALAR, False, 2048),
-                                                (abi.SPMV_ELL, True, 72), (abi.SPMV_CSR_SCALAR, True, 512)])
-def test_wide_rows_take_the_graph_loop(ctx, variant, fp32, limit):
-    n, iters = 5000, 20
-    for widest, one_launch in ((7, True), (limit, True), (limit + 1, False)):
+# (FP64 CSR has one only past 600,000 rows.)
+@pytest.mark.parametrize("variant,fp32,limit,n", [(abi.SPMV_ELL, False, 72, 5000), (abi.SPMV_ELL, True, 72, 5000),
+                                                  (abi.SPMV_CSR_SCALAR, False, 2048, 600001),
+                                                  (abi.SPMV_CSR_SCALAR, False, None, 5000),
+                                                  (abi.SPMV_CSR_SCALAR, True, 512, 5000)])
+def test_wide_rows_take_the_graph_loop(ctx, variant, fp32, limit, n):
+    iters = 20
+    for widest, one_launch in ((7, True), (limit, True), (limit + 1, False)) if limit else ((7, True), (5000, True)):
         row = np.concatenate([np.arange(n), np.full(widest - 1, n // 2)])
         col = np.concatenate([np.arange(n), np.delete(np.arange(n), n // 2)[: widest - 1]])
         order = np.lexsort((col, row))
