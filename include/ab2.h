@@ -275,7 +275,9 @@ typedef struct {
   int poly_order;
   int poly_factor_max_iter;
   int spmv_variant; /* AB2_SPMV_* used inside the loop */
-  int use_graph;    /* 1: iteration loop in a CUDA graph with a device-side while condition */
+  int use_graph;    /* 1: iteration loop on the device, in a CUDA graph with a device-side while
+                       condition or (CG with DIAG or NONE, small systems of short rows) in one
+                       cooperative launch, which waits until every SM is free; 0: host-driven */
   int ilu_schedule; /* AB2_ILU_* */
   int cheb_saad;    /* see ab2_precond_options */
   int cheb_lanczos;
