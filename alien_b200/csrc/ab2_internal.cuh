@@ -52,7 +52,7 @@ struct ab2_context {
   long long alloc_count = 0;
   long long fail_alloc_at = 0;
   // ... and (ab2_context_inject_lost_arrival) the grid barrier of the next one-launch
-  // CG loop at which a block keeps its arrival back (0: none).
+  // CG loop whose last arrival never comes (0: none).
   long long lose_arrival_at = 0;
   // Phase timers (ab2_context_set_phase_timing, or AB2_PERF_TIMER=1): null when off.
   ab2::PhaseTimer* timer = nullptr;

@@ -638,8 +638,9 @@ struct Pair2<float> {
   using type = float2;
 };
 
-// A grid barrier's bound, and the arrival count at which block 0 keeps its own back
-// (0: never): the failure the bound is there for, made without a fault.
+// A grid barrier's bound, and the arrival count at which the blocks wait for one
+// arrival more than there are (0: never): the failure the bound is there for, made
+// without a fault.
 struct LoopWait {
   long long cycles;
   unsigned int lost;
@@ -712,9 +713,9 @@ __device__ __forceinline__ bool loop_exchange(T (&acc)[V][NC], T* partials, unsi
   loop_partials<NC, V>(acc, s_warp, G, partials);
   __syncthreads();
   target += gridDim.x;
+  if (target == wait.lost) ++target;
   if (threadIdx.x == 0) {
-    if (blockIdx.x != 0 || target != wait.lost)
-      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
     const long long t0 = clock64();
     int ok = 1;
     for (unsigned it = 1;; ++it) {

@@ -88,7 +88,7 @@ extern "C" int ab2_context_inject_alloc_failure(ab2_context* ctx, long long nth)
 }
 
 // The failure the one-launch CG loop's bounded barriers are there for, without a
-// fault: one arrival is kept back (krylov.cu, LoopWait), the waits run out and the
+// fault: the blocks wait for one arrival too many (krylov.cu, LoopWait), run out and the
 // launch ends by itself.
 extern "C" int ab2_context_inject_lost_arrival(ab2_context* ctx, long long nth) {
   if (!ctx || nth < 0) return AB2_ERR_BAD_ARG;

@@ -547,7 +547,7 @@ int ab2_selftest_batch_build(const ab2_batch* batch, int* build);
 int ab2_context_inject_alloc_failure(ab2_context* ctx, long long nth);
 /* The same for the grid barriers of the one-launch CG loop: in the next such loop
  * on ctx (a solve of CG with AB2_PC_DIAG or AB2_PC_NONE, or a mixed solve's inner
- * one) one block never arrives at the nth barrier, every wait of that launch is
+ * one) an arrival at the nth barrier never comes, every wait of that launch is
  * bounded by ~20 ms instead of ~2 s, and the solve reports AB2_ERR_TIMEOUT; 0
  * turns it off. */
 int ab2_context_inject_lost_arrival(ab2_context* ctx, long long nth);
